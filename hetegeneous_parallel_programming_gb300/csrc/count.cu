@@ -3,8 +3,8 @@
 // Work is cut into 4096-edge tiles.  A planning pass computes per-tile
 // degree features and picks an exact intersection strategy ("arm") for each
 // tile, either with fixed degree thresholds or with the MLP cost model.
-// Tiles are radix-sorted into one queue per arm (heaviest first) and each
-// arm runs as a persistent kernel whose blocks pull tiles with an atomic
+// Tiles are binned into one queue per arm (heaviest first) and each arm that
+// the selector can choose runs as a persistent kernel whose blocks pull tiles with an atomic
 // head, so load balance does not depend on the launch grid.
 //
 // Arms (all exact; they replace the reference's warp_vertex +
@@ -148,46 +148,69 @@ struct PullKeys {
   }
 };
 
-// One warp per tile: features, the arm, the queue key and the algorithmic
+// Work queues: tiles are counted into bins (arm, log2 of their work in
+// quarter steps, heaviest first) and scattered bin by bin, so each arm's
+// queue starts with its heaviest tiles.  A queue only needs the order to a
+// quarter octave, so two launches (plan, queue) do what a 44-bit radix sort
+// of exact work keys took 18 launches for (120 us of every call; the plan,
+// queue and empty-arm launches of ER n = 16384 went from 300 to 100 us).
+constexpr int Q_LEVELS = 128;                       // 32 octaves of work, 4 steps each (heavier tiles share the first)
+constexpr int Q_BINS = TC_NUM_ARMS * Q_LEVELS;
+constexpr int Q_THREADS = 256;
+constexpr int Q_TILES = 1024;                       // tiles per block of queue_kernel
+static_assert(Q_BINS % Q_THREADS == 0, "each thread of a queue block scans the same number of bins");
+
+__device__ __forceinline__ int work_level(unsigned long long work) {
+  const int lg = 63 - __clzll((long long)(work | 1ull));
+  const int step = lg >= 2 ? (int)((work >> (lg - 2)) & 3ull) : 0;
+  return Q_LEVELS - 1 - min(Q_LEVELS - 1, 4 * lg + step);
+}
+
+// One block per tile: features, the arm, the queue bin and the algorithmic
 // bytes; a tile that goes to PULL also adds its edges' grouping keys to the
-// PULL histogram while its columns are still in cache.
+// PULL histogram while its columns are still in cache.  Bound by the latency
+// of its gathers (row pointers, target degrees): a block per tile gives every
+// thread 16 edges instead of the 128 per lane of a warp per tile, so graphs of
+// a few hundred tiles fill the GPU (33 tiles, ER n = 16384: the call went
+// from 547 to 350 us with this and the queues below; R-MAT scale 24, 63 569
+// tiles, from 55.76 to 54.98 ms).
+struct PlanPart {  // one warp's share of a tile
+  float sda, smin, salr, sin;
+  unsigned long long sdb, srow;
+  unsigned bins01, bins23, bins45, nrows, maxdr, maxwin;
+};
+
 __global__ void __launch_bounds__(PLAN_THREADS) plan_kernel(DevDag g, int64_t T, int selector, int force_arm,
-                                                           const float *__restrict__ mlp, float *__restrict__ feats,
+                                                           float *__restrict__ feats,
                                                            int32_t *__restrict__ arm_out,
-                                                           uint64_t *__restrict__ qkeys,
-                                                           uint32_t *__restrict__ qvals,
+                                                           uint32_t *__restrict__ tile_level,
                                                            unsigned long long *__restrict__ tile_bytes,
-                                                           PullKeys pk, unsigned *__restrict__ pull_cnt,
-                                                           float margin) {
-  extern __shared__ float s_w[];
-  const int lane = threadIdx.x & 31;
-  if (selector == TC_SELECT_LEARNED) {
-    for (int i = threadIdx.x; i < TC_MLP_PARAM_COUNT; i += blockDim.x)
-      s_w[i] = __bfloat162float(__float2bfloat16(mlp[i]));
-    __syncthreads();
-  }
+                                                           uint32_t *__restrict__ bin_cnt,
+                                                           unsigned long long *__restrict__ arm_bytes,
+                                                           PullKeys pk, unsigned *__restrict__ pull_cnt) {
+  __shared__ PlanPart s_part[PLAN_THREADS / 32];
+  __shared__ int s_arm;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // tiles interleaved over the PULL source blocks (see PL_INTERLEAVE): the
   // grid covers S * per slots, some past the last tile
   const int64_t per = pk.block_edges / TILE_EDGES, S = (T + per - 1) / per;
-  const int64_t i = (int64_t)blockIdx.x * (PLAN_THREADS / 32) + (threadIdx.x >> 5);
-  const bool lv = PL_INTERLEAVE && S > 1;
-  const int64_t t = lv ? (i % S) * per + i / S : i;
-  if (i >= (lv ? S * per : T) || t >= T) return;
+  const int64_t i = (int64_t)blockIdx.x;
+  const int64_t t = PL_INTERLEAVE && S > 1 ? (i % S) * per + i / S : i;
+  if (t >= T) return;
   const int64_t e0 = t * TILE_EDGES, e1 = min(g.m, e0 + TILE_EDGES);
-  float sda = 0, sdb = 0, smin = 0, smax = 0, salr = 0, sin = 0;
-  float bins[6] = {0, 0, 0, 0, 0, 0};
-  unsigned long long work = 0, alg = 0;
-  int nrows = 0;
-  long long maxdr = 0, maxwin = 0;
-  // PLAN_UNROLL edges per lane at a time, their loads in three rounds, each
+  float sda = 0, smin = 0, salr = 0, sin = 0;
+  unsigned long long sdb = 0, srow = 0;
+  unsigned bins01 = 0, bins23 = 0, bins45 = 0;  // two 16-bit counters each
+  unsigned nrows = 0, maxdr = 0, maxwin = 0;
+  // PLAN_UNROLL edges per thread at a time, their loads in three rounds, each
   // round's loads all in flight: (row, target, previous edge's row); (row
   // pointers, target degrees); for an edge that starts its row in the tile,
   // the two ends of its row window
-  for (int64_t eb = e0 + lane; eb < e1; eb += 32 * PLAN_UNROLL) {
+  for (int64_t eb = e0 + threadIdx.x; eb < e1; eb += PLAN_THREADS * PLAN_UNROLL) {
     int32_t rr[PLAN_UNROLL], ss[PLAN_UNROLL], pr[PLAN_UNROLL];
 #pragma unroll
     for (int u = 0; u < PLAN_UNROLL; ++u) {
-      const int64_t e = eb + 32 * u;
+      const int64_t e = eb + PLAN_THREADS * u;
       rr[u] = e < e1 ? g.src[e] : 0;
       ss[u] = e < e1 ? g.col[e] : 0;
       pr[u] = e < e1 && e > e0 ? g.src[e - 1] : -1;
@@ -196,7 +219,7 @@ __global__ void __launch_bounds__(PLAN_THREADS) plan_kernel(DevDag g, int64_t T,
     int2 dq[PLAN_UNROLL];
 #pragma unroll
     for (int u = 0; u < PLAN_UNROLL; ++u) {
-      const bool in = eb + 32 * u < e1;
+      const bool in = eb + PLAN_THREADS * u < e1;
       rbs[u] = in ? g.rowptr[rr[u]] : 0;
       res[u] = in ? g.rowptr[rr[u] + 1] : 0;
       if (!in) dq[u] = make_int2(0, 0);
@@ -206,7 +229,7 @@ __global__ void __launch_bounds__(PLAN_THREADS) plan_kernel(DevDag g, int64_t T,
     int32_t wlo[PLAN_UNROLL], whi[PLAN_UNROLL];
 #pragma unroll
     for (int u = 0; u < PLAN_UNROLL; ++u) {
-      const int64_t e = eb + 32 * u;
+      const int64_t e = eb + PLAN_THREADS * u;
       const int64_t s0 = g.restrict_after ? e + 1 : rbs[u];
       const bool wide = e < e1 && pr[u] != rr[u] && s0 < res[u];  // a row start with a window
       wlo[u] = wide ? g.col[s0] : 0;
@@ -214,117 +237,166 @@ __global__ void __launch_bounds__(PLAN_THREADS) plan_kernel(DevDag g, int64_t T,
     }
 #pragma unroll
     for (int u = 0; u < PLAN_UNROLL; ++u) {
-      const int64_t e = eb + 32 * u;
+      const int64_t e = eb + PLAN_THREADS * u;
       if (e >= e1) break;
       const int64_t rb = rbs[u], re = res[u];
       const int64_t a0 = g.restrict_after ? e + 1 : rb;
       const float da = (float)(re - a0);
-      const float db = (float)dq[u].x, ins = (float)dq[u].y;  // target's out-degree and DAG in-degree
+      const float db = (float)dq[u].x;  // target's out-degree
       sda += da;
-      sdb += db;
-      const float mn = fminf(da, db), mx = fmaxf(da, db);
+      sdb += (unsigned long long)(unsigned)dq[u].x;
+      srow += (unsigned long long)(re - rb);
+      const float mn = fminf(da, db);
       smin += mn;
-      smax += mx;
-      const float lr = flog2p1(da) - flog2p1(db);
-      salr += fabsf(lr);
-      sin += ins;  // how many edges share this target's list
-      const int bin = mn < 2.f ? 0 : mn < 8.f ? 1 : mn < 32.f ? 2 : mn < 128.f ? 3 : mn < 512.f ? 4 : 5;
-#pragma unroll
-      for (int k = 0; k < 6; ++k) bins[k] += (bin == k) ? 1.f : 0.f;
-      work += (unsigned long long)(da + db);
-      alg += 4ULL * (unsigned long long)((re - rb) + (int64_t)db) + 4ULL;
+      salr += fabsf(flog2p1(da) - flog2p1(db));
+      sin += (float)dq[u].y;  // DAG in-degree: how many edges share this target's list
+      const unsigned one = mn < 2.f || (mn >= 8.f && mn < 32.f) || (mn >= 128.f && mn < 512.f) ? 1u : 1u << 16;
+      if (mn < 8.f) bins01 += one;
+      else if (mn < 128.f) bins23 += one;
+      else bins45 += one;
       if (pr[u] != rr[u]) {  // the edge starts its row in the tile (pr = -1 for the tile's first edge)
         ++nrows;
-        maxdr = max(maxdr, (long long)(re - rb));
-        maxwin = max(maxwin, (long long)whi[u] - (long long)wlo[u] + 1);
+        maxdr = max(maxdr, (unsigned)(re - rb));
+        maxwin = max(maxwin, (unsigned)max((long long)whi[u] - (long long)wlo[u] + 1, 0ll));
       }
     }
   }
-  sda = warp_sum(sda); sdb = warp_sum(sdb); smin = warp_sum(smin); smax = warp_sum(smax);
-  salr = warp_sum(salr); sin = warp_sum(sin);
-#pragma unroll
-  for (int k = 0; k < 6; ++k) bins[k] = warp_sum(bins[k]);
-  work = warp_sum(work);
-  alg = warp_sum(alg);
-  nrows = warp_sum(nrows);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    maxdr = max(maxdr, __shfl_xor_sync(TC_FULL_MASK, maxdr, o));
-    maxwin = max(maxwin, __shfl_xor_sync(TC_FULL_MASK, maxwin, o));
-  }
-  const float ne = (float)(e1 - e0);
-  PlanStats st;
-  st.mean_da = sda / ne; st.mean_db = sdb / ne; st.mean_min = smin / ne; st.mean_max = smax / ne;
-  st.mean_in = sin / ne; st.alr = salr / ne;
-  st.nrows = (float)nrows; st.maxdr = (float)maxdr; st.maxwin = (float)maxwin; st.frac = ne / (float)TILE_EDGES;
-  float f[TC_MLP_FEATURES];
-  f[0] = flog2p1(st.mean_da) / 16.f;
-  f[1] = flog2p1(st.mean_db) / 16.f;
-  f[2] = flog2p1(st.mean_in) / 24.f;
-  f[3] = st.alr / 16.f;
-  f[4] = flog2p1(st.mean_min) / 16.f;
-  f[5] = flog2p1(st.mean_max) / 16.f;
-  f[6] = flog2p1(st.nrows) / 12.f;
-  f[7] = flog2p1(st.maxdr) / 16.f;
-#pragma unroll
-  for (int k = 0; k < 6; ++k) f[8 + k] = bins[k] / ne;
-  f[14] = flog2p1(st.maxwin) / 24.f;
-  f[15] = flog2p1((float)g.m) / 32.f;  // graph size: how much of it the L2 can hold
-  int arm;
-  if (selector == TC_SELECT_FORCE) arm = force_arm;
-  else if (selector == TC_SELECT_LEARNED) {
-    // The fixed rule keeps the PULL decision: a PULL tile's cost depends on
-    // how many of its targets' in-edges other PULL tiles share (the table
-    // build is spread over them), which per-tile costs profiled one arm at a
-    // time cannot show.  The cost model picks among the per-edge arms for
-    // every other tile.
-    const int fx = __shfl_sync(TC_FULL_MASK, fixed_select(st), 0);
-    arm = fx == TC_ARM_PULL ? TC_ARM_PULL : mlp_select(s_w, f, lane, TC_ARM_PULL, fx, margin);
-  } else {
-    arm = fixed_select(st);
-  }
-  arm = __shfl_sync(TC_FULL_MASK, arm, 0);
-  if (lane < TC_MLP_FEATURES) feats[t * TC_MLP_FEATURES + lane] = f[lane];
-  if (arm == TC_ARM_PULL) {
-    const int64_t kb = pk.block_base(t), lb = pk.low_base(t);
-    for (int64_t e = e0 + lane; e < e1; e += 32) atomicAdd(pull_cnt + pk.key_in(kb, lb, g.col[e]), 1u);
-  }
-  if (lane == 0) {
-    arm_out[t] = arm;
-    const unsigned long long W40 = (1ULL << 40) - 1;
-    qkeys[t] = ((unsigned long long)arm << 40) | (W40 - min(work, W40));
-    qvals[t] = (uint32_t)t;
-    tile_bytes[t] = alg;
-  }
-}
-
-// Algorithmic bytes of every arm's tiles (block a sums queue a).
-__global__ void arm_bytes_kernel(const uint32_t *__restrict__ qtiles, const int64_t *__restrict__ qoff,
-                                 const unsigned long long *__restrict__ tile_bytes,
-                                 unsigned long long *__restrict__ out) {
-  __shared__ unsigned long long part[8];
-  const int a = blockIdx.x;
-  unsigned long long s = 0;
-  for (int64_t i = qoff[a] + threadIdx.x; i < qoff[a + 1]; i += blockDim.x) s += tile_bytes[qtiles[i]];
-  s = warp_sum(s);
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+  PlanPart p;
+  p.sda = warp_sum(sda);
+  p.smin = warp_sum(smin);
+  p.salr = warp_sum(salr);
+  p.sin = warp_sum(sin);
+  p.sdb = warp_sum(sdb);
+  p.srow = warp_sum(srow);
+  p.bins01 = __reduce_add_sync(TC_FULL_MASK, bins01);
+  p.bins23 = __reduce_add_sync(TC_FULL_MASK, bins23);
+  p.bins45 = __reduce_add_sync(TC_FULL_MASK, bins45);
+  p.nrows = __reduce_add_sync(TC_FULL_MASK, nrows);
+  p.maxdr = __reduce_max_sync(TC_FULL_MASK, maxdr);
+  p.maxwin = __reduce_max_sync(TC_FULL_MASK, maxwin);
+  if (lane == 0) s_part[warp] = p;
   __syncthreads();
   if (threadIdx.x == 0) {
-    unsigned long long t = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += part[w];
-    out[a] = t;
+    p = s_part[0];
+    for (int w = 1; w < PLAN_THREADS / 32; ++w) {
+      const PlanPart &q = s_part[w];
+      p.sda += q.sda; p.smin += q.smin; p.salr += q.salr; p.sin += q.sin;
+      p.sdb += q.sdb; p.srow += q.srow;
+      p.bins01 += q.bins01; p.bins23 += q.bins23; p.bins45 += q.bins45;
+      p.nrows += q.nrows;
+      p.maxdr = max(p.maxdr, q.maxdr);
+      p.maxwin = max(p.maxwin, q.maxwin);
+    }
+    const float ne = (float)(e1 - e0);
+    PlanStats st;
+    st.mean_da = p.sda / ne; st.mean_db = (float)p.sdb / ne; st.mean_min = p.smin / ne;
+    st.mean_max = (p.sda + (float)p.sdb - p.smin) / ne;
+    st.mean_in = p.sin / ne; st.alr = p.salr / ne;
+    st.nrows = (float)p.nrows; st.maxdr = (float)p.maxdr; st.maxwin = (float)p.maxwin;
+    float f[TC_MLP_FEATURES];
+    f[0] = flog2p1(st.mean_da) / 16.f;
+    f[1] = flog2p1(st.mean_db) / 16.f;
+    f[2] = flog2p1(st.mean_in) / 24.f;
+    f[3] = st.alr / 16.f;
+    f[4] = flog2p1(st.mean_min) / 16.f;
+    f[5] = flog2p1(st.mean_max) / 16.f;
+    f[6] = flog2p1(st.nrows) / 12.f;
+    f[7] = flog2p1(st.maxdr) / 16.f;
+    f[8] = (float)(p.bins01 & 0xffffu) / ne;
+    f[9] = (float)(p.bins01 >> 16) / ne;
+    f[10] = (float)(p.bins23 & 0xffffu) / ne;
+    f[11] = (float)(p.bins23 >> 16) / ne;
+    f[12] = (float)(p.bins45 & 0xffffu) / ne;
+    f[13] = (float)(p.bins45 >> 16) / ne;
+    f[14] = flog2p1(st.maxwin) / 24.f;
+    f[15] = flog2p1((float)g.m) / 32.f;  // graph size: how much of it the L2 can hold
+    float4 *fo = reinterpret_cast<float4 *>(feats + t * TC_MLP_FEATURES);
+#pragma unroll
+    for (int k = 0; k < TC_MLP_FEATURES / 4; ++k) fo[k] = make_float4(f[4 * k], f[4 * k + 1], f[4 * k + 2], f[4 * k + 3]);
+    const int arm = selector == TC_SELECT_FORCE ? force_arm : fixed_select(st);
+    const int level = work_level((unsigned long long)p.sda + p.sdb);
+    const unsigned long long alg = 4ull * (p.srow + p.sdb + (unsigned long long)(e1 - e0));
+    arm_out[t] = arm;
+    tile_level[t] = (uint32_t)level;
+    tile_bytes[t] = alg;
+    if (selector != TC_SELECT_LEARNED) {  // the learned selection counts its own choices
+      atomicAdd(bin_cnt + arm * Q_LEVELS + level, 1u);
+      atomicAdd(arm_bytes + arm, alg);
+    }
+    s_arm = arm;
+  }
+  __syncthreads();
+  if (s_arm == TC_ARM_PULL) {
+    const int64_t kb = pk.block_base(t), lb = pk.low_base(t);
+    for (int64_t e = e0 + threadIdx.x; e < e1; e += PLAN_THREADS) atomicAdd(pull_cnt + pk.key_in(kb, lb, g.col[e]), 1u);
   }
 }
 
-__global__ void qoff_kernel(const uint64_t *__restrict__ keys, int64_t T, int64_t *__restrict__ qoff) {
-  const int k = threadIdx.x;
-  if (k > TC_NUM_ARMS) return;
-  int64_t lo = 0, hi = T;  // first index with arm >= k
-  while (lo < hi) {
-    const int64_t mid = (lo + hi) >> 1;
-    if ((int64_t)(keys[mid] >> 40) < k) lo = mid + 1; else hi = mid;
+// Learned selection, one warp per tile over the planner's features.  The
+// fixed rule keeps the PULL decision: a PULL tile's cost depends on how many
+// of its targets' in-edges other PULL tiles share (the table build is spread
+// over them), which per-tile costs profiled one arm at a time cannot show.
+// The cost model picks among the per-edge arms for every other tile.
+__global__ void __launch_bounds__(PLAN_THREADS) learned_select_kernel(int64_t T, const float *__restrict__ mlp,
+                                                                     const float *__restrict__ feats, float margin,
+                                                                     int32_t *__restrict__ arm_io,
+                                                                     const uint32_t *__restrict__ tile_level,
+                                                                     const unsigned long long *__restrict__ tile_bytes,
+                                                                     uint32_t *__restrict__ bin_cnt,
+                                                                     unsigned long long *__restrict__ arm_bytes) {
+  extern __shared__ float s_w[];
+  const int lane = threadIdx.x & 31;
+  for (int i = threadIdx.x; i < TC_MLP_PARAM_COUNT; i += blockDim.x)
+    s_w[i] = __bfloat162float(__float2bfloat16(mlp[i]));
+  __syncthreads();
+  const int64_t warps = (int64_t)gridDim.x * (PLAN_THREADS / 32);
+  for (int64_t t = (int64_t)blockIdx.x * (PLAN_THREADS / 32) + (threadIdx.x >> 5); t < T; t += warps) {
+    int arm = arm_io[t];
+    if (arm != TC_ARM_PULL) {
+      float f[TC_MLP_FEATURES];
+#pragma unroll
+      for (int k = 0; k < TC_MLP_FEATURES; ++k) f[k] = feats[t * TC_MLP_FEATURES + k];
+      arm = mlp_select(s_w, f, lane, TC_ARM_PULL, arm, margin);
+    }
+    if (lane == 0) {
+      arm_io[t] = arm;
+      atomicAdd(bin_cnt + arm * Q_LEVELS + tile_level[t], 1u);
+      atomicAdd(arm_bytes + arm, tile_bytes[t]);
+    }
   }
-  qoff[k] = lo;
+}
+
+// Scatters the tiles into their bins.  Every block scans the bin counts for
+// itself (Q_BINS words from L2); block 0 also writes the arms' queue offsets
+// and resets the queue heads.  bin_fill starts at zero.
+__global__ void __launch_bounds__(Q_THREADS) queue_kernel(int64_t T, const int32_t *__restrict__ arm,
+                                                         const uint32_t *__restrict__ tile_level,
+                                                         const uint32_t *__restrict__ bin_cnt,
+                                                         uint32_t *__restrict__ bin_fill, int64_t *__restrict__ qoff,
+                                                         uint32_t *__restrict__ qtiles, unsigned *__restrict__ heads) {
+  __shared__ uint32_t start[Q_BINS];
+  __shared__ uint32_t tmp[33];
+  constexpr int PER = Q_BINS / Q_THREADS;
+  uint32_t c[PER], s = 0;
+#pragma unroll
+  for (int k = 0; k < PER; ++k) s += c[k] = bin_cnt[threadIdx.x * PER + k];
+  uint32_t tot;
+  uint32_t run = block_exclusive_scan<uint32_t>(s, tmp, &tot);
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {
+    start[threadIdx.x * PER + k] = run;
+    run += c[k];
+  }
+  __syncthreads();
+  if (blockIdx.x == 0) {
+    if (threadIdx.x <= TC_NUM_ARMS) qoff[threadIdx.x] = threadIdx.x < TC_NUM_ARMS ? start[threadIdx.x * Q_LEVELS] : T;
+    if (threadIdx.x < 64) heads[threadIdx.x] = 0u;
+  }
+  const int64_t t1 = min(T, ((int64_t)blockIdx.x + 1) * Q_TILES);
+  for (int64_t t = (int64_t)blockIdx.x * Q_TILES + threadIdx.x; t < t1; t += Q_THREADS) {
+    const int b = arm[t] * Q_LEVELS + (int)tile_level[t];
+    qtiles[start[b] + atomicAdd(bin_fill + b, 1u)] = (uint32_t)t;
+  }
 }
 
 // ---- shared pieces of the arm kernels -----------------------------------------
@@ -2175,7 +2247,7 @@ static int arm_smem(int arm) { return arm == TC_ARM_BITMAP ? BM_SMEM_BYTES : 0; 
 
 tc_status init_arm_occupancy(tc_ctx *ctx) {
   TC_CHECK_CUDA(ctx, cudaFuncSetAttribute(bitmap_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BM_SMEM_BYTES));
-  TC_CHECK_CUDA(ctx, cudaFuncSetAttribute(plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  TC_CHECK_CUDA(ctx, cudaFuncSetAttribute(learned_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)(TC_MLP_PARAM_COUNT * sizeof(float))));
   for (int a = 0; a < TC_NUM_ARMS; ++a) {
     int nb = 0;
@@ -2191,7 +2263,7 @@ tc_status init_arm_occupancy(tc_ctx *ctx) {
 static int64_t pull_key_count(int64_t n, int64_t T, int block_tiles, PullKeys *pk);
 
 static size_t count_sort_scratch_bytes(const tc_ctx *ctx, int64_t n, int64_t T) {
-  return std::max(radix_sort_scratch_bytes(ctx, T > 0 ? T : 1), scan_scratch_bytes(ctx, pull_key_count(n, T, ctx->pull_block_tiles, nullptr) + 1));
+  return scan_scratch_bytes(ctx, pull_key_count(n, T, ctx->pull_block_tiles, nullptr) + 1);
 }
 
 // Hub bit rows: one row per dense hub (the top min(n, PL_DENSE_HUB) ids), each
@@ -2204,15 +2276,13 @@ size_t count_scratch_bytes(const tc_ctx *ctx, int64_t n, int64_t m) {
   const int64_t T = (m + TILE_EDGES - 1) / TILE_EDGES;
   Sizer sz;
   sz.take<float>(T * TC_MLP_FEATURES);
-  sz.take<uint64_t>(T);
-  sz.take<uint64_t>(T);
   sz.take<uint32_t>(T);
   sz.take<uint32_t>(T);
   sz.take<int32_t>(T);
   sz.take<int64_t>(TC_NUM_ARMS + 1);
   sz.take<unsigned long long>(T);
   sz.take<unsigned long long>(T);
-  sz.take<unsigned long long>(TC_NUM_ARMS);
+  sz.take<unsigned long long>(TC_NUM_ARMS + Q_BINS);
   sz.take<uint32_t>(pull_key_count(n, T, ctx->pull_block_tiles, nullptr) + 1);
   sz.take<uint2>(m);
   sz.take<uint4>(hub_bits_words4(n));
@@ -2222,16 +2292,14 @@ size_t count_scratch_bytes(const tc_ctx *ctx, int64_t n, int64_t m) {
 tc_status count_carve(const tc_ctx *ctx, int64_t n, int64_t m, Bump &bump, CountBufs &cb, bool want_cycles) {
   const int64_t T = (m + TILE_EDGES - 1) / TILE_EDGES;
   cb.features = bump.take<float>(T * TC_MLP_FEATURES);
-  cb.qkeys0 = bump.take<uint64_t>(T);
-  cb.qkeys1 = bump.take<uint64_t>(T);
-  cb.qvals0 = bump.take<uint32_t>(T);
-  cb.qvals1 = bump.take<uint32_t>(T);
+  cb.tile_level = bump.take<uint32_t>(T);
+  cb.qtiles = bump.take<uint32_t>(T);
   cb.arm = bump.take<int32_t>(T);
   cb.qoff = bump.take<int64_t>(TC_NUM_ARMS + 1);
   unsigned long long *cyc = bump.take<unsigned long long>(T);
   cb.tile_cycles = want_cycles ? cyc : nullptr;
   cb.tile_bytes = bump.take<unsigned long long>(T);
-  cb.arm_bytes = bump.take<unsigned long long>(TC_NUM_ARMS);
+  cb.arm_bytes = bump.take<unsigned long long>(TC_NUM_ARMS + Q_BINS);  // then the bin counts and fills
   cb.pull_pos = bump.take<uint32_t>(pull_key_count(n, T, ctx->pull_block_tiles, nullptr) + 1);
   cb.pull_er = bump.take<uint2>(m);
   cb.hub_bits = bump.take<uint4>(hub_bits_words4(n));
@@ -2368,6 +2436,15 @@ static tc_status run_pull(tc_ctx *ctx, const DevDag &g_in, CountBufs &cb, uint32
   return TC_OK;
 }
 
+// Arms that the selector can choose; the others' queues are empty, so they
+// are not launched (each empty launch costs 4 to 8 us on a small graph).
+static bool arm_possible(const tc_opts &opts, int a) {
+  if (opts.selector == TC_SELECT_FORCE) return a == opts.force_arm;
+  if (opts.selector == TC_SELECT_LEARNED) return true;
+  return a == TC_ARM_PULL || a == TC_ARM_BITMAP || a == TC_ARM_BSEARCH_32 || a == TC_ARM_MPATH_2 ||
+         a == TC_ARM_BSEARCH_4;  // fixed_select's choices
+}
+
 tc_status run_count(tc_ctx *ctx, const DevDag &g_in, const tc_opts &opts, CountBufs &cb, uint32_t *out, bool timing) {
   DevDag g = g_in;
   g.flags = ctx->d_flags;
@@ -2381,43 +2458,42 @@ tc_status run_count(tc_ctx *ctx, const DevDag &g_in, const tc_opts &opts, CountB
     TC_CHECK_CUDA(ctx, cudaMemsetAsync(cb.qoff, 0, sizeof(int64_t) * (TC_NUM_ARMS + 1), ctx->stream));
     TC_CHECK_CUDA(ctx, cudaMemsetAsync(cb.arm_bytes, 0, sizeof(unsigned long long) * TC_NUM_ARMS, ctx->stream));
   } else {
-    const size_t plan_smem = opts.selector == TC_SELECT_LEARNED ? TC_MLP_PARAM_COUNT * sizeof(float) : 0;
     PullKeys pk;
     const int64_t K = pull_key_count(g.n, T, ctx->pull_block_tiles, &pk);
     const int64_t per = pk.block_edges / TILE_EDGES, S = (T + per - 1) / per;
     const int64_t slots = PL_INTERLEAVE && S > 1 ? S * per : T;
-    const int plan_blocks = (int)((slots + (PLAN_THREADS / 32) - 1) / (PLAN_THREADS / 32));
+    uint32_t *bin_cnt = reinterpret_cast<uint32_t *>(cb.arm_bytes + TC_NUM_ARMS), *bin_fill = bin_cnt + Q_BINS;
     TC_CHECK_CUDA(ctx, cudaMemsetAsync(cb.pull_pos, 0, sizeof(uint32_t) * (K + 1), ctx->stream));
-    plan_kernel<<<plan_blocks, PLAN_THREADS, plan_smem, ctx->stream>>>(g, T, opts.selector, opts.force_arm,
-                                                                       ctx->d_mlp, cb.features, cb.arm, cb.qkeys0,
-                                                                       cb.qvals0, cb.tile_bytes, pk, cb.pull_pos, ctx->mlp_margin);
+    TC_CHECK_CUDA(ctx, cudaMemsetAsync(cb.arm_bytes, 0, sizeof(unsigned long long) * (TC_NUM_ARMS + Q_BINS), ctx->stream));
+    plan_kernel<<<(unsigned)slots, PLAN_THREADS, 0, ctx->stream>>>(g, T, opts.selector, opts.force_arm, cb.features,
+                                                                   cb.arm, cb.tile_level, cb.tile_bytes, bin_cnt,
+                                                                   cb.arm_bytes, pk, cb.pull_pos);
+    TC_CHECK_LAUNCH(ctx);
+    if (opts.selector == TC_SELECT_LEARNED) {
+      learned_select_kernel<<<grid_for(ctx, T, PLAN_THREADS / 32, 4), PLAN_THREADS, TC_MLP_PARAM_COUNT * sizeof(float),
+                              ctx->stream>>>(T, ctx->d_mlp, cb.features, ctx->mlp_margin, cb.arm, cb.tile_level,
+                                             cb.tile_bytes, bin_cnt, cb.arm_bytes);
+      TC_CHECK_LAUNCH(ctx);
+    }
+    queue_kernel<<<(unsigned)((T + Q_TILES - 1) / Q_TILES), Q_THREADS, 0, ctx->stream>>>(
+        T, cb.arm, cb.tile_level, bin_cnt, bin_fill, cb.qoff, cb.qtiles, ctx->d_heads);
     TC_CHECK_LAUNCH(ctx);
   }
-  uint64_t *sk = cb.qkeys0;
-  uint32_t *sv = cb.qvals0;
-  constexpr int ARM_BITS = 4;  // queue key = (arm << 40) | inverted work
-  static_assert(TC_NUM_ARMS <= (1 << ARM_BITS), "arm field of the queue key");
-  if (T > 1)
-    TC_TRY(radix_sort(ctx, cb.qkeys0, cb.qkeys1, cb.qvals0, cb.qvals1, T, 0, 40 + ARM_BITS, cb.sort_scratch, &sk, &sv));
-  if (T > 0) {
-    qoff_kernel<<<1, 32, 0, ctx->stream>>>(sk, T, cb.qoff);
-    TC_CHECK_LAUNCH(ctx);
-    arm_bytes_kernel<<<TC_NUM_ARMS, 256, 0, ctx->stream>>>(sv, cb.qoff, cb.tile_bytes, cb.arm_bytes);
-    TC_CHECK_LAUNCH(ctx);
-  }
-  TC_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_heads, 0, sizeof(unsigned) * 64, ctx->stream));
   if (cb.tile_cycles && T > 0)
     TC_CHECK_CUDA(ctx, cudaMemsetAsync(cb.tile_cycles, 0, sizeof(unsigned long long) * T, ctx->stream));
   if (timing) TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[9], ctx->stream));
+  ctx->arms_run = 0;
   for (int a = 0; a < TC_NUM_ARMS; ++a) {
-    if (T > 0 && a == TC_ARM_PULL) {
+    if (T == 0 || !arm_possible(opts, a)) continue;
+    if (a == TC_ARM_PULL) {
       TC_TRY(run_pull(ctx, g, cb, out, T, timing));
-    } else if (T > 0) {
+    } else {
       const int grid = ctx->num_sms * ctx->arm_blocks_per_sm[a];
-      arm_kernel(a)<<<grid, arm_threads(a), arm_smem(a), ctx->stream>>>(g, sv, cb.qoff, a, ctx->d_heads + a, out,
+      arm_kernel(a)<<<grid, arm_threads(a), arm_smem(a), ctx->stream>>>(g, cb.qtiles, cb.qoff, a, ctx->d_heads + a, out,
                                                                         ctx->d_total, cb.tile_cycles);
       TC_CHECK_LAUNCH(ctx);
     }
+    ctx->arms_run |= 1u << a;
     if (timing) TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[10 + a], ctx->stream));
   }
   TC_CHECK_CUDA(ctx, cudaMemcpyAsync(&ctx->h_pinned[PIN_QOFF], cb.qoff, sizeof(int64_t) * (TC_NUM_ARMS + 1),
@@ -2578,8 +2654,13 @@ void count_stats(tc_ctx *ctx, tc_stats *st, bool timing) {
     ctx->pull_timed = false;
   }
   st->ms_plan = ev_ms(ctx->ev[8], ctx->ev[9]);
-  st->ms_count = ev_ms(ctx->ev[9], ctx->ev[10 + TC_NUM_ARMS - 1]);
-  for (int a = 0; a < TC_NUM_ARMS; ++a) st->ms_arm[a] = ev_ms(ctx->ev[a == 0 ? 9 : 9 + a], ctx->ev[10 + a]);
+  int last = 9;  // event at the end of the previous arm that ran
+  for (int a = 0; a < TC_NUM_ARMS; ++a) {
+    if (!(ctx->arms_run >> a & 1u)) continue;
+    st->ms_arm[a] = ev_ms(ctx->ev[last], ctx->ev[10 + a]);
+    last = 10 + a;
+  }
+  if (last != 9) st->ms_count = ev_ms(ctx->ev[9], ctx->ev[last]);
 }
 
 }  // namespace tc

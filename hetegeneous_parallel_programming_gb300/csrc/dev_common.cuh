@@ -35,6 +35,7 @@ struct tc_ctx {
   // [10 + a] end of arm a's kernel, [10 + TC_NUM_ARMS] and [11 + TC_NUM_ARMS]
   // around the PULL arm's probing kernel (pull_kernel) alone
   cudaEvent_t ev[12 + TC_NUM_ARMS] = {};
+  unsigned arms_run = 0;                  // arms launched by this call (bit a: arm a)
   bool pull_timed = false;                // the pull_kernel events belong to this call
   // host input of tc_count: the column array is uploaded in pieces on a
   // second stream while the orientation starts (one event per piece)

@@ -108,13 +108,13 @@ tc_status launch_shift_rowptr(tc_ctx *ctx, const int64_t *rowptr, int64_t n, int
 // Counting.
 struct CountBufs {
   float *features;        // [T][TC_MLP_FEATURES]
-  uint64_t *qkeys0, *qkeys1;  // [T]
-  uint32_t *qvals0, *qvals1;  // [T]
+  uint32_t *tile_level;   // [T] work level of each tile (queue order inside an arm)
+  uint32_t *qtiles;       // [T] tiles by arm, heaviest first
   int32_t *arm;           // [T]
   int64_t *qoff;          // [TC_NUM_ARMS+1]
   unsigned long long *tile_cycles;  // [T] (optional)
   unsigned long long *tile_bytes;   // [T] algorithmic bytes per tile
-  unsigned long long *arm_bytes;    // [TC_NUM_ARMS]
+  unsigned long long *arm_bytes;    // [TC_NUM_ARMS], then the queue bins' counts and fills
   uint32_t *pull_pos;     // [keys+1] PULL grouping: key counts, then group offsets
   uint2 *pull_er;         // [m] PULL grouping: (edge id, row) grouped by key (source block, target)
   uint4 *hub_bits;        // [hub rows][hub words / 4] PULL dense edges: bit rows of the hubs' out-lists

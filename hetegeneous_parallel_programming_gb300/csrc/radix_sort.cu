@@ -10,6 +10,8 @@
 // lanes own consecutive items of a round.
 #include <stdarg.h>
 
+#include <algorithm>
+
 #include "dev_common.cuh"
 
 namespace tc {
@@ -77,9 +79,12 @@ static RsGeom rs_geom(const tc_ctx *ctx, int64_t N) {
   return g;
 }
 
+// Scratch sizes hold for every N up to the one given: a smaller N can take
+// more blocks (its chunks are smaller), up to one per tile or the grid's cap.
 size_t radix_sort_scratch_bytes(const tc_ctx *ctx, int64_t N) {
-  RsGeom g = rs_geom(ctx, N);
-  return align_up((size_t)256 * g.G * sizeof(uint32_t), 256) + align_up((size_t)256 * g.G * sizeof(uint64_t), 256);
+  const int64_t G = std::max<int64_t>(
+      1, std::min<int64_t>((N + RS_TILE - 1) / RS_TILE, (int64_t)ctx->num_sms * RS_BLOCKS_PER_SM));
+  return align_up((size_t)256 * G * sizeof(uint32_t), 256) + align_up((size_t)256 * G * sizeof(uint64_t), 256);
 }
 
 __global__ void __launch_bounds__(RS_THREADS) rs_hist_kernel(const uint64_t *__restrict__ keys, int64_t N, int shift,
@@ -249,11 +254,12 @@ tc_status radix_sort(tc_ctx *ctx, uint64_t *k0, uint64_t *k1, uint32_t *v0, uint
 constexpr int SC_THREADS = 256;
 constexpr int SC_IPT = 8;
 constexpr int SC_TILE = SC_THREADS * SC_IPT;
+constexpr int SC_BLOCKS_PER_SM = 4;
 
 static RsGeom sc_geom(const tc_ctx *ctx, int64_t N) {
   RsGeom g;
   int64_t tiles = (N + SC_TILE - 1) / SC_TILE;
-  int64_t G = (int64_t)ctx->num_sms * 4;
+  int64_t G = (int64_t)ctx->num_sms * SC_BLOCKS_PER_SM;
   if (G > tiles) G = tiles;
   if (G < 1) G = 1;
   g.chunk = ((tiles + G - 1) / G) * SC_TILE;
@@ -263,8 +269,9 @@ static RsGeom sc_geom(const tc_ctx *ctx, int64_t N) {
 }
 
 size_t scan_scratch_bytes(const tc_ctx *ctx, int64_t N) {
-  RsGeom g = sc_geom(ctx, N);
-  return align_up((size_t)(g.G + 1) * sizeof(int64_t), 256);
+  const int64_t G = std::max<int64_t>(
+      1, std::min<int64_t>((N + SC_TILE - 1) / SC_TILE, (int64_t)ctx->num_sms * SC_BLOCKS_PER_SM));
+  return align_up((size_t)(G + 1) * sizeof(int64_t), 256);
 }
 
 template <typename T>
