@@ -527,6 +527,56 @@ tc_status tc_ctx_sync(tc_ctx *ctx) {
   return TC_OK;
 }
 
+// A small graph's call (direct_fits): input to the device, direct count.
+// The caller's buffers are in the memory kind of g->on_device.  *declined:
+// nothing was counted, the general path has to.
+static tc_status count_direct(tc_ctx *ctx, const tc_csr *g, DirectReq rq, uint64_t *total, uint32_t *edge_counts,
+                              uint64_t *vertex_counts, const uint8_t *labels, tc_stats *stats, bool *declined) {
+  ctx->launches = 0;
+  tc_stats st;
+  memset(&st, 0, sizeof(st));
+  Sizer sz;
+  rq.vertex_counts = reinterpret_cast<unsigned long long *>(vertex_counts);
+  direct_sizes(ctx, g->n, g->nnz, rq, sz);
+  if (!g->on_device) {
+    sz.take<int64_t>(g->n + 1);
+    sz.take<int32_t>(g->nnz);
+    if (edge_counts) sz.take<uint32_t>(g->nnz);
+    if (vertex_counts) sz.take<unsigned long long>(g->n);
+    if (labels) sz.take<uint8_t>(g->n);
+  }
+  TC_TRY(arena_reserve(ctx, sz.used));
+  Bump bump{ctx->arena, ctx->arena_cap};
+  TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
+  DevCSR d;
+  TC_TRY(stage_csr(ctx, g, bump, d, &st.h2d_bytes));
+  rq.edge_counts = edge_counts;
+  rq.labels = labels;
+  if (!g->on_device) {
+    if (edge_counts) {
+      rq.edge_host = edge_counts;
+      rq.edge_counts = bump.take<uint32_t>(g->nnz);
+    }
+    if (vertex_counts) {
+      rq.vertex_host = vertex_counts;
+      rq.vertex_counts = bump.take<unsigned long long>(g->n);
+    }
+    if (labels) {
+      uint8_t *tmp = bump.take<uint8_t>(g->n);
+      if (bump.overflow) return set_error(ctx, TC_ERR_OOM, "arena overflow");
+      TC_CHECK_CUDA(ctx, cudaMemcpyAsync(tmp, labels, (size_t)g->n, cudaMemcpyHostToDevice, ctx->stream));
+      st.h2d_bytes += (uint64_t)g->n;
+      rq.labels = tmp;
+    }
+    if (bump.overflow) return set_error(ctx, TC_ERR_OOM, "arena overflow");
+  }
+  TC_TRY(direct_run(ctx, d, rq, bump, &st, declined));
+  if (*declined) return TC_OK;
+  *total = ctx->h_pinned[0];
+  if (stats) *stats = st;
+  return TC_OK;
+}
+
 tc_status tc_count(tc_ctx *ctx, const tc_csr *g, const tc_opts *opts_in, uint64_t *total, uint32_t *edge_counts,
                    int64_t edge_capacity, tc_stats *stats) {
   if (!ctx || !total) return set_error(ctx, TC_ERR_INVALID_ARG, "null ctx or total");
@@ -535,6 +585,13 @@ tc_status tc_count(tc_ctx *ctx, const tc_csr *g, const tc_opts *opts_in, uint64_
   tc_opts_default(&o);
   if (opts_in) o = *opts_in;
   TC_CHECK_CUDA(ctx, cudaSetDevice(ctx->device));
+  if (direct_fits(g->n, g->nnz, o)) {
+    DirectReq rq;
+    rq.cap = edge_capacity;
+    bool declined = false;
+    const tc_status s = count_direct(ctx, g, rq, total, edge_counts, nullptr, nullptr, stats, &declined);
+    if (!declined) return s;
+  }
   ctx->launches = 0;
   tc_stats st;
   memset(&st, 0, sizeof(st));
@@ -622,9 +679,18 @@ tc_status tc_count_labelled(tc_ctx *ctx, const tc_csr *g, const uint8_t *vertex_
   tc_opts o;
   tc_opts_default(&o);
   if (opts_in) o = *opts_in;
+  TC_CHECK_CUDA(ctx, cudaSetDevice(ctx->device));
+  o.selector = TC_SELECT_FIXED;  // the caller's selector is ignored
+  if (direct_fits(g->n, g->nnz, o)) {
+    DirectReq rq;
+    rq.cap = edge_capacity;
+    rq.label = label;
+    bool declined = false;
+    const tc_status s = count_direct(ctx, g, rq, total, edge_counts, nullptr, vertex_labels, stats, &declined);
+    if (!declined) return s;
+  }
   o.selector = TC_SELECT_FORCE;  // only the PULL arm filters hits by label
   o.force_arm = TC_ARM_PULL;
-  TC_CHECK_CUDA(ctx, cudaSetDevice(ctx->device));
   ctx->launches = 0;
   tc_stats st;
   memset(&st, 0, sizeof(st));
@@ -711,9 +777,15 @@ tc_status tc_count_vertices(tc_ctx *ctx, const tc_csr *g, const tc_opts *opts_in
   tc_opts o;
   tc_opts_default(&o);
   if (opts_in) o = *opts_in;
+  TC_CHECK_CUDA(ctx, cudaSetDevice(ctx->device));
+  o.selector = TC_SELECT_FIXED;  // the caller's selector is ignored
+  if (direct_fits(g->n, g->nnz, o)) {
+    bool declined = false;
+    const tc_status s = count_direct(ctx, g, DirectReq(), total, nullptr, vertex_counts, nullptr, stats, &declined);
+    if (!declined) return s;
+  }
   o.selector = TC_SELECT_FORCE;  // only the PULL arm attributes the top edge of a triangle
   o.force_arm = TC_ARM_PULL;
-  TC_CHECK_CUDA(ctx, cudaSetDevice(ctx->device));
   ctx->launches = 0;
   tc_stats st;
   memset(&st, 0, sizeof(st));
@@ -812,10 +884,21 @@ static tc_status count_dag_impl(tc_ctx *ctx, const tc_csr *dag_in, const tc_opts
   // The counted edges: all of them, or the entries of a row range
   // [e0, e1) = [rowptr[row_begin], rowptr[row_end]).
   int64_t e0 = 0, e1 = m;
+  if (rr && (rr->row_begin < 0 || rr->row_begin > rr->row_end || rr->row_end > dag_in->n))
+    return set_error(ctx, TC_ERR_INVALID_ARG, "row range [%lld, %lld) outside [0, %lld]", (long long)rr->row_begin,
+                     (long long)rr->row_end, (long long)dag_in->n);
+  if (!pr && direct_fits(dag_in->n, m, o)) {  // reads the range's row pointers on the device
+    DirectReq rq;
+    rq.orient = false;
+    rq.row_begin = rr ? rr->row_begin : 0;
+    rq.row_end = rr ? rr->row_end : dag_in->n;
+    rq.cap = edge_capacity;
+    bool declined = false;
+    const tc_status s = count_direct(ctx, dag_in, rq, total, edge_counts, nullptr, nullptr, stats, &declined);
+    if (!declined) return s;
+    ctx->launches = 0;
+  }
   if (rr) {
-    if (rr->row_begin < 0 || rr->row_begin > rr->row_end || rr->row_end > dag_in->n)
-      return set_error(ctx, TC_ERR_INVALID_ARG, "row range [%lld, %lld) outside [0, %lld]", (long long)rr->row_begin,
-                       (long long)rr->row_end, (long long)dag_in->n);
     if (dag_in->on_device) {
       TC_CHECK_CUDA(ctx, cudaMemcpy(&e0, dag_in->rowptr + rr->row_begin, sizeof(int64_t), cudaMemcpyDeviceToHost));
       TC_CHECK_CUDA(ctx, cudaMemcpy(&e1, dag_in->rowptr + rr->row_end, sizeof(int64_t), cudaMemcpyDeviceToHost));

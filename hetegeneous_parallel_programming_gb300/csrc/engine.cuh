@@ -141,6 +141,26 @@ tc_status count_carve(const tc_ctx *ctx, int64_t n, int64_t m, Bump &bump, Count
 tc_status run_count(tc_ctx *ctx, const DevDag &dag, const tc_opts &opts, CountBufs &cb, uint32_t *out, bool timing);
 void count_stats(tc_ctx *ctx, tc_stats *st, bool timing);
 
+// Direct counting of small graphs (direct.cu): no relabelling, no grouping,
+// one host read at the end.  Validated input only.
+struct DirectReq {
+  bool orient = true;                  // false: the graph is an oriented one
+  int64_t row_begin = 0, row_end = 0;  // counted rows of an oriented graph
+  uint32_t *edge_counts = nullptr;     // device, cap entries
+  int64_t cap = 0;
+  uint32_t *edge_host = nullptr;       // host copy of edge_counts
+  unsigned long long *vertex_counts = nullptr;  // device, n entries
+  uint64_t *vertex_host = nullptr;
+  const uint8_t *labels = nullptr;     // device, input ids
+  int label = 0;
+};
+bool direct_fits(int64_t n, int64_t nnz, const tc_opts &o);
+void direct_sizes(const tc_ctx *ctx, int64_t n, int64_t nnz, const DirectReq &rq, Sizer &sz);
+// Leaves the total in ctx->h_pinned[0] and fills st (its h2d fields are the
+// caller's); the ctx's event 0 marks the call's start.  *declined: the lists
+// are too long for it, nothing was counted.
+tc_status direct_run(tc_ctx *ctx, const DevCSR &d, const DirectReq &rq, Bump &bump, tc_stats *st, bool *declined);
+
 // Shared by the entry points (capi.cu, batch.cu).
 // pieces > 1 (host input only): rowptr is copied on the ctx stream, the
 // column array in `pieces` uploads on ctx->copy_stream, each recording

@@ -1,0 +1,100 @@
+"""Direct counting of small graphs (csrc/direct.cu): validated calls with the
+fixed selector below its size limits.  Counts are whole numbers, so every
+comparison is for equality."""
+import numpy as np
+import pytest
+
+import hetegeneous_parallel_programming_gb300 as tc
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def engine():
+    with tc.Engine(0) as eng:
+        yield eng
+
+
+def csr_of(n, s, d):
+    return oracle.csr_from_edges(n, np.asarray(s, np.int32), np.asarray(d, np.int32))
+
+
+def rmat(scale, degree, seed=1):
+    return csr_of(*tc.gen_edges_host(tc.GenSpec("rmat", scale=scale, edge_factor=degree / 2, seed=seed)))
+
+
+def path_with_rows(entries, n):
+    """`entries` (even) adjacency entries: a path, so the last 32-entry group and 1024-entry block are ragged."""
+    k = entries // 2
+    return csr_of(n, np.arange(k), np.arange(1, k + 1))
+
+
+def clique(k, n, first):
+    i, j = np.triu_indices(k, 1)
+    return csr_of(n, i + first, j + first)
+
+
+CASES = {
+    "no_edges": lambda: csr_of(40, [], []),
+    "one_edge_last_ids": lambda: csr_of(70000, [69998], [69999]),
+    "path_1022": lambda: path_with_rows(1022, 600),
+    "path_1024": lambda: path_with_rows(1024, 600),
+    "path_1026_many_empty_rows": lambda: path_with_rows(1026, 200000),
+    "star_and_rim": lambda: csr_of(5000, [0] * 4999 + list(range(1, 4999)), list(range(1, 5000)) + list(range(2, 5000))),
+    "clique_ends_16384": lambda: clique(130, 16384, 16384 - 130),
+    "clique_ends_16385": lambda: clique(130, 16385, 16385 - 130),
+    "clique_ends_65536": lambda: clique(70, 65536, 65536 - 70),
+    "clique_across_65536": lambda: clique(300, 65700, 65700 - 300),
+    "rmat_13_degree_60": lambda: rmat(13, 60),
+    "rmat_17_degree_6": lambda: rmat(17, 6),
+    "chung_lu_130k": lambda: csr_of(*tc.gen_edges_host(tc.GenSpec("chung_lu", n=130001, avg_degree=9, seed=2))),
+    "declined_clique_1300": lambda: clique(1300, 1300, 0),  # lists longer than the limit: the general path counts
+}
+
+
+@pytest.mark.parametrize("name", CASES)
+def test_direct_counts(engine, name):
+    rowptr, colidx = CASES[name]()
+    n = len(rowptr) - 1
+    total, per_edge, orow, ocol = oracle.triangles(rowptr, colidx, per_edge=True)
+    got, pe, st = engine.count(rowptr, colidx, edge_counts=True)
+    assert got == total and np.array_equal(pe, per_edge) and st["m"] == len(ocol)
+    assert engine.count(rowptr, colidx)[0] == total
+    gen, gpe, _ = engine.count(rowptr, colidx, edge_counts=True, validate=False)  # the general path
+    assert gen == total and np.array_equal(gpe, pe)
+    src = np.repeat(np.arange(n), np.diff(orow))
+    got, pv, _ = engine.count_vertices(rowptr, colidx)
+    gen, gpv, _ = engine.count_vertices(rowptr, colidx, validate=False)
+    assert got == gen == total and np.array_equal(pv, gpv) and int(pv.sum()) == 3 * total
+    labels = (np.arange(n) * 7 % 3).astype(np.uint8)
+    for lab in (0, 2):
+        a, ape, _ = engine.count_labelled(rowptr, colidx, labels, lab, edge_counts=True)
+        b, bpe, _ = engine.count_labelled(rowptr, colidx, labels, lab, edge_counts=True, validate=False)
+        assert a == b and np.array_equal(ape, bpe)
+    got, pe, _ = engine.count_dag(orow, ocol, edge_counts=True)
+    assert got == total and np.array_equal(pe, per_edge)
+    for lo, hi in ((0, n), (n // 3, n - n // 4), (n // 2, n // 2)):
+        got, pe, st = engine.count_dag_range(orow, ocol, lo, hi, edge_counts=True)
+        assert st["m"] == orow[hi] - orow[lo]
+        assert np.array_equal(pe, per_edge[orow[lo]:orow[hi]]) and got == int(per_edge[orow[lo]:orow[hi]].sum())
+    assert len(src) == len(ocol)
+
+
+def test_direct_refuses_what_the_general_path_refuses(engine):
+    rowptr, colidx = rmat(9, 12)
+    row = int(np.argmax(np.diff(rowptr)))
+    a = int(rowptr[row])
+    bad_id, loop, unsorted, dup = (colidx.copy() for _ in range(4))
+    bad_id[-1] = len(rowptr) - 1
+    loop[a] = row
+    unsorted[a], unsorted[a + 1] = colidx[a + 1], colidx[a]
+    dup[a + 1] = dup[a]
+    bad_row = rowptr.copy()
+    bad_row[5] = bad_row[6] + 3
+    for r, c in ((rowptr, bad_id), (rowptr, loop), (rowptr, unsorted), (rowptr, dup), (bad_row, colidx)):
+        for call in (engine.count, engine.count_vertices, engine.count_dag):
+            with pytest.raises(tc.TCError) as e:
+                call(r, c)
+            assert e.value.status == 2
+    assert engine.count(rowptr, colidx)[0] == oracle.triangles(rowptr, colidx)
