@@ -83,6 +83,42 @@ tc_status tc_batch_count(tc_ctx *ctx, const tc_batch *b, const tc_opts *opts_in,
   }
   if (nnz < 0 || nnz >= (int64_t(1) << 32) || (nnz > 0 && !b->colidx))
     return set_error(ctx, TC_ERR_UNSUPPORTED, "batch nnz=%lld outside [0, 2^32)", (long long)nnz);
+  // the batch's arrays on the device, copies where they are the host's
+  DevCSR d;  // local column ids: the passes add each row's graph base
+  d.n = n;
+  d.nnz = nnz;
+  const int64_t *d_off = b->vtx_off;
+  auto stage = [&](Bump &bump) -> tc_status {
+    d.rowptr = b->rowptr;
+    d.col = b->colidx;
+    if (b->on_device) return TC_OK;
+    int64_t *o1 = bump.take<int64_t>(G + 1), *r1 = bump.take<int64_t>(n + 1);
+    int32_t *c1 = bump.take<int32_t>(nnz);
+    if (bump.overflow) return set_error(ctx, TC_ERR_OOM, "arena overflow");
+    TC_CHECK_CUDA(ctx, cudaMemcpyAsync(o1, b->vtx_off, sizeof(int64_t) * (G + 1), cudaMemcpyHostToDevice, ctx->stream));
+    TC_CHECK_CUDA(ctx, cudaMemcpyAsync(r1, b->rowptr, sizeof(int64_t) * (n + 1), cudaMemcpyHostToDevice, ctx->stream));
+    if (nnz > 0)
+      TC_CHECK_CUDA(ctx, cudaMemcpyAsync(c1, b->colidx, sizeof(int32_t) * nnz, cudaMemcpyHostToDevice, ctx->stream));
+    st.h2d_bytes = sizeof(int64_t) * (G + 1 + n + 1) + sizeof(int32_t) * nnz;
+    d_off = o1;
+    d.rowptr = r1;
+    d.col = c1;
+    return TC_OK;
+  };
+  if (direct_batch_fits(nnz, o)) {
+    Sizer sz;
+    if (!b->on_device) { sz.take<int64_t>(G + 1); sz.take<int64_t>(n + 1); sz.take<int32_t>(nnz); }
+    direct_batch_sizes(ctx, G, n, nnz, sz);
+    TC_TRY(arena_reserve(ctx, sz.used));
+    Bump bump{ctx->arena, ctx->arena_cap};
+    TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
+    TC_TRY(stage(bump));
+    bool declined = false;
+    const tc_status s = direct_batch(ctx, d, d_off, G, bump, totals, &st, &declined);
+    if (s == TC_OK && !declined && stats) *stats = st;
+    if (!declined) return s;
+    ctx->launches = 0;
+  }
   const int gbits = bit_width_u64((uint64_t)(G > 1 ? G - 1 : 1));
   Sizer sz;
   if (!b->on_device) { sz.take<int64_t>(G + 1); sz.take<int64_t>(n + 1); sz.take<int32_t>(nnz); }
@@ -94,21 +130,9 @@ tc_status tc_batch_count(tc_ctx *ctx, const tc_batch *b, const tc_opts *opts_in,
   TC_TRY(arena_reserve(ctx, sz.used));
   Bump bump{ctx->arena, ctx->arena_cap};
   TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
-  const int64_t *d_off = b->vtx_off, *d_row = b->rowptr;
-  const int32_t *d_col = b->colidx;
-  if (!b->on_device) {
-    int64_t *o1 = bump.take<int64_t>(G + 1), *r1 = bump.take<int64_t>(n + 1);
-    int32_t *c1 = bump.take<int32_t>(nnz);
-    if (bump.overflow) return set_error(ctx, TC_ERR_OOM, "arena overflow");
-    TC_CHECK_CUDA(ctx, cudaMemcpyAsync(o1, b->vtx_off, sizeof(int64_t) * (G + 1), cudaMemcpyHostToDevice, ctx->stream));
-    TC_CHECK_CUDA(ctx, cudaMemcpyAsync(r1, b->rowptr, sizeof(int64_t) * (n + 1), cudaMemcpyHostToDevice, ctx->stream));
-    if (nnz > 0)
-      TC_CHECK_CUDA(ctx, cudaMemcpyAsync(c1, b->colidx, sizeof(int32_t) * nnz, cudaMemcpyHostToDevice, ctx->stream));
-    st.h2d_bytes = sizeof(int64_t) * (G + 1 + n + 1) + sizeof(int32_t) * nnz;
-    d_off = o1;
-    d_row = r1;
-    d_col = c1;
-  }
+  TC_TRY(stage(bump));
+  const int64_t *d_row = d.rowptr;
+  const int32_t *d_col = d.col;
   int32_t *vgroup = bump.take<int32_t>(n);
   OrientBufs ob;
   orient_carve(ctx, n, nnz, false, false, bump, ob);
@@ -120,11 +144,6 @@ tc_status tc_batch_count(tc_ctx *ctx, const tc_batch *b, const tc_opts *opts_in,
   uint32_t *cnt = bump.take<uint32_t>(nnz);
   unsigned long long *d_tot = bump.take<unsigned long long>(G);
   if (bump.overflow) return set_error(ctx, TC_ERR_OOM, "arena overflow");
-  DevCSR d;  // local column ids: the kept-count pass adds each row's graph base (ob.vtx_off)
-  d.n = n;
-  d.nnz = nnz;
-  d.rowptr = d_row;
-  d.col = d_col;
   // Front half (graph ids, validation, rank sort, kept counts, scans and the
   // queued copies of m and the flags), replayed as a CUDA graph when the
   // batch shape and buffers repeat; the host then reads m and the flags.

@@ -486,6 +486,7 @@ tc_status tc_ctx_create(int device, tc_ctx **out) {
     return fail(set_error(nullptr, TC_ERR_OOM, "ctx state allocation failed"));
   }
   tc_status st = init_arm_occupancy(ctx);
+  if (st == TC_OK) st = direct_init(ctx);
   if (st != TC_OK) return fail(st);
   *out = ctx;
   return TC_OK;

@@ -154,12 +154,19 @@ struct DirectReq {
   const uint8_t *labels = nullptr;     // device, input ids
   int label = 0;
 };
+tc_status direct_init(tc_ctx *ctx);  // once per ctx
 bool direct_fits(int64_t n, int64_t nnz, const tc_opts &o);
 void direct_sizes(const tc_ctx *ctx, int64_t n, int64_t nnz, const DirectReq &rq, Sizer &sz);
 // Leaves the total in ctx->h_pinned[0] and fills st (its h2d fields are the
 // caller's); the ctx's event 0 marks the call's start.  *declined: the lists
 // are too long for it, nothing was counted.
 tc_status direct_run(tc_ctx *ctx, const DevCSR &d, const DirectReq &rq, Bump &bump, tc_stats *st, bool *declined);
+
+// The same for a batch (column ids local to each graph), totals in host memory.
+bool direct_batch_fits(int64_t nnz, const tc_opts &o);
+void direct_batch_sizes(const tc_ctx *ctx, int64_t G, int64_t n, int64_t nnz, Sizer &sz);
+tc_status direct_batch(tc_ctx *ctx, const DevCSR &d, const int64_t *vtx_off, int64_t G, Bump &bump, uint64_t *totals,
+                       tc_stats *st, bool *declined);
 
 // Shared by the entry points (capi.cu, batch.cu).
 // pieces > 1 (host input only): rowptr is copied on the ctx stream, the

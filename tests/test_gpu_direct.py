@@ -98,3 +98,41 @@ def test_direct_refuses_what_the_general_path_refuses(engine):
                 call(r, c)
             assert e.value.status == 2
     assert engine.count(rowptr, colidx)[0] == oracle.triangles(rowptr, colidx)
+
+
+@pytest.mark.parametrize("sizes", [
+    [1], [3, 1, 2], [40] * 70, [16384, 5, 16384], [16385, 900], [32769, 64, 2], [65536, 65537, 300], [70000, 1, 1, 9]])
+def test_direct_batches(engine, sizes):
+    """Batches of graphs around the bitmap widths (16384, 32768, 65536 ids), with empty and one-vertex
+    graphs, edges of several graphs in one group of 32, and cliques on the last ids of each graph."""
+    rowptr, colidx, off, want = [np.zeros(1, np.int64)], [], [0], []
+    for i, n in enumerate(sizes):
+        k = min(n, 11 + 17 * (i % 3))
+        s, d = np.triu_indices(k, 1)
+        s, d = list(s + n - k), list(d + n - k)
+        s += list(range(0, n - 1, 1 + i % 4))
+        d += [x + 1 for x in range(0, n - 1, 1 + i % 4)]
+        r, c = csr_of(n, s, d)
+        want.append(oracle.triangles(r, c))
+        rowptr.append(r[1:] + rowptr[-1][-1])
+        colidx.append(c)
+        off.append(off[-1] + n)
+    rowptr, colidx = np.concatenate(rowptr), np.concatenate(colidx)
+    got, st = engine.batch_count(np.array(off), rowptr, colidx)
+    assert got.tolist() == want and st["m"] == len(colidx) // 2
+    assert engine.batch_count(np.array(off), rowptr, colidx, validate=False)[0].tolist() == want
+    if len(colidx) > 2:
+        bad = colidx.copy()
+        bad[-1] = sizes[-1]  # outside its graph
+        with pytest.raises(tc.TCError) as e:
+            engine.batch_count(np.array(off), rowptr, bad)
+        assert e.value.status == 2
+
+
+def test_direct_batch_declines_long_lists(engine):
+    """Complete graphs have lists longer than the limit per entry: the general path counts them."""
+    k, graphs = 700, 3
+    r, c = clique(k, k, 0)
+    rowptr = np.concatenate([[0]] + [r[1:] + g * r[-1] for g in range(graphs)])
+    got, _ = engine.batch_count(np.arange(graphs + 1) * k, rowptr, np.tile(c, graphs))
+    assert got.tolist() == [k * (k - 1) * (k - 2) // 6] * graphs
