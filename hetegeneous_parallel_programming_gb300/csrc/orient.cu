@@ -320,8 +320,7 @@ tc_status orient_phase_a(tc_ctx *ctx, const DevCSR &g, OrientBufs &b) {
   // Ids start in ascending order and the sort is stable, so sorting on the
   // (group, degree) bits alone yields the (group, degree, id) order.
   uint64_t *sorted = nullptr;
-  TC_TRY(radix_sort(ctx, b.vkeys0, b.vkeys1, nullptr, nullptr, g.n, bits, 2 * bits + gbits, b.sort_scratch, &sorted,
-                    nullptr));
+  TC_TRY(radix_sort(ctx, b.vkeys0, b.vkeys1, b.vkeys0, g.n, bits, 2 * bits + gbits, b.sort_scratch, &sorted));
   rank_kernel<<<grid_for(ctx, g.n, 256, 8), 256, 0, ctx->stream>>>(sorted, g.n, (1ULL << bits) - 1, b.rank);
   TC_CHECK_LAUNCH(ctx);
   TC_CHECK_CUDA(ctx, cudaMemsetAsync(b.kept, 0, sizeof(int64_t) * (size_t)(g.n + 1), ctx->stream));
