@@ -273,6 +273,7 @@ tc_status tc_plan_arms(tc_ctx *ctx, const tc_csr *g, const tc_opts *opts_in, int
   OrientBufs ob;
   orient_carve(ctx, d.n, d.nnz, false, false, bump, ob);
   CountBufs cb;
+  cb.selection_only = true;
   if (count_carve(ctx, d.n, d.nnz, bump, cb, false) != TC_OK || bump.overflow) return set_error(ctx, TC_ERR_OOM, "arena");
   int64_t m = 0;
   float a, bb;

@@ -690,8 +690,6 @@ tc_status tc_count_labelled(tc_ctx *ctx, const tc_csr *g, const uint8_t *vertex_
     const tc_status s = count_direct(ctx, g, rq, total, edge_counts, nullptr, vertex_labels, stats, &declined);
     if (!declined) return s;
   }
-  o.selector = TC_SELECT_FORCE;  // only the PULL arm filters hits by label
-  o.force_arm = TC_ARM_PULL;
   ctx->launches = 0;
   tc_stats st;
   memset(&st, 0, sizeof(st));
@@ -785,8 +783,6 @@ tc_status tc_count_vertices(tc_ctx *ctx, const tc_csr *g, const tc_opts *opts_in
     const tc_status s = count_direct(ctx, g, DirectReq(), total, nullptr, vertex_counts, nullptr, stats, &declined);
     if (!declined) return s;
   }
-  o.selector = TC_SELECT_FORCE;  // only the PULL arm attributes the top edge of a triangle
-  o.force_arm = TC_ARM_PULL;
   ctx->launches = 0;
   tc_stats st;
   memset(&st, 0, sizeof(st));

@@ -57,6 +57,7 @@ struct PlanStats {
   float mean_da, mean_db, mean_min, mean_max;
   float mean_in;  // mean DAG in-degree of the edges' targets
   float alr;  // mean |log2 ratio| of the two list lengths
+  float low_da;  // mean row suffix of the edges whose targets are not hubs (wedge tests), per edge of the tile
   float nrows, maxdr, maxwin, frac;
   float bins[6];
 };
@@ -80,6 +81,16 @@ __device__ __forceinline__ int fixed_select(const PlanStats &s) {
   // list; fitted to per-tile costs of R-MAT and of mixed small-graph batches.
   if (s.alr <= 2.5f) return TC_ARM_MPATH_2;
   return TC_ARM_BSEARCH_4;
+}
+
+// PULL tiles that the wedge tests count sooner.  A pair with a hub target costs
+// one bit (about 2 ps) and another pair a search (15 ps), against PULL's 90
+// ps an edge for grouping it plus 1 ps an entry: short suffixes of mostly hub
+// targets stay out of PULL.  One call: R-MAT scale 18 1.38 -> 1.13 ms, scale
+// 20 3.45 -> 2.79, Chung-Lu n = 2 M 4.81 -> 4.77; with 120 for 80, scale 22
+// 10.8 -> 10.95 and scale 24 53.9 -> 54.8.
+__device__ __forceinline__ bool wedge_beats_pull(const PlanStats &s) {
+  return s.mean_da <= 64.f && 14.f * s.low_da + (s.mean_da - s.low_da) < 80.f;
 }
 
 // MLP cost model (16 -> 64 -> 64 -> arms, ReLU); weights staged in shared
@@ -148,6 +159,11 @@ struct PullKeys {
   }
 };
 
+// Whether BSEARCH_4's tiles run as wedge tests (wedge_kernel), and whether they
+// and PULL's are the only ones (hits are attributed or filtered: per-vertex and
+// labelled counts).
+enum { PLAN_NO_WEDGE, PLAN_WEDGE, PLAN_ATTRIBUTE };
+
 // Work queues: tiles are counted into bins (arm, log2 of their work in
 // quarter steps, heaviest first) and scattered bin by bin, so each arm's
 // queue starts with its heaviest tiles.  A queue only needs the order to a
@@ -156,6 +172,7 @@ struct PullKeys {
 // queue and empty-arm launches of ER n = 16384 went from 300 to 100 us).
 constexpr int Q_LEVELS = 128;                       // 32 octaves of work, 4 steps each (heavier tiles share the first)
 constexpr int Q_BINS = TC_NUM_ARMS * Q_LEVELS;
+constexpr uint32_t TILE_SETTLED = 0x80000000u;      // in tile_level: not for the learned selection
 constexpr int Q_THREADS = 256;
 constexpr int Q_TILES = 1024;                       // tiles per block of queue_kernel
 static_assert(Q_BINS % Q_THREADS == 0, "each thread of a queue block scans the same number of bins");
@@ -175,7 +192,7 @@ __device__ __forceinline__ int work_level(unsigned long long work) {
 // from 547 to 350 us with this and the queues below; R-MAT scale 24, 63 569
 // tiles, from 55.76 to 54.98 ms).
 struct PlanPart {  // one warp's share of a tile
-  float sda, smin, salr, sin;
+  float sda, smin, salr, sin, slow;
   unsigned long long sdb, srow;
   unsigned bins01, bins23, bins45, nrows, maxdr, maxwin;
 };
@@ -187,7 +204,7 @@ __global__ void __launch_bounds__(PLAN_THREADS) plan_kernel(DevDag g, int64_t T,
                                                            unsigned long long *__restrict__ tile_bytes,
                                                            uint32_t *__restrict__ bin_cnt,
                                                            unsigned long long *__restrict__ arm_bytes,
-                                                           PullKeys pk, unsigned *__restrict__ pull_cnt) {
+                                                           PullKeys pk, unsigned *__restrict__ pull_cnt, int wedge) {
   __shared__ PlanPart s_part[PLAN_THREADS / 32];
   __shared__ int s_arm;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -198,7 +215,7 @@ __global__ void __launch_bounds__(PLAN_THREADS) plan_kernel(DevDag g, int64_t T,
   const int64_t t = PL_INTERLEAVE && S > 1 ? (i % S) * per + i / S : i;
   if (t >= T) return;
   const int64_t e0 = t * TILE_EDGES, e1 = min(g.m, e0 + TILE_EDGES);
-  float sda = 0, smin = 0, salr = 0, sin = 0;
+  float sda = 0, smin = 0, salr = 0, sin = 0, slow = 0;
   unsigned long long sdb = 0, srow = 0;
   unsigned bins01 = 0, bins23 = 0, bins45 = 0;  // two 16-bit counters each
   unsigned nrows = 0, maxdr = 0, maxwin = 0;
@@ -244,6 +261,7 @@ __global__ void __launch_bounds__(PLAN_THREADS) plan_kernel(DevDag g, int64_t T,
       const float da = (float)(re - a0);
       const float db = (float)dq[u].x;  // target's out-degree
       sda += da;
+      slow += (int64_t)ss[u] < pk.hub0 ? da : 0.f;
       sdb += (unsigned long long)(unsigned)dq[u].x;
       srow += (unsigned long long)(re - rb);
       const float mn = fminf(da, db);
@@ -266,6 +284,7 @@ __global__ void __launch_bounds__(PLAN_THREADS) plan_kernel(DevDag g, int64_t T,
   p.smin = warp_sum(smin);
   p.salr = warp_sum(salr);
   p.sin = warp_sum(sin);
+  p.slow = warp_sum(slow);
   p.sdb = warp_sum(sdb);
   p.srow = warp_sum(srow);
   p.bins01 = __reduce_add_sync(TC_FULL_MASK, bins01);
@@ -280,7 +299,7 @@ __global__ void __launch_bounds__(PLAN_THREADS) plan_kernel(DevDag g, int64_t T,
     p = s_part[0];
     for (int w = 1; w < PLAN_THREADS / 32; ++w) {
       const PlanPart &q = s_part[w];
-      p.sda += q.sda; p.smin += q.smin; p.salr += q.salr; p.sin += q.sin;
+      p.sda += q.sda; p.smin += q.smin; p.salr += q.salr; p.sin += q.sin; p.slow += q.slow;
       p.sdb += q.sdb; p.srow += q.srow;
       p.bins01 += q.bins01; p.bins23 += q.bins23; p.bins45 += q.bins45;
       p.nrows += q.nrows;
@@ -292,6 +311,7 @@ __global__ void __launch_bounds__(PLAN_THREADS) plan_kernel(DevDag g, int64_t T,
     st.mean_da = p.sda / ne; st.mean_db = (float)p.sdb / ne; st.mean_min = p.smin / ne;
     st.mean_max = (p.sda + (float)p.sdb - p.smin) / ne;
     st.mean_in = p.sin / ne; st.alr = p.salr / ne;
+    st.low_da = p.slow / ne;
     st.nrows = (float)p.nrows; st.maxdr = (float)p.maxdr; st.maxwin = (float)p.maxwin;
     float f[TC_MLP_FEATURES];
     f[0] = flog2p1(st.mean_da) / 16.f;
@@ -313,11 +333,13 @@ __global__ void __launch_bounds__(PLAN_THREADS) plan_kernel(DevDag g, int64_t T,
     float4 *fo = reinterpret_cast<float4 *>(feats + t * TC_MLP_FEATURES);
 #pragma unroll
     for (int k = 0; k < TC_MLP_FEATURES / 4; ++k) fo[k] = make_float4(f[4 * k], f[4 * k + 1], f[4 * k + 2], f[4 * k + 3]);
-    const int arm = selector == TC_SELECT_FORCE ? force_arm : fixed_select(st);
+    int arm = selector == TC_SELECT_FORCE ? force_arm : fixed_select(st);
+    bool settled = arm == TC_ARM_PULL;  // the learned selection keeps the PULL decision
+    if (wedge != PLAN_NO_WEDGE && (settled ? wedge_beats_pull(st) : wedge == PLAN_ATTRIBUTE)) arm = TC_ARM_BSEARCH_4;
     const int level = work_level((unsigned long long)p.sda + p.sdb);
     const unsigned long long alg = 4ull * (p.srow + p.sdb + (unsigned long long)(e1 - e0));
     arm_out[t] = arm;
-    tile_level[t] = (uint32_t)level;
+    tile_level[t] = (uint32_t)level | (settled ? TILE_SETTLED : 0u);
     tile_bytes[t] = alg;
     if (selector != TC_SELECT_LEARNED) {  // the learned selection counts its own choices
       atomicAdd(bin_cnt + arm * Q_LEVELS + level, 1u);
@@ -352,7 +374,8 @@ __global__ void __launch_bounds__(PLAN_THREADS) learned_select_kernel(int64_t T,
   const int64_t warps = (int64_t)gridDim.x * (PLAN_THREADS / 32);
   for (int64_t t = (int64_t)blockIdx.x * (PLAN_THREADS / 32) + (threadIdx.x >> 5); t < T; t += warps) {
     int arm = arm_io[t];
-    if (arm != TC_ARM_PULL) {
+    const uint32_t level = tile_level[t];
+    if (!(level & TILE_SETTLED)) {
       float f[TC_MLP_FEATURES];
 #pragma unroll
       for (int k = 0; k < TC_MLP_FEATURES; ++k) f[k] = feats[t * TC_MLP_FEATURES + k];
@@ -360,7 +383,7 @@ __global__ void __launch_bounds__(PLAN_THREADS) learned_select_kernel(int64_t T,
     }
     if (lane == 0) {
       arm_io[t] = arm;
-      atomicAdd(bin_cnt + arm * Q_LEVELS + tile_level[t], 1u);
+      atomicAdd(bin_cnt + arm * Q_LEVELS + (level & ~TILE_SETTLED), 1u);
       atomicAdd(arm_bytes + arm, tile_bytes[t]);
     }
   }
@@ -394,7 +417,7 @@ __global__ void __launch_bounds__(Q_THREADS) queue_kernel(int64_t T, const int32
   }
   const int64_t t1 = min(T, ((int64_t)blockIdx.x + 1) * Q_TILES);
   for (int64_t t = (int64_t)blockIdx.x * Q_TILES + threadIdx.x; t < t1; t += Q_THREADS) {
-    const int b = arm[t] * Q_LEVELS + (int)tile_level[t];
+    const int b = arm[t] * Q_LEVELS + (int)(tile_level[t] & ~TILE_SETTLED);
     qtiles[start[b] + atomicAdd(bin_fill + b, 1u)] = (uint32_t)t;
   }
 }
@@ -2014,12 +2037,18 @@ __device__ __forceinline__ int64_t pull_pack(const DevDag &g, const uint2 *__res
 
 // Work is taken in chunks of grouped entries that shrink from `item` to
 // `item_min` as the remaining work falls, so the last chunks end together
-// (the ctx's pull_item / pull_item_min; 512 and 128 unless tuned).
-__device__ __forceinline__ unsigned pull_next_chunk(unsigned *head, int64_t np, int64_t warps, int item,
+// (the ctx's pull_item / pull_item_min; 512 and 128 unless tuned).  A chunk of
+// a hub's long suffixes takes many times the mean, so a warp's share of what
+// is left is cut in 16 (R-MAT scale 20: this kernel 0.88 ms with a whole
+// share, 0.50 with an eighth, 0.41 with a sixteenth; scale 24, whose chunks
+// stay at `item`: 30.6, 30.7, 30.7; with a hundredth 31.3).
+// A caller's DAG (share 1) has no such order of suffixes, and its chunks pay
+// for rebuilding tables.
+__device__ __forceinline__ unsigned pull_next_chunk(unsigned *head, int64_t np, int64_t warps, int share, int item,
                                                     int item_min, int64_t *end) {
   const int64_t seen = (int64_t)*(volatile unsigned *)head;
   const int64_t left = np - seen;
-  int64_t chunk = left / warps;
+  int64_t chunk = left / (share * warps);
   chunk = chunk >= item ? item : chunk <= item_min ? item_min : chunk;
   const unsigned start = atomicAdd(head, (unsigned)chunk);
   *end = min(np, (int64_t)start + chunk);
@@ -2049,7 +2078,7 @@ __global__ void __launch_bounds__(PL_THREADS, TC_PL_MIN_BLOCKS) pull_kernel(DevD
   for (;;) {
     unsigned it = 0;
     int64_t p1 = 0;
-    if (lane == 0) it = pull_next_chunk(head, np, warps, item, item_min, &p1);
+    if (lane == 0) it = pull_next_chunk(head, np, warps, g.restrict_after ? 16 : 1, item, item_min, &p1);
     it = __shfl_sync(TC_FULL_MASK, it, 0);
     p1 = __shfl_sync(TC_FULL_MASK, (long long)p1, 0);
     if ((int64_t)it >= np) break;
@@ -2215,6 +2244,186 @@ __global__ void __launch_bounds__(PL_THREADS, TC_PL_MIN_BLOCKS) pull_kernel(DevD
   flush_total(acc, total);
 }
 
+// ---- BSEARCH_4's tiles of a relabelled graph ----------------------------------------
+//
+// Tiles of short rows with long target lists.  Where the target v is a hub,
+// every entry that can close a triangle with it is one too, so each entry w
+// after v in the row is one bit of v's hub row (hub_bits_kernel): two loads
+// deep, instead of the row pointers and the log2(d+(v)) dependent loads of a
+// search in a list of hundreds.  The other edges search the shorter list's
+// entries in the longer one.  Both are flattened over the lanes, 32 edges a
+// warp at a time, so short rows do not idle lanes.  Bound by the latency of
+// the random loads.  Against the 4-lane searches (bsearch_kernel<4>): R-MAT
+// scale 24, 24.7 M edges, 2.79 -> 1.75 ms; Chung-Lu n = 8 M, 50.7 M edges,
+// 5.06 -> 3.25 ms; scale 22 0.75 -> 0.44 ms.
+constexpr int WD_THREADS = 256;
+constexpr int WD_WARPS = WD_THREADS / 32;
+constexpr int WD_U = 4;                   // loads or searches in flight per lane
+constexpr int64_t WD_MIN_TILES = 1024;    // without PULL tiles, fewer do not pay for building the bit rows
+
+// Whether the hub bit rows are built: some tile is PULL's, or BSEARCH_4 has many.
+__device__ __forceinline__ bool hub_bits_used(const int64_t *__restrict__ qoff) {
+  return qoff[TC_ARM_PULL + 1] > qoff[TC_ARM_PULL] ||
+         qoff[TC_ARM_BSEARCH_4 + 1] - qoff[TC_ARM_BSEARCH_4] >= WD_MIN_TILES;
+}
+
+// MODE as for pull_kernel.
+template <int MODE>
+__global__ void __launch_bounds__(WD_THREADS, 4) wedge_kernel(DevDag g, int32_t hub0,
+                                                             const uint32_t *__restrict__ qtiles,
+                                                             const int64_t *__restrict__ qoff, unsigned *head,
+                                                             uint32_t *out, unsigned long long *total) {
+  __shared__ int4 s_rec[WD_WARPS][32];
+  __shared__ uint32_t s_hits[WD_WARPS][32];
+  __shared__ int64_t s_tile;
+  const int64_t qb = qoff[TC_ARM_BSEARCH_4], qn = qoff[TC_ARM_BSEARCH_4 + 1] - qb;
+  const int32_t first_hub = hub_bits_used(qoff) ? hub0 : INT32_MAX;
+  const uint32_t *__restrict__ bits = reinterpret_cast<const uint32_t *>(g.hub_bits);
+  const uint32_t wpr = 4u * (uint32_t)g.hub_wpr4;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const unsigned lt = lanemask_lt();
+  int4 *rec = s_rec[w];
+  uint32_t *hits = s_hits[w];
+  const int32_t *__restrict__ col = g.col;
+  unsigned long long acc = 0;
+  for (;;) {
+    int64_t tile, e0, e1;
+    if (!next_sub_tile(qtiles, qb, qn, head, &s_tile, g.m, &tile, &e0, &e1)) break;
+    for (int64_t f = e0 + 32 * w; f < e1; f += WD_THREADS) {
+      const int64_t e = f + lane;
+      const bool in = e < e1;
+      const int32_t v = in ? __ldg(col + e) : 0;
+      const uint32_t na = in ? (uint32_t)(g.rowptr[__ldg(g.src + e) + 1] - e - 1) : 0u;  // entries after v in the row
+      const bool hub = na > 0 && v >= first_hub;
+      const bool search = na > 0 && !hub;
+      uint32_t b0 = 0, nb = 0;
+      if (search) {
+        b0 = (uint32_t)g.rowptr[v];
+        nb = (uint32_t)g.rowptr[v + 1] - b0;
+      }
+      if (out) hits[lane] = 0u;
+      // hub targets: (edge, entry) pairs
+      uint32_t incl = hub ? na : 0u;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(TC_FULL_MASK, incl, o);
+        if (lane >= o) incl += y;
+      }
+      uint32_t tot = __shfl_sync(TC_FULL_MASK, incl, 31), excl = incl - (hub ? na : 0u);
+      unsigned full = __ballot_sync(TC_FULL_MASK, hub);
+      if (hub)
+        rec[__popc(full & lt)] = make_int4((int)((uint32_t)(e + 1) - excl), v - hub0, lane, 0);
+      __syncwarp();
+      int base = -1;
+      for (uint32_t i0 = 0; i0 < tot; i0 += 32 * WD_U) {
+        uint32_t d[WD_U], word[WD_U], at_u[WD_U];  // at_u: the entry's index in col
+        int row[WD_U], ce[WD_U];
+#pragma unroll
+        for (int j = 0; j < WD_U; ++j) {
+          const uint32_t i = i0 + 32 * j + lane, s = excl - (i0 + 32 * j);
+          const unsigned starts = __reduce_or_sync(TC_FULL_MASK, hub && s < 32u ? 1u << s : 0u);
+          const int at = base + __popc(starts & ((2u << lane) - 1u));
+          base += __popc(starts);
+          d[j] = at_u[j] = 0u;
+          row[j] = -1;
+          ce[j] = 0;
+          if (i < tot) {
+            const int4 r = rec[at];
+            at_u[j] = (uint32_t)r.x + i;
+            d[j] = (uint32_t)(__ldg(col + at_u[j]) - hub0);
+            row[j] = r.y;
+            ce[j] = r.z;
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < WD_U; ++j) word[j] = row[j] >= 0 ? __ldg(bits + (size_t)row[j] * wpr + (d[j] >> 5)) : 0u;
+#pragma unroll
+        for (int j = 0; j < WD_U; ++j) {
+          uint32_t hit = (word[j] >> (d[j] & 31u)) & 1u;
+          if (MODE == 2 && hit) hit = g.vlabel[hub0 + (int32_t)d[j]] == g.label;
+          if (MODE == 1 && hit) atomicAdd(g.top + at_u[j], 1u);
+          if (!out) acc += hit;
+          else if (hit) atomicAdd(hits + ce[j], 1u);
+        }
+      }
+      __syncwarp();
+      // the other targets: the shorter list's entries searched in the longer
+      full = __ballot_sync(TC_FULL_MASK, search && nb > 0);
+      if (full) {
+        const bool a_short = na <= nb, mine = search && nb > 0;
+        const uint32_t ns = mine ? (a_short ? na : nb) : 0u, a0 = (uint32_t)(e + 1);
+        incl = ns;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t y = __shfl_up_sync(TC_FULL_MASK, incl, o);
+          if (lane >= o) incl += y;
+        }
+        tot = __shfl_sync(TC_FULL_MASK, incl, 31);
+        excl = incl - ns;
+        if (mine)
+          rec[__popc(full & lt)] = make_int4((int)((a_short ? a0 : b0) - excl), (int)(a_short ? b0 : a0),
+                                             (int)(a_short ? nb : na), lane << 1 | (int)a_short);
+        __syncwarp();
+        base = -1;
+        for (uint32_t i0 = 0; i0 < tot; i0 += 32 * WD_U) {
+          int32_t key[WD_U];
+          uint32_t lo[WD_U], hi[WD_U], end[WD_U], at_k[WD_U];
+          int ce[WD_U], width = 0;
+#pragma unroll
+          for (int j = 0; j < WD_U; ++j) {
+            const uint32_t i = i0 + 32 * j + lane, s = excl - (i0 + 32 * j);
+            const unsigned starts = __reduce_or_sync(TC_FULL_MASK, mine && s < 32u ? 1u << s : 0u);
+            const int at = base + __popc(starts & ((2u << lane) - 1u));
+            base += __popc(starts);
+            key[j] = 0;
+            lo[j] = hi[j] = end[j] = at_k[j] = 0u;
+            ce[j] = 0;
+            if (i < tot) {
+              const int4 r = rec[at];
+              at_k[j] = (uint32_t)r.x + i;
+              key[j] = __ldg(col + at_k[j]);
+              lo[j] = (uint32_t)r.y;
+              hi[j] = end[j] = lo[j] + (uint32_t)r.z;
+              width = max(width, r.z);
+              ce[j] = r.w;  // edge << 1 | its row's entries are the keys
+            }
+          }
+          while (width > 0) {
+#pragma unroll
+            for (int j = 0; j < WD_U; ++j)
+              if (lo[j] < hi[j]) {
+                const uint32_t mid = lo[j] + ((hi[j] - lo[j]) >> 1);
+                if (__ldg(col + mid) < key[j]) lo[j] = mid + 1;
+                else hi[j] = mid;
+              }
+            width >>= 1;
+          }
+#pragma unroll
+          for (int j = 0; j < WD_U; ++j)
+            if (lo[j] < end[j] && __ldg(col + lo[j]) == key[j]) {
+              if (MODE == 2 && g.vlabel[key[j]] != g.label) continue;
+              // the row's own entry: the key's place, or where it was found
+              if (MODE == 1) atomicAdd(g.top + ((ce[j] & 1) ? at_k[j] : lo[j]), 1u);
+              if (!out) ++acc;
+              else atomicAdd(hits + (ce[j] >> 1), 1u);
+            }
+        }
+        __syncwarp();
+      }
+      if (out) {
+        __syncwarp();
+        if (in) {
+          const uint32_t c = hits[lane];
+          put_edge_count(g, out, e, c);
+          acc += c;
+        }
+        __syncwarp();
+      }
+    }
+  }
+  flush_total(acc, total);
+}
+
 // ---- host side ---------------------------------------------------------------------
 
 typedef void (*ArmKernel)(DevDag, const uint32_t *, const int64_t *, int, unsigned *, uint32_t *,
@@ -2346,10 +2555,10 @@ static int64_t pull_key_count(int64_t n, int64_t T, int block_tiles, PullKeys *p
 // Bit rows of the hubs' out-lists, one warp per hub row: the warp clears the
 // row, then ORs in its entries, one OR per distinct word (lanes matched by
 // word).  Every entry of a hub row is a hub (it ranks above its row).  Nothing
-// is done when no edge was grouped for the PULL arm.
-__global__ void hub_bits_kernel(DevDag g, int32_t hub0, int wpr4, const unsigned *__restrict__ npull,
+// is done when neither PULL nor the wedge tests read them (hub_bits_used).
+__global__ void hub_bits_kernel(DevDag g, int32_t hub0, int wpr4, const int64_t *__restrict__ qoff,
                                 uint4 *__restrict__ bits) {
-  if (*npull == 0) return;
+  if (!hub_bits_used(qoff)) return;
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < g.n - hub0; row += warps) {
@@ -2399,16 +2608,7 @@ static tc_status run_pull(tc_ctx *ctx, const DevDag &g_in, CountBufs &cb, uint32
                                                                      g_in.restrict_after, cb.arm, g_in.m, pk, pos,
                                                                      cb.pull_er);
   TC_CHECK_LAUNCH(ctx);
-  DevDag g = g_in;
-  // dense edges: plain and labelled counts of a relabelled DAG (rows hold
-  // higher ids only; labelled tables hold only the labelled entries)
-  if (g.restrict_after && !g.top && g.m > 0) {
-    const int32_t hub0 = (int32_t)(g.n - hub_rows(g.n));
-    hub_bits_kernel<<<ctx->num_sms * 8, 256, 0, ctx->stream>>>(g, hub0, hub_wpr4(g.n), pos + K, cb.hub_bits);
-    TC_CHECK_LAUNCH(ctx);
-    g.hub_bits = cb.hub_bits;
-    g.hub_wpr4 = hub_wpr4(g.n);
-  }
+  const DevDag &g = g_in;
   // pos[K] (no edge has key K) still holds the number of grouped edges
   const int grid = ctx->num_sms * ctx->arm_blocks_per_sm[TC_ARM_PULL];
   if (timing) {
@@ -2445,14 +2645,26 @@ static bool arm_possible(const tc_opts &opts, int a) {
          a == TC_ARM_BSEARCH_4;  // fixed_select's choices
 }
 
-tc_status run_count(tc_ctx *ctx, const DevDag &g_in, const tc_opts &opts, CountBufs &cb, uint32_t *out, bool timing) {
+tc_status run_count(tc_ctx *ctx, const DevDag &g_in, const tc_opts &opts_in, CountBufs &cb, uint32_t *out, bool timing) {
   DevDag g = g_in;
   g.flags = ctx->d_flags;
+  tc_opts opts = opts_in;
+  // only PULL and the wedge tests attribute or filter hits; recording costs
+  // leaves PULL alone
+  const bool attribute = g.top != nullptr || g.vlabel != nullptr;
+  if (attribute) {
+    opts.selector = cb.tile_cycles ? TC_SELECT_FORCE : TC_SELECT_FIXED;
+    opts.force_arm = TC_ARM_PULL;
+  }
   const int64_t T = (g.m + TILE_EDGES - 1) / TILE_EDGES;
   if (opts.selector == TC_SELECT_LEARNED && !ctx->mlp_loaded)
     return set_error(ctx, TC_ERR_INVALID_ARG, "learned selector requested but no MLP weights are loaded");
   if (opts.selector == TC_SELECT_FORCE && (opts.force_arm < 0 || opts.force_arm >= TC_NUM_ARMS))
     return set_error(ctx, TC_ERR_INVALID_ARG, "force_arm %d outside [0,%d)", opts.force_arm, TC_NUM_ARMS);
+  // forced arms and recorded costs keep each arm's own kernel
+  const int wedge = !g.restrict_after || cb.tile_cycles || cb.selection_only || opts.selector == TC_SELECT_FORCE ? PLAN_NO_WEDGE
+                    : attribute                                                             ? PLAN_ATTRIBUTE
+                                                                                            : PLAN_WEDGE;
   if (timing) TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[8], ctx->stream));
   if (T == 0) {
     TC_CHECK_CUDA(ctx, cudaMemsetAsync(cb.qoff, 0, sizeof(int64_t) * (TC_NUM_ARMS + 1), ctx->stream));
@@ -2467,7 +2679,7 @@ tc_status run_count(tc_ctx *ctx, const DevDag &g_in, const tc_opts &opts, CountB
     TC_CHECK_CUDA(ctx, cudaMemsetAsync(cb.arm_bytes, 0, sizeof(unsigned long long) * (TC_NUM_ARMS + Q_BINS), ctx->stream));
     plan_kernel<<<(unsigned)slots, PLAN_THREADS, 0, ctx->stream>>>(g, T, opts.selector, opts.force_arm, cb.features,
                                                                    cb.arm, cb.tile_level, cb.tile_bytes, bin_cnt,
-                                                                   cb.arm_bytes, pk, cb.pull_pos);
+                                                                   cb.arm_bytes, pk, cb.pull_pos, wedge);
     TC_CHECK_LAUNCH(ctx);
     if (opts.selector == TC_SELECT_LEARNED) {
       learned_select_kernel<<<grid_for(ctx, T, PLAN_THREADS / 32, 4), PLAN_THREADS, TC_MLP_PARAM_COUNT * sizeof(float),
@@ -2482,10 +2694,26 @@ tc_status run_count(tc_ctx *ctx, const DevDag &g_in, const tc_opts &opts, CountB
   if (cb.tile_cycles && T > 0)
     TC_CHECK_CUDA(ctx, cudaMemsetAsync(cb.tile_cycles, 0, sizeof(unsigned long long) * T, ctx->stream));
   if (timing) TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[9], ctx->stream));
+  // hub bit rows for PULL's dense edges (plain and labelled counts: labelled
+  // tables hold only the labelled entries) and the wedge tests of a relabelled
+  // DAG (rows hold higher ids only)
+  const int32_t hub0 = (int32_t)(g.n - hub_rows(g.n));
+  if (T > 0 && g.restrict_after && arm_possible(opts, TC_ARM_PULL) && (!g.top || wedge != PLAN_NO_WEDGE)) {
+    hub_bits_kernel<<<ctx->num_sms * 8, 256, 0, ctx->stream>>>(g, hub0, hub_wpr4(g.n), cb.qoff, cb.hub_bits);
+    TC_CHECK_LAUNCH(ctx);
+    g.hub_bits = cb.hub_bits;
+    g.hub_wpr4 = hub_wpr4(g.n);
+  }
   ctx->arms_run = 0;
   for (int a = 0; a < TC_NUM_ARMS; ++a) {
     if (T == 0 || !arm_possible(opts, a)) continue;
-    if (a == TC_ARM_PULL) {
+    if (wedge == PLAN_ATTRIBUTE && a != TC_ARM_BSEARCH_4 && a != TC_ARM_PULL) continue;
+    if (a == TC_ARM_BSEARCH_4 && wedge != PLAN_NO_WEDGE) {
+      const auto kernel = g.top ? wedge_kernel<1> : g.vlabel ? wedge_kernel<2> : wedge_kernel<0>;
+      kernel<<<ctx->num_sms * 8, WD_THREADS, 0, ctx->stream>>>(g, hub0, cb.qtiles, cb.qoff, ctx->d_heads + a, out,
+                                                               ctx->d_total);
+      TC_CHECK_LAUNCH(ctx);
+    } else if (a == TC_ARM_PULL) {
       TC_TRY(run_pull(ctx, g, cb, out, T, timing));
     } else {
       const int grid = ctx->num_sms * ctx->arm_blocks_per_sm[a];

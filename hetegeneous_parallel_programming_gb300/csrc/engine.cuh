@@ -117,6 +117,7 @@ struct CountBufs {
   unsigned long long *arm_bytes;    // [TC_NUM_ARMS], then the queue bins' counts and fills
   uint32_t *pull_pos;     // [keys+1] PULL grouping: key counts, then group offsets
   uint2 *pull_er;         // [m] PULL grouping: (edge id, row) grouped by key (source block, target)
+  bool selection_only = false;  // report the selector's arms: PULL tiles stay PULL's
   uint4 *hub_bits;        // [hub rows][hub words / 4] PULL dense edges: bit rows of the hubs' out-lists
   void *sort_scratch;
 };
