@@ -2744,13 +2744,47 @@ static float ev_ms(cudaEvent_t a, cudaEvent_t b) {
 // counts c (edge r->s is the lowest pair of c[e] triangles) and the top
 // counts (edge r->s joins the lowest and highest vertex of top[e]
 // triangles): t[r] += c[e], t[s] += c[e] + top[e]; then per input id.
-__global__ void vertex_sum_kernel(DevDag g, const uint32_t *__restrict__ c, const uint32_t *__restrict__ top,
-                                  unsigned long long *__restrict__ t) {
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < g.m; e += (int64_t)gridDim.x * blockDim.x) {
-    const uint32_t ce = c[e], te = top[e];
-    if (ce) atomicAdd(t + g.src[e], (unsigned long long)ce);
-    if (ce + te) atomicAdd(t + g.col[e], (unsigned long long)(ce + te));
+// Bound by additions that meet at one address: a row's 32 consecutive edges
+// are summed across lanes first, and the last VS_HUBS ids, the hubs that most
+// edges point to, are summed per block in shared memory (R-MAT scale 20, 15.7 M
+// edges: 130 us, 635 with an addition per edge end).
+constexpr int VS_HUBS = 4096;
+constexpr int VS_THREADS = 512;
+
+__global__ void __launch_bounds__(VS_THREADS) vertex_sum_kernel(DevDag g, const uint32_t *__restrict__ c,
+                                                               const uint32_t *__restrict__ top,
+                                                               unsigned long long *__restrict__ t) {
+  __shared__ unsigned long long s_hub[VS_HUBS];
+  const int32_t hub0 = (int32_t)(g.n > VS_HUBS ? g.n - VS_HUBS : 0);
+  for (int i = threadIdx.x; i < VS_HUBS; i += VS_THREADS) s_hub[i] = 0ull;
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  auto add = [&](int32_t v, unsigned long long x) {
+    if (v >= hub0) atomicAdd(&s_hub[v - hub0], x);
+    else atomicAdd(t + v, x);
+  };
+  const int64_t stride = (int64_t)gridDim.x * VS_THREADS;
+  for (int64_t e0 = (int64_t)blockIdx.x * VS_THREADS + threadIdx.x - lane; e0 < g.m; e0 += stride) {
+    const int64_t e = e0 + lane;
+    const bool in = e < g.m;
+    const uint32_t ce = in ? c[e] : 0u, te = in ? top[e] : 0u;
+    if (ce | te) add(g.col[e], (unsigned long long)ce + te);
+    if (!__any_sync(TC_FULL_MASK, ce != 0u)) continue;
+    // rows are runs of lanes: sums up to and with each lane, the run's in its last lane
+    const int32_t r = in ? g.src[e] : -1;
+    unsigned long long x = ce;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long y = __shfl_up_sync(TC_FULL_MASK, x, o);
+      const int32_t ry = __shfl_up_sync(TC_FULL_MASK, r, o);
+      if (lane >= o && ry == r) x += y;
+    }
+    const int32_t rn = __shfl_down_sync(TC_FULL_MASK, r, 1);
+    if (in && x && (lane == 31 || rn != r)) add(r, x);
   }
+  __syncthreads();
+  for (int i = threadIdx.x; i < VS_HUBS; i += VS_THREADS)
+    if (s_hub[i]) atomicAdd(t + hub0 + i, s_hub[i]);
 }
 
 __global__ void vertex_unrank_kernel(const unsigned long long *__restrict__ t, const int32_t *__restrict__ rank,
@@ -2776,7 +2810,7 @@ tc_status launch_vertex_sums(tc_ctx *ctx, const DevDag &g, const uint32_t *c, co
                              unsigned long long *t, const int32_t *rank, unsigned long long *out) {
   TC_CHECK_CUDA(ctx, cudaMemsetAsync(t, 0, sizeof(unsigned long long) * (size_t)g.n, ctx->stream));
   if (g.m > 0) {
-    vertex_sum_kernel<<<grid_for(ctx, g.m, 256, 8), 256, 0, ctx->stream>>>(g, c, top, t);
+    vertex_sum_kernel<<<grid_for(ctx, g.m, VS_THREADS, 3), VS_THREADS, 0, ctx->stream>>>(g, c, top, t);
     TC_CHECK_LAUNCH(ctx);
   }
   vertex_unrank_kernel<<<grid_for(ctx, g.n, 256, 8), 256, 0, ctx->stream>>>(t, rank, g.n, out);
