@@ -50,11 +50,12 @@ class Stats(C.Structure):
 
     _PER_ARM = ("tiles_per_arm", "ms_arm", "alg_bytes_arm")
 
+    _SCALARS = tuple(k for k, t in _fields_ if not issubclass(t, C.Array))
+
     def as_dict(self) -> dict:
-        d = {k: getattr(self, k) for k, _ in self._fields_ if k not in self._PER_ARM}
+        d = {k: getattr(self, k) for k in self._SCALARS}
         for k in self._PER_ARM:
-            arr = getattr(self, k)
-            d[k] = {ARM_NAMES[i]: (float(arr[i]) if k == "ms_arm" else int(arr[i])) for i in range(TC_NUM_ARMS)}
+            d[k] = dict(zip(ARM_NAMES, getattr(self, k)[:]))
         return d
 
 

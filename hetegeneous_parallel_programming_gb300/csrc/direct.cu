@@ -111,8 +111,28 @@ __device__ __forceinline__ void entry_rows(const int64_t *__restrict__ rowptr, u
   }
 }
 
-// Results of a direct call, copied to the host in one piece.
-enum { DX_TOTAL, DX_M, DX_ALG, DX_FLAGS, DX_WORK, DX_GUESS, DX_MAXN, DX_WORDS };
+// Results of a direct call, all zero at its start.  DX_DONE counts the counting
+// kernel's blocks, and the last one hands the words to the host; DX_START,
+// DX_COUNT and DX_END are the device's clock (ns) when the passes and the
+// counting start and when they end.
+enum { DX_TOTAL, DX_M, DX_ALG, DX_FLAGS, DX_WORK, DX_GUESS, DX_MAXN, DX_DONE, DX_START, DX_COUNT, DX_END, DX_WORDS };
+
+// A small graph's passes are a few microseconds each, so a kernel's launch
+// overlaps the end of the one before it (programmatic dependent launch): it
+// lets its successor be scheduled as it starts, and waits here for its
+// predecessor's results.  With the results written by the last block and no
+// events between the passes, ER n = 300 went from 56.6 to 40.5 us a call, ER n
+// = 16384 from 68 to 51.
+__device__ __forceinline__ void begin_pass() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+__device__ __forceinline__ unsigned long long clock_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
 
 // Whether the later kernels have nothing to do: invalid input, or lists too
 // long.
@@ -174,6 +194,8 @@ __global__ void __launch_bounds__(DR_THREADS) direct_rows_kernel(
   __shared__ bool s_bad;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned lt = lanemask_lt();
+  begin_pass();
+  if (blockIdx.x == 0 && threadIdx.x == 0) res[DX_START] = clock_ns();
   if (threadIdx.x == 0) {
     s_work = 0;
     s_bad = vtx_off && (unsigned)res[DX_FLAGS];  // the graphs' vertex ranges; other blocks may be adding flags
@@ -302,6 +324,7 @@ __global__ void __launch_bounds__(DR_THREADS) direct_place_kernel(
     unsigned long long max_work) {
   __shared__ uint32_t s_off[DR_SMEM_BLOCKS + 1];
   __shared__ uint32_t tmp[33];
+  begin_pass();
   if (direct_off(res, max_work)) return;
   if (!boff) {
     const int per = ((blocks + DR_THREADS - 1) / DR_THREADS) | 1;  // odd: the threads' slices start in different banks
@@ -387,12 +410,12 @@ constexpr int DC_SEARCH = 8;        // target list this many times the row's: se
 // additions to one address take turns: the warps spread them over `copies`
 // arrays of n counts.
 template <int MODE>
-__global__ void __launch_bounds__(DC_THREADS, DC_BLOCKS) direct_count_kernel(DirectDag g, uint32_t *__restrict__ out,
-                                                                 unsigned long long cap, int chunk,
-                                                                 unsigned long long *__restrict__ vcount, int copies,
-                                                                 unsigned long long *__restrict__ totals,
-                                                                 unsigned long long *__restrict__ res,
-                                                                 unsigned long long max_work) {
+__device__ __forceinline__ void direct_count_block(const DirectDag &g, uint32_t *__restrict__ out,
+                                                   unsigned long long cap, int chunk,
+                                                   unsigned long long *__restrict__ vcount, int copies,
+                                                   unsigned long long *__restrict__ totals,
+                                                   unsigned long long *__restrict__ res,
+                                                   unsigned long long max_work) {
   extern __shared__ __align__(16) uint32_t s_bm[];
   __shared__ int4 s_rec[DC_WARPS][32];
   __shared__ uint32_t s_hits[DC_WARPS][32];
@@ -673,11 +696,36 @@ __global__ void __launch_bounds__(DC_THREADS, DC_BLOCKS) direct_count_kernel(Dir
   if (threadIdx.x < 2 && s_sum[threadIdx.x]) atomicAdd(res + (threadIdx.x ? DX_ALG : DX_TOTAL), s_sum[threadIdx.x]);
 }
 
+// The last block to finish writes the results to `host` (mapped page-locked
+// memory, or null), so that the host waits for the stream and has them: a copy
+// of its own after the kernel took 6 us.
+template <int MODE>
+__global__ void __launch_bounds__(DC_THREADS, DC_BLOCKS) direct_count_kernel(
+    DirectDag g, uint32_t *__restrict__ out, unsigned long long cap, int chunk,
+    unsigned long long *__restrict__ vcount, int copies, unsigned long long *__restrict__ totals,
+    unsigned long long *res, unsigned long long max_work, volatile unsigned long long *host) {
+  __shared__ bool s_last;
+  begin_pass();
+  if (blockIdx.x == 0 && threadIdx.x == 0) res[DX_COUNT] = clock_ns();
+  direct_count_block<MODE>(g, out, cap, chunk, vcount, copies, totals, res, max_work);
+  if (!host) return;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(res + DX_DONE, 1ull) == gridDim.x - 1;
+  __syncthreads();
+  if (s_last && threadIdx.x < DX_WORDS) {
+    __threadfence();
+    host[threadIdx.x] = threadIdx.x == DX_END ? clock_ns() : __ldcg(res + threadIdx.x);
+    __threadfence_system();
+  }
+}
+
 // Sums the copies of the vertex counts.
 __global__ void __launch_bounds__(DC_THREADS) direct_vsum_kernel(const unsigned long long *__restrict__ t, int64_t n,
                                                                 int copies, unsigned long long *__restrict__ out,
                                                                 const unsigned long long *__restrict__ res,
                                                                 unsigned long long max_work) {
+  begin_pass();
   if (direct_off(res, max_work)) return;
   for (int64_t u = (int64_t)blockIdx.x * DC_THREADS + threadIdx.x; u < n; u += (int64_t)gridDim.x * DC_THREADS) {
     unsigned long long s = 0;
@@ -690,7 +738,7 @@ __global__ void __launch_bounds__(DC_THREADS) direct_vsum_kernel(const unsigned 
 
 // Which calls count directly.  Measured against the general path (us, one
 // call, whole-GPU clock; W = summed list lengths, see direct_rows_kernel):
-//   ER n = 300, 1.5 K entries       297 ->  57    ER n = 16384, degree 16  350 ->  69
+//   ER n = 300, 1.5 K entries       297 ->  41    ER n = 16384, degree 16  350 ->  51
 //   R-MAT scale 15, 0.9 M entries   940 -> 142    Chung-Lu n = 50000       974 -> 140
 //   R-MAT scale 16, degree 64, W = 0.50 G        1865 -> 487
 //   complete graph of 1500 vertices, W = 1.7 G    793 -> 835
@@ -710,6 +758,23 @@ static unsigned long long direct_max_work(int64_t n, bool per_vertex) {
   const bool exact = n <= 32 * DC_WORDS;
   if (per_vertex) return exact ? 1ull << 29 : 1ull << 27;
   return exact ? 1ull << 30 : 3ull << 27;
+}
+
+// Launches a pass that calls begin_pass.
+template <typename... P, typename... A>
+static cudaError_t launch_pass(tc_ctx *ctx, void (*kernel)(P...), int grid, int threads, int smem, A... args) {
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = ctx->stream;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  ctx->launches++;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
 tc_status direct_init(tc_ctx *ctx) {
@@ -760,14 +825,13 @@ static void set_bitmaps(DirectDag &g, int64_t n) {
 template <int MODE>
 static tc_status launch_count(tc_ctx *ctx, const DirectDag &g, int64_t edges, int chunk, const DirectReq &rq,
                               unsigned long long *vcount, int copies, unsigned long long *totals,
-                              unsigned long long *res, unsigned long long max_work) {
+                              unsigned long long *res, unsigned long long max_work, unsigned long long *host) {
   const int64_t batches = std::max<int64_t>(1, (edges + 31) / 32);
   const int smem = DC_WARPS * g.words * g.slots * (int)sizeof(uint32_t);
   const int grid = grid_for(ctx, batches, DC_WARPS, smem > 48 * 1024 ? 3 : 4);
   chunk = (int)std::max<int64_t>(1, std::min<int64_t>(chunk, batches / ((int64_t)grid * DC_WARPS)));
-  direct_count_kernel<MODE><<<grid, DC_THREADS, smem, ctx->stream>>>(g, rq.edge_counts, (unsigned long long)rq.cap,
-                                                                        chunk, vcount, copies, totals, res, max_work);
-  TC_CHECK_LAUNCH(ctx);
+  TC_CHECK_CUDA(ctx, launch_pass(ctx, direct_count_kernel<MODE>, grid, DC_THREADS, smem, g, rq.edge_counts,
+                                 (unsigned long long)rq.cap, chunk, vcount, copies, totals, res, max_work, host));
   return TC_OK;
 }
 
@@ -795,7 +859,6 @@ tc_status direct_run(tc_ctx *ctx, const DevCSR &d, const DirectReq &rq, Bump &bu
   unsigned long long *vcount = rq.vertex_counts;
   if (copies > 1) vcount = bump.take<unsigned long long>(n * copies);
   if (bump.overflow) return set_error(ctx, TC_ERR_OOM, "arena overflow");
-  TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[1], ctx->stream));
   TC_CHECK_CUDA(ctx, cudaMemsetAsync(res, 0, sizeof(unsigned long long) * DX_WORDS, ctx->stream));
   if (nnz >= DS_MIN_NNZ) {
     constexpr int blocks = DS_WARPS / (DR_THREADS / 32);
@@ -812,48 +875,41 @@ tc_status direct_run(tc_ctx *ctx, const DevCSR &d, const DirectReq &rq, Bump &bu
   }
   if (rq.vertex_counts)
     TC_CHECK_CUDA(ctx, cudaMemsetAsync(vcount, 0, sizeof(unsigned long long) * (size_t)(n * copies), ctx->stream));
+  unsigned long long *h = ctx->h_pinned;  // page-locked: the device writes it where it lies
+  DirectDag g{nullptr, 0, nullptr, nullptr, n, 0, n, nullptr, nullptr, rq.labels, rq.label, 0, 0};
+  set_bitmaps(g, n);
   if (rq.orient) {
-    direct_rows_kernel<true><<<B, DR_THREADS, 0, ctx->stream>>>(d.rowptr, d.col, n, nnz, nullptr, nullptr, nullptr, ku, kv, mask,
-                                                               gpre, bsum, res);
-    TC_CHECK_LAUNCH(ctx);
-    if (B > DR_SMEM_BLOCKS) {  // too many block sums for a block to scan
+    TC_CHECK_CUDA(ctx, launch_pass(ctx, direct_rows_kernel<true>, B, DR_THREADS, 0, d.rowptr, d.col, n, nnz, nullptr,
+                                   nullptr, nullptr, ku, kv, mask, gpre, bsum, res));
+    const bool scan = B > DR_SMEM_BLOCKS;  // too many block sums for a block to scan
+    if (scan) {
       TC_CHECK_CUDA(ctx, cudaMemsetAsync(bsum + B, 0, sizeof(uint32_t), ctx->stream));
       TC_TRY(exclusive_scan_u32(ctx, bsum, boff, B + 1, scratch));
     }
-    direct_place_kernel<<<B, DR_THREADS, 0, ctx->stream>>>(d.rowptr, n, nnz, B, bsum,
-                                                           B > DR_SMEM_BLOCKS ? boff : nullptr, mask, gpre, ku, kv, src,
-                                                           col, drow, res, max_work);
-    TC_CHECK_LAUNCH(ctx);
+    TC_CHECK_CUDA(ctx, launch_pass(ctx, direct_place_kernel, B, DR_THREADS, 0, d.rowptr, n, nnz, B, bsum,
+                                   scan ? boff : nullptr, mask, gpre, ku, kv, src, col, drow, res, max_work));
+    g.rp = drow;
+    g.col = col;
+    g.src = src;
   } else {
-    direct_rows_kernel<false><<<B, DR_THREADS, 0, ctx->stream>>>(d.rowptr, d.col, n, nnz, nullptr, nullptr, nullptr, ku, nullptr,
-                                                                nullptr, nullptr, nullptr, res);
-    TC_CHECK_LAUNCH(ctx);
+    TC_CHECK_CUDA(ctx, launch_pass(ctx, direct_rows_kernel<false>, B, DR_THREADS, 0, d.rowptr, d.col, n, nnz, nullptr,
+                                   nullptr, nullptr, ku, nullptr, nullptr, nullptr, nullptr, res));
+    g.rp = reinterpret_cast<const uint32_t *>(d.rowptr);
+    g.shift = 1;
+    g.col = d.col;
+    g.src = ku;
+    g.row_begin = rq.row_begin;
+    g.row_end = rq.row_end;
   }
-  TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[5], ctx->stream));
-  if (rq.orient) {
-    DirectDag g{drow, 0, col, src, n, 0, n, nullptr, nullptr, rq.labels, rq.label, 0, 0};
-    set_bitmaps(g, n);
-    if (rq.vertex_counts) TC_TRY(launch_count<1>(ctx, g, nnz / 2, 1, rq, vcount, copies, nullptr, res, max_work));
-    else if (rq.labels) TC_TRY(launch_count<2>(ctx, g, nnz / 2, 1, rq, nullptr, 1, nullptr, res, max_work));
-    else TC_TRY(launch_count<0>(ctx, g, nnz / 2, 1, rq, nullptr, 1, nullptr, res, max_work));
-    if (copies > 1) {
-      direct_vsum_kernel<<<grid_for(ctx, n, DC_THREADS, 8), DC_THREADS, 0, ctx->stream>>>(vcount, n, copies,
-                                                                                         rq.vertex_counts, res,
-                                                                                         max_work);
-      TC_CHECK_LAUNCH(ctx);
-    }
-  } else {
-    DirectDag g{reinterpret_cast<const uint32_t *>(d.rowptr), 1, d.col, ku, n, rq.row_begin, rq.row_end, nullptr,
-                      nullptr, nullptr, 0, 0, 0};
-    set_bitmaps(g, n);
-    TC_TRY(launch_count<0>(ctx, g, nnz, 1, rq, nullptr, 1, nullptr, res, max_work));
-  }
+  const int64_t edges = rq.orient ? nnz / 2 : nnz;
+  if (rq.vertex_counts) TC_TRY(launch_count<1>(ctx, g, edges, 1, rq, vcount, copies, nullptr, res, max_work, h));
+  else if (rq.labels) TC_TRY(launch_count<2>(ctx, g, edges, 1, rq, nullptr, 1, nullptr, res, max_work, h));
+  else TC_TRY(launch_count<0>(ctx, g, edges, 1, rq, nullptr, 1, nullptr, res, max_work, h));
+  if (copies > 1)
+    TC_CHECK_CUDA(ctx, launch_pass(ctx, direct_vsum_kernel, grid_for(ctx, n, DC_THREADS, 8), DC_THREADS, 0, vcount, n,
+                                   copies, rq.vertex_counts, res, max_work));
   TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[6], ctx->stream));
-  TC_CHECK_CUDA(ctx, cudaMemcpyAsync(&ctx->h_pinned[0], res, sizeof(unsigned long long) * DX_WORDS,
-                                     cudaMemcpyDeviceToHost, ctx->stream));
-  TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[7], ctx->stream));
   TC_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  const unsigned long long *h = ctx->h_pinned;
   if (const unsigned f = (unsigned)h[DX_FLAGS]) return set_error(ctx, TC_ERR_INVALID_GRAPH, "%s", flag_text(f));
   if (h[DX_WORK] > max_work) {
     *declined = true;
@@ -871,11 +927,12 @@ tc_status direct_run(tc_ctx *ctx, const DevCSR &d, const DirectReq &rq, Bump &bu
   st->tiles = (m + TILE_EDGES - 1) / TILE_EDGES;
   st->tiles_per_arm[TC_ARM_FLAT] = st->tiles;  // 32 edges' lists as one flattened run, as that arm
   st->alg_bytes_arm[TC_ARM_FLAT] = st->alg_bytes = h[DX_ALG];
-  st->ms_h2d = elapsed(ctx->ev[0], ctx->ev[1]);
-  st->ms_orient = elapsed(ctx->ev[1], ctx->ev[5]);
-  st->ms_arm[TC_ARM_FLAT] = st->ms_count = elapsed(ctx->ev[5], ctx->ev[6]);
-  st->ms_d2h = elapsed(ctx->ev[6], ctx->ev[7]);
-  st->ms_total = elapsed(ctx->ev[0], ctx->ev[7]);
+  // events between the passes would keep them apart: the parts are the device clock's
+  const float passes = 1e-6f * (float)(h[DX_END] - h[DX_START]);
+  st->ms_total = elapsed(ctx->ev[0], ctx->ev[6]);
+  st->ms_h2d = st->h2d_bytes ? std::max(0.f, st->ms_total - passes) : 0.f;
+  st->ms_orient = 1e-6f * (float)(h[DX_COUNT] - h[DX_START]);
+  st->ms_arm[TC_ARM_FLAT] = st->ms_count = 1e-6f * (float)(h[DX_END] - h[DX_COUNT]);
   st->d2h_bytes += sizeof(unsigned long long) + (rq.edge_host ? sizeof(uint32_t) * (size_t)m : 0) +
                    (rq.vertex_host ? sizeof(uint64_t) * (size_t)n : 0);
   st->kernel_launches = ctx->launches;
@@ -961,22 +1018,20 @@ tc_status direct_batch(tc_ctx *ctx, const DevCSR &d, const int64_t *vtx_off, int
     return TC_OK;
   }
   const int64_t max_n = (int64_t)h[DX_MAXN];
-  direct_rows_kernel<true><<<B, DR_THREADS, 0, ctx->stream>>>(d.rowptr, d.col, n, nnz, vgroup, vtx_off, deg, ku, kv, mask,
-                                                             gpre, bsum, res);
-  TC_CHECK_LAUNCH(ctx);
+  TC_CHECK_CUDA(ctx, launch_pass(ctx, direct_rows_kernel<true>, B, DR_THREADS, 0, d.rowptr, d.col, n, nnz, vgroup, vtx_off,
+                                 deg, ku, kv, mask, gpre, bsum, res));
   const bool scan = B > DR_SMEM_BLOCKS;
   if (scan) {
     TC_CHECK_CUDA(ctx, cudaMemsetAsync(bsum + B, 0, sizeof(uint32_t), ctx->stream));
     TC_TRY(exclusive_scan_u32(ctx, bsum, boff, B + 1, scratch));
   }
-  direct_place_kernel<<<std::min(B, ctx->num_sms * 32), DR_THREADS, 0, ctx->stream>>>(
-      d.rowptr, n, nnz, B, bsum, scan ? boff : nullptr, mask, gpre, ku, kv, src, col, drow, res, max_work);
-  TC_CHECK_LAUNCH(ctx);
+  TC_CHECK_CUDA(ctx, launch_pass(ctx, direct_place_kernel, std::min(B, ctx->num_sms * 32), DR_THREADS, 0, d.rowptr, n, nnz,
+                                 B, bsum, scan ? boff : nullptr, mask, gpre, ku, kv, src, col, drow, res, max_work));
   TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[5], ctx->stream));
   // runs of 8 batches of 32 edges: a warp rarely leaves a graph inside one
   DirectDag g{drow, 0, col, src, n, 0, n, vgroup, vtx_off, nullptr, 0, 0, 0};
   set_bitmaps(g, max_n);
-  TC_TRY(launch_count<0>(ctx, g, nnz / 2, 8, DirectReq(), nullptr, 1, tot, res, max_work));
+  TC_TRY(launch_count<0>(ctx, g, nnz / 2, 8, DirectReq(), nullptr, 1, tot, res, max_work, nullptr));
   TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[6], ctx->stream));
   TC_CHECK_CUDA(ctx, cudaMemcpyAsync(&ctx->h_pinned[0], res, sizeof(unsigned long long) * DX_WORDS,
                                      cudaMemcpyDeviceToHost, ctx->stream));
