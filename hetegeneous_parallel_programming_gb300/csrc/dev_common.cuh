@@ -286,17 +286,9 @@ __device__ void expand_rows(const int64_t *__restrict__ rowptr, int64_t n, int64
   }
   if (lane == 31) scan_tmp[warp] = x;
   __syncthreads();
-  if (warp == 0) {
-    int w = lane < (int)(blockDim.x >> 5) ? scan_tmp[lane] : -1;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      int y = __shfl_up_sync(TC_FULL_MASK, w, o);
-      if (lane >= o) w = max(w, y);
-    }
-    scan_tmp[lane] = w;
-  }
-  __syncthreads();
-  int carry = warp > 0 ? scan_tmp[warp - 1] : -1;
+  // every warp takes the maximum of the warps before it for itself: one
+  // barrier less than a scan by the first warp
+  int carry = __reduce_max_sync(TC_FULL_MASK, lane < warp ? scan_tmp[lane] : -1);
   int xin = __shfl_up_sync(TC_FULL_MASK, x, 1);
   if (lane > 0) carry = max(carry, xin);
 #pragma unroll

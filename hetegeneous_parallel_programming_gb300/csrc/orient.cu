@@ -383,13 +383,14 @@ __global__ void __launch_bounds__(OR_THREADS, 6) place_kernel(const int64_t *__r
                                                           const int64_t *__restrict__ rowbase) {
   __shared__ int rows[row_slots<ENTRY_TILE>()];
   __shared__ int scan_tmp[32];
-  __shared__ long long s_wbase[OR_THREADS / 32 + 1];
   constexpr int NW = OR_THREADS / 32;
+  __shared__ int s_wcnt[2][NW];
   const int64_t b = (int64_t)blockIdx.x * chunk, e_end = min(nnz, b + chunk);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned lt = lanemask_lt();
   long long carry = boff[blockIdx.x];
   int64_t hint = -1;
+  int flip = 0;
   for (int64_t t0 = b; t0 < e_end; t0 += ENTRY_TILE) {
     const int64_t t1 = min(e_end, t0 + ENTRY_TILE);
     expand_rows<ENTRY_TILE>(rowptr, n, t0, t1, rows, scan_tmp, hint);
@@ -417,19 +418,15 @@ __global__ void __launch_bounds__(OR_THREADS, 6) place_kernel(const int64_t *__r
       bal[k] = __ballot_sync(TC_FULL_MASK, keep);
       cnt += __popc(bal[k]);
     }
-    if (lane == 0) s_wbase[warp] = cnt;
+    // the warps' counts, double-buffered (expand_rows of the next tile is the
+    // barrier between its writes and these reads): every warp sums for itself
+    if (lane == 0) s_wcnt[flip][warp] = cnt;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      long long acc = 0;
-      for (int w = 0; w < NW; ++w) {
-        const long long c = s_wbase[w];
-        s_wbase[w] = acc;
-        acc += c;
-      }
-      s_wbase[NW] = acc;
-    }
-    __syncthreads();
-    long long pos = carry + s_wbase[warp];
+    const int wc = lane < NW ? s_wcnt[flip][lane] : 0;
+    const int before = __reduce_add_sync(TC_FULL_MASK, lane < warp ? wc : 0);
+    const int tile_kept = __reduce_add_sync(TC_FULL_MASK, wc);
+    flip ^= 1;
+    long long pos = carry + before;
 #pragma unroll
     for (int k = 0; k < OR_PER; ++k) {
       if ((bal[k] >> lane) & 1u) {
@@ -445,8 +442,7 @@ __global__ void __launch_bounds__(OR_THREADS, 6) place_kernel(const int64_t *__r
       }
       pos += __popc(bal[k]);
     }
-    carry += s_wbase[NW];
-    __syncthreads();
+    carry += tile_kept;
   }
 }
 
@@ -679,14 +675,20 @@ template <bool VALS>
 __device__ __forceinline__ void pack_cmp(uint32_t &key, uint32_t &val, int lane, int partner) {
   const uint32_t ok = __shfl_sync(TC_FULL_MASK, key, partner);
   const uint32_t ov = VALS ? __shfl_sync(TC_FULL_MASK, val, partner) : 0u;
-  const bool take = lane < partner ? ok < key : ok > key;
-  if (take) {
-    key = ok;
-    if (VALS) val = ov;
+  if (!VALS) {
+    key = lane < partner ? min(key, ok) : max(key, ok);
+  } else {
+    const bool take = lane < partner ? ok < key : ok > key;
+    key = take ? ok : key;
+    val = take ? ov : val;
   }
 }
 
-template <bool VALS>
+// PLACED (rows with a payload, at most 2^22 vertices): the entry's place in the
+// pack below the id (5 + 22 + 5 bits), the payload fetched by it afterwards.
+constexpr int64_t SEG_PACK_PLACE_MAX_N = int64_t(1) << 22;
+
+template <bool VALS, bool PLACED>
 __global__ void __launch_bounds__(256) seg_sort_pack_kernel(const int64_t *__restrict__ nrowptr, int64_t n,
                                                            int32_t *__restrict__ ncol, uint32_t *__restrict__ perm,
                                                            int32_t *__restrict__ src) {
@@ -729,7 +731,9 @@ __global__ void __launch_bounds__(256) seg_sort_pack_kernel(const int64_t *__res
           __reduce_or_sync(TC_FULL_MASK, (in >> lane) & 1u ? 1u << (excl - before) : 0u);
       if ((in >> lane) & 1u) s_row[w][buf][__popc(in & lt)] = lane;
       const int ord = __popc(starts & le) - 1;
-      key = lane < cnt ? (uint32_t)ord << SEG_PACK_BITS | (uint32_t)ncol[b + lane] : 0xffffffffu;
+      key = lane >= cnt ? 0xffffffffu
+            : PLACED    ? (uint32_t)ord << SEG_PACK_BITS | (uint32_t)ncol[b + lane] << 5 | (uint32_t)lane
+                        : (uint32_t)ord << SEG_PACK_BITS | (uint32_t)ncol[b + lane];
       val = VALS && lane < cnt ? perm[b + lane] : 0u;
     };
     load(0);
@@ -744,12 +748,13 @@ __global__ void __launch_bounds__(256) seg_sort_pack_kernel(const int64_t *__res
       if (multi & ((pt < 32 ? (1u << pt) : 0u) - (1u << ps))) {  // some row of rows [ps, pt) has two entries
 #pragma unroll
         for (int lv = 2; lv <= 32; lv <<= 1) {
-          pack_cmp<VALS>(k, v, lane, lane ^ (lv - 1));
+          pack_cmp<VALS && !PLACED>(k, v, lane, lane ^ (lv - 1));
 #pragma unroll
-          for (int j = lv >> 2; j >= 1; j >>= 1) pack_cmp<VALS>(k, v, lane, lane ^ j);
+          for (int j = lv >> 2; j >= 1; j >>= 1) pack_cmp<VALS && !PLACED>(k, v, lane, lane ^ j);
         }
+        if (PLACED) v = __shfl_sync(TC_FULL_MASK, v, (int)(k & 31u));
         if (lane < pcnt) {
-          ncol[pb + lane] = (int32_t)(k & ((1u << SEG_PACK_BITS) - 1u));
+          ncol[pb + lane] = (int32_t)((k & ((1u << SEG_PACK_BITS) - 1u)) >> (PLACED ? 5 : 0));
           if (VALS) perm[pb + lane] = v;
         }
       }
@@ -766,10 +771,27 @@ __global__ void __launch_bounds__(256) seg_sort_pack_kernel(const int64_t *__res
 // 1), slot E - 1 - x; its half-cleaner partner at distance j is i ^ j.
 template <bool VALS>
 __device__ __forceinline__ void reg_keep(int32_t &k, uint32_t &v, int32_t ok, uint32_t ov, bool lower) {
-  if (lower ? ok < k : ok > k) {
-    k = ok;
-    if (VALS) v = ov;
+  if (!VALS) {  // one min/max instruction, no branch
+    k = lower ? min(k, ok) : max(k, ok);
+  } else {
+    const bool take = lower ? ok < k : ok > k;
+    k = take ? ok : k;
+    v = take ? ov : v;
   }
+}
+
+// Two entries of one lane into order.
+template <bool VALS>
+__device__ __forceinline__ void reg_order(int32_t &a, uint32_t &va, int32_t &b, uint32_t &vb) {
+  const bool swap = b < a;
+  const int32_t lo = min(a, b), hi = max(a, b);
+  if (VALS) {
+    const uint32_t t = va;
+    va = swap ? vb : va;
+    vb = swap ? t : vb;
+  }
+  a = lo;
+  b = hi;
 }
 
 template <int E, bool VALS>
@@ -782,16 +804,7 @@ __device__ __forceinline__ void warp_sort_blocked(int32_t (&k)[E], uint32_t (&v)
 #pragma unroll
       for (int x = 0; x < E; ++x) {
         const int y = x ^ (lv - 1);
-        if (y > x && k[y] < k[x]) {
-          const int32_t t = k[x];
-          k[x] = k[y];
-          k[y] = t;
-          if (VALS) {
-            const uint32_t s = v[x];
-            v[x] = v[y];
-            v[y] = s;
-          }
-        }
+        if (y > x) reg_order<VALS>(k[x], v[x], k[y], v[y]);
       }
     } else {
       // entries x and E-1-x trade with the partner's E-1-x and x: both keys
@@ -815,16 +828,7 @@ __device__ __forceinline__ void warp_sort_blocked(int32_t (&k)[E], uint32_t (&v)
         for (int x = 0; x < E; ++x) {
           if (x & j) continue;
           const int y = x | j;
-          if (k[y] < k[x]) {
-            const int32_t t = k[x];
-            k[x] = k[y];
-            k[y] = t;
-            if (VALS) {
-              const uint32_t s = v[x];
-              v[x] = v[y];
-              v[y] = s;
-            }
-          }
+          reg_order<VALS>(k[x], v[x], k[y], v[y]);
         }
       } else {
         const int pl = lane ^ (j / E);
@@ -862,9 +866,42 @@ __device__ __forceinline__ void warp_sort_row_blocked(int32_t *__restrict__ ncol
   }
 }
 
+// The same for rows with a payload in graphs of at most 2^24 vertices: a key
+// is the id above the entry's place in its row (24 + 8 bits), so the network
+// moves one word per entry, and the payload is fetched by place afterwards.
+// (Sign bit flipped: the comparisons are signed.)
+constexpr int64_t SEG_PLACE_MAX_N = int64_t(1) << 24;
+
+template <int E>
+__device__ __forceinline__ void warp_sort_row_placed(int32_t *__restrict__ ncol, uint32_t *__restrict__ perm,
+                                                     int64_t b, int L, int lane) {
+  int32_t k[E];
+  uint32_t v[E];
+#pragma unroll
+  for (int x = 0; x < E; ++x) {
+    const int i = lane * E + x;
+    k[x] = i < L ? (int32_t)(((uint32_t)ncol[b + i] << 8 | (uint32_t)i) ^ 0x80000000u) : INT32_MAX;
+  }
+  warp_sort_blocked<E, false>(k, v, lane);
+#pragma unroll
+  for (int x = 0; x < E; ++x) v[x] = lane * E + x < L ? perm[b + ((uint32_t)k[x] & 255u)] : 0u;
+  __syncwarp();  // every payload is read before one is written
+#pragma unroll
+  for (int x = 0; x < E; ++x) {
+    const int i = lane * E + x;
+    if (i < L) {
+      ncol[b + i] = (int32_t)(((uint32_t)k[x] ^ 0x80000000u) >> 8);
+      perm[b + i] = v[x];
+    }
+  }
+}
+
 // Rows of 33..SEG_WARP_MAX entries: one warp per row, 2, 4 or 8 keys per
-// lane in registers (warp_sort_blocked).
-template <bool VALS>
+// lane in registers (warp_sort_blocked).  Bound by issue and, while the
+// compare-exchanges were branches, by their resolution: as min/max R-MAT scale
+// 24 takes 0.59 ms for 2.08.  PLACED: rows with a payload, see above (R-MAT
+// scale 20: 252 -> 94 us).
+template <bool VALS, bool PLACED>
 __global__ void __launch_bounds__(256) seg_sort_warpreg_kernel(const int64_t *__restrict__ nrowptr,
                                                               const int32_t *__restrict__ list,
                                                               const unsigned *count, int32_t *__restrict__ ncol,
@@ -877,9 +914,15 @@ __global__ void __launch_bounds__(256) seg_sort_warpreg_kernel(const int64_t *__
     const int32_t r = list[i];
     const int64_t b = nrowptr[r];
     const int L = (int)(nrowptr[r + 1] - b);
-    if (L <= 64) warp_sort_row_blocked<2, VALS>(ncol, perm, b, L, lane);
-    else if (L <= 128) warp_sort_row_blocked<4, VALS>(ncol, perm, b, L, lane);
-    else warp_sort_row_blocked<8, VALS>(ncol, perm, b, L, lane);
+    if (PLACED) {
+      if (L <= 64) warp_sort_row_placed<2>(ncol, perm, b, L, lane);
+      else if (L <= 128) warp_sort_row_placed<4>(ncol, perm, b, L, lane);
+      else warp_sort_row_placed<8>(ncol, perm, b, L, lane);
+    } else {
+      if (L <= 64) warp_sort_row_blocked<2, VALS>(ncol, perm, b, L, lane);
+      else if (L <= 128) warp_sort_row_blocked<4, VALS>(ncol, perm, b, L, lane);
+      else warp_sort_row_blocked<8, VALS>(ncol, perm, b, L, lane);
+    }
     put_row_src(src, b, L, r, lane, 32);
   }
 }
@@ -1009,6 +1052,82 @@ __global__ void __launch_bounds__(256) seg_sort_warpsmem_kernel(const int64_t *_
 // are distinct), a block prefix of the words' popcounts, then every thread
 // writes its words' set bits in order.
 constexpr int SEG_BITMAP_KEYS = SEG_SMEM_MAX / 256;  // keys per thread (256 threads)
+
+// With a payload the words' prefix sums give every entry its rank, and the row
+// goes out by rank from a copy in shared memory (R-MAT scale 20, 257 to 4096
+// entries: 162 -> 69 us).
+constexpr int SEG_RANK_WORDS = SEG_SMEM_MAX;  // ids may span 32 times as many values
+
+__global__ void __launch_bounds__(256) seg_sort_rank_kernel(const int64_t *__restrict__ nrowptr,
+                                                           const int32_t *__restrict__ list, const unsigned *count,
+                                                           int32_t *__restrict__ ncol, uint32_t *__restrict__ perm,
+                                                           int32_t *__restrict__ defer, unsigned *defer_count,
+                                                           int32_t *__restrict__ src) {
+  extern __shared__ uint32_t s_mem[];
+  uint32_t *bm = s_mem;                                                 // [SEG_RANK_WORDS]
+  int32_t *skey = reinterpret_cast<int32_t *>(bm + SEG_RANK_WORDS);     // [SEG_SMEM_MAX]
+  uint32_t *sval = reinterpret_cast<uint32_t *>(skey + SEG_SMEM_MAX);   // [SEG_SMEM_MAX]
+  uint16_t *pre = reinterpret_cast<uint16_t *>(sval + SEG_SMEM_MAX);    // [SEG_RANK_WORDS]
+  __shared__ int32_t s_red[2][8];
+  __shared__ int tmp[33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned cnt = *count;
+  for (unsigned i = blockIdx.x; i < cnt; i += gridDim.x) {
+    const int32_t r = list[i];
+    const int64_t b = nrowptr[r];
+    const int L = (int)(nrowptr[r + 1] - b);
+    int32_t lo = INT32_MAX, hi = -1;
+    for (int k = threadIdx.x; k < L; k += 256) {
+      const int32_t x = ncol[b + k];
+      skey[k] = x;
+      sval[k] = perm[b + k];
+      lo = min(lo, x);
+      hi = max(hi, x);
+    }
+    lo = __reduce_min_sync(TC_FULL_MASK, lo);
+    hi = __reduce_max_sync(TC_FULL_MASK, hi);
+    if (lane == 0) {
+      s_red[0][warp] = lo;
+      s_red[1][warp] = hi;
+    }
+    __syncthreads();
+    lo = __reduce_min_sync(TC_FULL_MASK, s_red[0][lane & 7]);
+    hi = __reduce_max_sync(TC_FULL_MASK, s_red[1][lane & 7]);
+    const int64_t span = (int64_t)hi - lo + 1;
+    const int W = span <= 32 * (int64_t)SEG_RANK_WORDS ? (int)((span + 31) >> 5) : 0;
+    for (int q = threadIdx.x; q < W; q += 256) bm[q] = 0u;
+    __syncthreads();
+    if (W > 0)
+      for (int k = threadIdx.x; k < L; k += 256) {
+        const uint32_t d = (uint32_t)(skey[k] - lo);
+        atomicOr(&bm[d >> 5], 1u << (d & 31));
+      }
+    __syncthreads();
+    const int per = (W + 255) / 256, w0 = min(W, (int)threadIdx.x * per), w1 = min(W, w0 + per);
+    int c = 0, tot;
+    for (int q = w0; q < w1; ++q) c += __popc(bm[q]);
+    int run = block_exclusive_scan<int>(c, tmp, &tot);
+    for (int q = w0; q < w1; ++q) {
+      pre[q] = (uint16_t)run;
+      run += __popc(bm[q]);
+    }
+    if (W == 0 || tot != L) {  // too wide, or duplicate ids (unvalidated input): left to the block sort
+      if (threadIdx.x == 0) defer[atomicAdd(defer_count, 1u)] = r;
+      __syncthreads();
+      continue;
+    }
+    put_row_src(src, b, L, r, threadIdx.x, blockDim.x);
+    __syncthreads();
+    for (int k = threadIdx.x; k < L; k += 256) {
+      const uint32_t d = (uint32_t)(skey[k] - lo);
+      const int at = pre[d >> 5] + __popc(bm[d >> 5] & ((1u << (d & 31)) - 1u));
+      ncol[b + at] = skey[k];
+      perm[b + at] = sval[k];
+    }
+    __syncthreads();
+  }
+}
+constexpr int SEG_RANK_SMEM = SEG_RANK_WORDS * 6 + SEG_SMEM_MAX * 8;
 
 template <bool VALS>
 __global__ void __launch_bounds__(256) seg_sort_smem_kernel(const int64_t *__restrict__ nrowptr,
@@ -1142,8 +1261,10 @@ template <bool VALS>
 static tc_status launch_row_sorts(tc_ctx *ctx, const DevCSR &g, OrientBufs &b) {
   uint32_t *pv = VALS ? b.perm : nullptr;
   int32_t *sv = SORT_SRC ? b.nsrc : nullptr;  // rows written by the sorts (every row visits one)
-  if (g.n <= SEG_PACK_MAX_N)
-    seg_sort_pack_kernel<VALS><<<grid_for(ctx, g.n, 256, 8), 256, 0, ctx->stream>>>(b.nrowptr, g.n, b.ncol, pv, sv);
+  if (VALS && g.n <= SEG_PACK_PLACE_MAX_N)
+    seg_sort_pack_kernel<VALS, true><<<grid_for(ctx, g.n, 256, 8), 256, 0, ctx->stream>>>(b.nrowptr, g.n, b.ncol, pv, sv);
+  else if (g.n <= SEG_PACK_MAX_N)
+    seg_sort_pack_kernel<VALS, false><<<grid_for(ctx, g.n, 256, 8), 256, 0, ctx->stream>>>(b.nrowptr, g.n, b.ncol, pv, sv);
   else if (SEG_WARP_CHUNK)
     seg_sort_warp_chunk_kernel<VALS><<<grid_for(ctx, g.n, 256, 8), 256, 0, ctx->stream>>>(b.nrowptr, g.n, b.ncol,
                                                                                           pv, sv);
@@ -1151,9 +1272,12 @@ static tc_status launch_row_sorts(tc_ctx *ctx, const DevCSR &g, OrientBufs &b) {
     seg_sort_warp_kernel<VALS><<<grid_for(ctx, g.n * 32, 256, 8), 256, 0, ctx->stream>>>(b.nrowptr, g.n, b.ncol, pv,
                                                                                          sv);
   TC_CHECK_LAUNCH(ctx);
-  if (SEG_WARP_REG)
-    seg_sort_warpreg_kernel<VALS><<<ctx->num_sms * 8, 256, 0, ctx->stream>>>(b.nrowptr, b.mid_list, b.seg_counts,
-                                                                            b.ncol, pv, sv);
+  if (SEG_WARP_REG && VALS && g.n <= SEG_PLACE_MAX_N)
+    seg_sort_warpreg_kernel<VALS, true><<<ctx->num_sms * 8, 256, 0, ctx->stream>>>(b.nrowptr, b.mid_list, b.seg_counts,
+                                                                                  b.ncol, pv, sv);
+  else if (SEG_WARP_REG)
+    seg_sort_warpreg_kernel<VALS, false><<<ctx->num_sms * 8, 256, 0, ctx->stream>>>(b.nrowptr, b.mid_list, b.seg_counts,
+                                                                                   b.ncol, pv, sv);
   else
     seg_sort_warpsmem_kernel<VALS><<<ctx->num_sms * 8, 256, 0, ctx->stream>>>(b.nrowptr, b.mid_list, b.seg_counts,
                                                                             b.ncol, pv, sv);
@@ -1163,6 +1287,13 @@ static tc_status launch_row_sorts(tc_ctx *ctx, const DevCSR &g, OrientBufs &b) {
     // which the warp sort above has finished with) through the block sort
     seg_sort_warpbits_kernel<<<ctx->num_sms * 4, WB_WARPS * 32, 0, ctx->stream>>>(
         b.nrowptr, b.big_list, b.seg_counts + 1, b.ncol, b.mid_list, b.seg_counts + 3, sv);
+    TC_CHECK_LAUNCH(ctx);
+    seg_sort_smem_kernel<VALS><<<ctx->num_sms * 8, 256, 0, ctx->stream>>>(b.nrowptr, b.mid_list, b.seg_counts + 3,
+                                                                          b.ncol, pv, sv);
+  } else if (VALS) {
+    TC_CHECK_CUDA(ctx, cudaFuncSetAttribute(seg_sort_rank_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SEG_RANK_SMEM));
+    seg_sort_rank_kernel<<<ctx->num_sms * 4, 256, SEG_RANK_SMEM, ctx->stream>>>(
+        b.nrowptr, b.big_list, b.seg_counts + 1, b.ncol, pv, b.mid_list, b.seg_counts + 3, sv);
     TC_CHECK_LAUNCH(ctx);
     seg_sort_smem_kernel<VALS><<<ctx->num_sms * 8, 256, 0, ctx->stream>>>(b.nrowptr, b.mid_list, b.seg_counts + 3,
                                                                           b.ncol, pv, sv);
