@@ -30,22 +30,14 @@ constexpr int PLAN_THREADS = 256;
 // 1: the planner visits tiles interleaved over the PULL source blocks, so
 // the SMs' histogram atomics at any moment go to different blocks' hub keys
 // instead of all to the hot hubs of one block (R-MAT scale 24: plan 3.88 ->
-// 2.80 ms).  The scatter keeps tile order (PL_SCATTER_INTERLEAVE 0): the
-// records of a target group then follow the rows' order, which the probing
-// kernel's suffix loads profit from; interleaved tile by tile, or in chunks
-// of 64 or 256 tiles, the PULL arm took 1.3, 1.4 and 1.7 ms longer.
+// 2.80 ms).  The scatter keeps tile order: the records of a target group then
+// follow the rows' order, which the probing kernel's suffix loads profit from;
+// interleaved tile by tile, or in chunks of 64 or 256 tiles, the PULL arm took
+// 1.3, 1.4 and 1.7 ms longer.
 #ifndef TC_PL_INTERLEAVE
 #define TC_PL_INTERLEAVE 1
 #endif
 constexpr bool PL_INTERLEAVE = TC_PL_INTERLEAVE != 0;
-#ifndef TC_PL_SCATTER_INTERLEAVE
-#define TC_PL_SCATTER_INTERLEAVE 0
-#endif
-constexpr bool PL_SCATTER_INTERLEAVE = TC_PL_SCATTER_INTERLEAVE != 0;
-#ifndef TC_PL_SCATTER_GRAIN
-#define TC_PL_SCATTER_GRAIN 1
-#endif
-constexpr int64_t PL_SCATTER_GRAIN = TC_PL_SCATTER_GRAIN;  // tiles per interleaved chunk of the scatter
 #ifndef TC_PLAN_UNROLL
 #define TC_PLAN_UNROLL 2
 #endif
@@ -1445,18 +1437,6 @@ constexpr int PL_UNROLL = 4;      // table build: list loads in flight per lane
 #endif
 constexpr int PL_GUNROLL = TC_PL_GUNROLL;  // flattened probing: 16-byte loads in flight per lane
 constexpr int PL_GROUP_THREADS = 256;
-// edges per thread whose atomics are issued together in the scatter (1: at
-// R-MAT scale 24, 2 and 4 were 0.3 ms slower; at scale 22 4 was 0.05 ms faster)
-#ifndef TC_PL_SCATTER_UNROLL
-#define TC_PL_SCATTER_UNROLL 1
-#endif
-constexpr int PL_SCATTER_UNROLL = TC_PL_SCATTER_UNROLL;
-// 1: the scatter streams its column and row reads and its record stores with
-// evict-first hints, so the grouping counters (K * 4 bytes) stay in L2
-#ifndef TC_PL_SCATTER_STREAM
-#define TC_PL_SCATTER_STREAM 1
-#endif
-constexpr bool PL_SCATTER_STREAM = TC_PL_SCATTER_STREAM != 0;
 // Dense edges: an edge u->v whose source is a hub and whose row suffix holds
 // more than dense_num / dense_den entries per 32-bit word of v's bitmap
 // table (ctx->pull_dense_num / pull_dense_den, 1/1 unless tuned) is counted
@@ -1498,51 +1478,60 @@ constexpr int64_t PL_LOW_KEY_BUDGET = (int64_t)1 << 28;  // keys of the non-hub 
 // relabelled (the probed suffix is (e, rowptr[row + 1])), else (edge id,
 // row).  Edges are visited in order, so the row ends are read almost
 // sequentially here instead of at random in the probing kernel.
+//
+// Bound by the slots' atomics, which take turns where edges meet: a tile has a
+// hundred rows, and most of them end in the same few hubs.  The last PL_HOT
+// ids are therefore counted per tile in shared memory first, one global atomic
+// takes the tile's slots of each, and the edges share them out (hot0: first of
+// these ids; a caller's DAG has none).  One call, an atomic per edge -> this:
+// R-MAT scale 18 1.03 -> 1.00 ms, 20 2.57 -> 2.50, 22 9.99 -> 9.89, 24 51.25 ->
+// 50.98; 4096 hot ids 51.5, 256 51.1 (their table is walked once per tile).
+constexpr int PL_HOT = 1024;
+constexpr int PL_SCATTER_PER = TILE_EDGES / PL_GROUP_THREADS;  // edges per thread of a tile
+
 __global__ void __launch_bounds__(PL_GROUP_THREADS) pull_scatter_kernel(const int32_t *__restrict__ col,
                                                                        const int32_t *__restrict__ src,
                                                                        const int64_t *__restrict__ rowptr,
-                                                                       int row_end,
+                                                                       int row_end, int64_t hot0,
                                                                        const int32_t *__restrict__ arm, int64_t m,
                                                                        PullKeys pk,
                                                                        unsigned *__restrict__ pos,
                                                                        uint2 *__restrict__ er) {
+  __shared__ unsigned s_hot[PL_HOT];
   const int64_t T = (m + TILE_EDGES - 1) / TILE_EDGES;
-  constexpr int U = PL_SCATTER_UNROLL;  // edges per thread in flight: their atomics overlap
-  // tiles in order, or chunks of PL_SCATTER_GRAIN tiles interleaved over the
-  // source blocks (see PL_INTERLEAVE)
-  const int64_t per = pk.block_edges / TILE_EDGES, S = (T + per - 1) / per;
-  const bool il = PL_SCATTER_INTERLEAVE && S > 1 && per % PL_SCATTER_GRAIN == 0;
-  const int64_t cpb = per / PL_SCATTER_GRAIN;  // chunks per source block
-  for (int64_t i = blockIdx.x; i < (il ? S * per : T); i += gridDim.x) {
-    const int64_t c = i / PL_SCATTER_GRAIN;
-    const int64_t t = il ? ((c % S) * cpb + c / S) * PL_SCATTER_GRAIN + i % PL_SCATTER_GRAIN : i;
-    if (t >= T || arm[t] != TC_ARM_PULL) continue;
-    const int64_t e1 = min(m, (t + 1) * TILE_EDGES), kb = pk.block_base(t), lb = pk.low_base(t);
-    for (int64_t eb = t * TILE_EDGES + threadIdx.x; eb < e1; eb += U * PL_GROUP_THREADS) {
-      int64_t key[U];
-      int32_t r[U];
-      unsigned slot[U];
+  for (int i = threadIdx.x; i < PL_HOT; i += PL_GROUP_THREADS) s_hot[i] = 0u;
+  for (int64_t t = blockIdx.x; t < T; t += gridDim.x) {
+    if (arm[t] != TC_ARM_PULL) continue;
+    __syncthreads();
+    const int64_t e0 = t * TILE_EDGES, e1 = min(m, e0 + TILE_EDGES), kb = pk.block_base(t), lb = pk.low_base(t);
+    int32_t v[PL_SCATTER_PER];
+    unsigned slot[PL_SCATTER_PER];  // of a hot target: its place among the tile's
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int64_t e = eb + u * PL_GROUP_THREADS;
-        key[u] = -1;
-        r[u] = 0;
-        if (e < e1) {  // read once: streamed past L2, which keeps the counters
-          key[u] = pk.key_in(kb, lb, PL_SCATTER_STREAM ? __ldcs(col + e) : __ldg(col + e));
-          r[u] = PL_SCATTER_STREAM ? __ldcs(src + e) : __ldg(src + e);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u) slot[u] = key[u] >= 0 ? atomicAdd(pos + key[u], 1u) : 0u;
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        if (key[u] < 0) continue;
-        const uint32_t y = row_end ? (uint32_t)__ldg(rowptr + r[u] + 1) : (uint32_t)r[u];
-        const uint2 rec = make_uint2((uint32_t)(eb + u * PL_GROUP_THREADS), y);  // one 8-byte store
-        if (PL_SCATTER_STREAM) __stcs(er + slot[u], rec);  // evict-first: the counters stay in L2
-        else er[slot[u]] = rec;
-      }
+    for (int j = 0; j < PL_SCATTER_PER; ++j) {  // read once: streamed past L2, which keeps the counters
+      const int64_t e = e0 + j * PL_GROUP_THREADS + threadIdx.x;
+      v[j] = e < e1 ? __ldcs(col + e) : -1;
     }
+#pragma unroll
+    for (int j = 0; j < PL_SCATTER_PER; ++j) {
+      slot[j] = 0u;
+      if (v[j] >= hot0) slot[j] = atomicAdd(&s_hot[v[j] - hot0], 1u);
+      else if (v[j] >= 0) slot[j] = atomicAdd(pos + pk.key_in(kb, lb, v[j]), 1u);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < PL_HOT; i += PL_GROUP_THREADS)
+      if (const unsigned c = s_hot[i]) s_hot[i] = atomicAdd(pos + pk.key_in(kb, lb, (int32_t)(hot0 + i)), c);
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < PL_SCATTER_PER; ++j) {
+      const int64_t e = e0 + j * PL_GROUP_THREADS + threadIdx.x;
+      if (v[j] < 0) continue;
+      const unsigned at = slot[j] + (v[j] >= hot0 ? s_hot[v[j] - hot0] : 0u);
+      const int32_t r = __ldcs(src + e);
+      const uint32_t y = row_end ? (uint32_t)__ldg(rowptr + r + 1) : (uint32_t)r;
+      __stcs(er + at, make_uint2((uint32_t)e, y));  // one 8-byte store, evict-first
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < PL_HOT; i += PL_GROUP_THREADS) s_hot[i] = 0u;
   }
 }
 
@@ -2604,8 +2593,9 @@ static tc_status run_pull(tc_ctx *ctx, const DevDag &g_in, CountBufs &cb, uint32
   unsigned *pos = cb.pull_pos;
   const int gblocks = (int)std::min<int64_t>(T, (int64_t)ctx->num_sms * 8);
   TC_TRY(exclusive_scan_u32(ctx, cb.pull_pos, cb.pull_pos, K + 1, cb.sort_scratch));
+  const int64_t hot0 = !g_in.restrict_after ? g_in.n : std::max<int64_t>(0, g_in.n - PL_HOT);
   pull_scatter_kernel<<<gblocks, PL_GROUP_THREADS, 0, ctx->stream>>>(g_in.col, g_in.src, g_in.rowptr,
-                                                                     g_in.restrict_after, cb.arm, g_in.m, pk, pos,
+                                                                     g_in.restrict_after, hot0, cb.arm, g_in.m, pk, pos,
                                                                      cb.pull_er);
   TC_CHECK_LAUNCH(ctx);
   const DevDag &g = g_in;
