@@ -58,8 +58,8 @@ int grid_for(const tc_ctx *ctx, int64_t items, int per_block, int blocks_per_sm)
 
 constexpr int RS_THREADS = 256;
 constexpr int RS_WARPS = RS_THREADS / 32;
-constexpr int RS_IPL = 16;                        // keys per lane per tile
-constexpr int RS_TILE = RS_THREADS * RS_IPL;      // 4096 keys
+constexpr int RS_IPL = 10;                        // keys per lane per tile
+constexpr int RS_TILE = RS_THREADS * RS_IPL;      // 2560 keys
 constexpr int RS_BLOCKS_PER_SM = 4;
 constexpr int RS_MAX_PASSES = 8;
 
@@ -148,10 +148,11 @@ __global__ void __launch_bounds__(RS_THREADS) rs_scan_kernel(const uint32_t *__r
 // Places one digit's keys.  Lanes that hold the same digit find each other by
 // one ballot per digit bit (a match instruction took 47 cycles a round); the
 // warps' counts give each key its place in the tile, where the keys meet in
-// shared memory, and the tile leaves digit by digit, 16 keys (128 bytes) a
+// shared memory, and the tile leaves digit by digit, 10 keys (80 bytes) a
 // run on average.  Bound by memory: 16 bytes per key plus 8 for the
-// histogram.  33.6 M keys take 202 us, 2.7 TB/s (the direct scatter it
-// replaces 460), the histogram 47 us, 5.7 TB/s (172).
+// histogram.  33.6 M keys take 163 us, 3.3 TB/s (the direct scatter it
+// replaces 460; 16 keys a lane 202, 12 and a tile of 3072 185), the histogram
+// 46 us, 5.8 TB/s (172).
 __global__ void __launch_bounds__(RS_THREADS, RS_BLOCKS_PER_SM) rs_scatter_kernel(
     const uint64_t *__restrict__ kin, uint64_t *__restrict__ kout, int64_t N, int shift, int dbits, int64_t chunk,
     const uint32_t *__restrict__ offs, int G) {
@@ -167,30 +168,34 @@ __global__ void __launch_bounds__(RS_THREADS, RS_BLOCKS_PER_SM) rs_scatter_kerne
   for (int64_t t0 = b; t0 < e; t0 += RS_TILE) {
     const int nt = (int)min((int64_t)RS_TILE, e - t0);
     uint64_t k[RS_IPL];
-    uint32_t r[RS_IPL / 2];  // ranks, 16 bits each
+    uint32_t r[RS_IPL];  // the lanes with the key's digit, then its rank in the warp
     const int base = warp * (32 * RS_IPL) + lane;
 #pragma unroll
     for (int it = 0; it < RS_IPL; ++it) k[it] = base + it * 32 < nt ? kin[t0 + base + it * 32] : ~0ull;
     for (int i = threadIdx.x; i < RS_WARPS * 256 / 2; i += RS_THREADS) reinterpret_cast<uint32_t *>(&s_cnt[0][0])[i] = 0u;
     __syncthreads();
+    // every round's ballots first: they do not depend on one another
 #pragma unroll
     for (int it = 0; it < RS_IPL; ++it) {
       const bool in = base + it * 32 < nt;
-      const unsigned d = (unsigned)(k[it] >> shift) & dmask;
-      unsigned peers = __ballot_sync(TC_FULL_MASK, in);
-      peers = in ? peers : ~peers;
+      const unsigned d = (unsigned)(k[it] >> shift) & dmask, all = __ballot_sync(TC_FULL_MASK, in);
+      r[it] = in ? all : ~all;
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
         if (q >= dbits) break;
         const bool bit = (d >> q) & 1u;
         const unsigned bal = __ballot_sync(TC_FULL_MASK, bit);
-        peers &= bit ? bal : ~bal;
+        r[it] &= bit ? bal : ~bal;
       }
-      const uint16_t before = s_cnt[warp][d];
-      const uint32_t rank = before + __popc(peers & lt);
-      r[it / 2] = (it & 1) ? r[it / 2] | rank << 16 : rank;
+    }
+#pragma unroll
+    for (int it = 0; it < RS_IPL; ++it) {
+      const unsigned d = (unsigned)(k[it] >> shift) & dmask, peers = r[it];
+      const uint32_t before = s_cnt[warp][d];
+      r[it] = before + __popc(peers & lt);
       __syncwarp();
-      if (in && (peers >> lane) == 1u) s_cnt[warp][d] = (uint16_t)(before + __popc(peers));  // the last of them
+      if (base + it * 32 < nt && (peers >> lane) == 1u)  // the last of them
+        s_cnt[warp][d] = (uint16_t)(before + __popc(peers));
       __syncwarp();
     }
     __syncthreads();
@@ -210,7 +215,7 @@ __global__ void __launch_bounds__(RS_THREADS, RS_BLOCKS_PER_SM) rs_scatter_kerne
     __syncthreads();
 #pragma unroll
     for (int it = 0; it < RS_IPL; ++it)
-      if (base + it * 32 < nt) s_key[s_cnt[warp][(unsigned)(k[it] >> shift) & dmask] + ((r[it / 2] >> (16 * (it & 1))) & 0xffffu)] = k[it];
+      if (base + it * 32 < nt) s_key[s_cnt[warp][(unsigned)(k[it] >> shift) & dmask] + r[it]] = k[it];
     __syncthreads();
     for (int i = threadIdx.x; i < nt; i += RS_THREADS) {
       const uint64_t x = s_key[i];
