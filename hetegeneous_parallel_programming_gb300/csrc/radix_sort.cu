@@ -151,8 +151,10 @@ __global__ void __launch_bounds__(RS_THREADS) rs_scan_kernel(const uint32_t *__r
 // shared memory, and the tile leaves digit by digit, 10 keys (80 bytes) a
 // run on average.  Bound by memory: 16 bytes per key plus 8 for the
 // histogram.  33.6 M keys take 163 us, 3.3 TB/s (the direct scatter it
-// replaces 460; 16 keys a lane 202, 12 and a tile of 3072 185), the histogram
-// 46 us, 5.8 TB/s (172).
+// replaces 460; 16 keys a lane with the ballots of a round after the counters of
+// the one before 202), the histogram 46 us, 5.8 TB/s (172).  Keys a lane, by the
+// time of a whole R-MAT scale 21 build at four blocks an SM: 10 2562 us, 12 2766,
+// 14 at three 2639.  10 spills 8 bytes at that occupancy, 16 spilled 100.
 __global__ void __launch_bounds__(RS_THREADS, RS_BLOCKS_PER_SM) rs_scatter_kernel(
     const uint64_t *__restrict__ kin, uint64_t *__restrict__ kout, int64_t N, int shift, int dbits, int64_t chunk,
     const uint32_t *__restrict__ offs, int G) {
