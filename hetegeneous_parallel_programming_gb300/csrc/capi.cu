@@ -957,7 +957,7 @@ static tc_status count_dag_impl(tc_ctx *ctx, const tc_csr *dag_in, const tc_opts
   TC_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_flags, 0, sizeof(unsigned) * 8, ctx->stream));
   TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[1], ctx->stream));
   // A DAG row may hold any larger-or-smaller ids; only sortedness is required.
-  if (o.validate) TC_TRY(launch_validate(ctx, d, true));
+  TC_TRY(launch_dag_entries(ctx, d, o.validate != 0, src, indeg));
   TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[2], ctx->stream));
   TC_CHECK_CUDA(ctx, cudaMemcpyAsync(&ctx->h_pinned[1], ctx->d_flags, sizeof(unsigned) * 2, cudaMemcpyDeviceToHost,
                                      ctx->stream));
@@ -965,8 +965,6 @@ static tc_status count_dag_impl(tc_ctx *ctx, const tc_csr *dag_in, const tc_opts
   const unsigned flags = (unsigned)(ctx->h_pinned[1] & 0xffffffffu);
   if (flags) return set_error(ctx, TC_ERR_INVALID_GRAPH, "%s", flag_text(flags));
   TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[4], ctx->stream));
-  TC_TRY(launch_expand_src(ctx, d.rowptr, d.n, m, src));
-  TC_TRY(launch_indeg(ctx, d.col, d.n, m, indeg));
   // A row range is counted in place: its edges are entries [e0, e1) of the
   // column array, so the count runs on col + e0 with row pointers shifted by
   // -e0 (every row's list, inside the range or not, stays where it is).

@@ -49,10 +49,10 @@ struct DevDag {
 };
 
 // Validation: sets VF_* bits in ctx->d_flags[0].
-tc_status launch_validate(tc_ctx *ctx, const DevCSR &g, bool require_sorted_simple);
 tc_status launch_validate_rowptr(tc_ctx *ctx, const DevCSR &g);
-// in-degree of every vertex of a caller-oriented DAG (histogram of col)
-tc_status launch_indeg(tc_ctx *ctx, const int32_t *col, int64_t n, int64_t m, int32_t *indeg);
+// A caller-oriented DAG: row of every entry, in-degrees, and with `validate`
+// the checks of row pointers, ids, self loops and sorted rows.
+tc_status launch_dag_entries(tc_ctx *ctx, const DevCSR &g, bool validate, int32_t *src, int32_t *indeg);
 
 // Orientation.  Phase A (before the host learns m): degree keys, rank sort,
 // kept counts per row and per block.  Phase B: compaction + relabel sort.
@@ -101,8 +101,6 @@ tc_status orient_phase_a(tc_ctx *ctx, const DevCSR &g, OrientBufs &b);
 tc_status orient_phase_b(tc_ctx *ctx, const DevCSR &g, OrientBufs &b, int64_t m, bool want_perm,
                          bool want_dag_cols, DevDag *out);
 
-// Row of every entry of a CSR (for counting a caller-oriented DAG).
-tc_status launch_expand_src(tc_ctx *ctx, const int64_t *rowptr, int64_t n, int64_t m, int32_t *src);
 tc_status launch_shift_rowptr(tc_ctx *ctx, const int64_t *rowptr, int64_t n, int64_t shift, int64_t *out);
 
 // Counting.
