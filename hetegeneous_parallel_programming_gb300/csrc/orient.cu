@@ -1306,9 +1306,9 @@ tc_status orient_phase_b(tc_ctx *ctx, const DevCSR &g, OrientBufs &b, int64_t m,
 // the columns, in one pass over them.  Bound by the random in-degree atomics; a
 // block counts the ids that came first to a slot of a small table in shared
 // memory (mostly the common ones) and adds them once at its end.  DAG of 16.8 M
-// edges, whole call: 2826 us with a pass each for the checks, the sources and
-// the in-degrees, 2735 in one pass, 2717 with 2048 slots (2707 with 4096, whose
-// 32 KB are more to clear and add on small inputs).
+// edges, whole call: 2826 -> 2731 us against a pass each for the checks, the
+// sources and the in-degrees.  Of that the table gives 18 us; 4096 slots give 10
+// more there, but are twice as much to clear and add on small inputs.
 constexpr int DE_SLOTS = 2048;
 constexpr int DE_BLOCKS_PER_SM = 4;
 __global__ void __launch_bounds__(OR_THREADS) dag_entries_kernel(const int64_t *__restrict__ rowptr,
