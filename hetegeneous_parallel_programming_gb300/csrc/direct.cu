@@ -381,13 +381,13 @@ struct DirectDag {
 
 constexpr int DC_THREADS = 256;
 constexpr int DC_WARPS = DC_THREADS / 32;
-constexpr int DC_BLOCKS = 4;        // blocks per SM that the registers allow
+constexpr int DC_BLOCKS = 3;        // blocks per SM that the registers allow (and the 64 KB of bitmaps)
 constexpr int DC_WORDS = 2048;      // most shared-memory words of a warp: bitmaps of 65536 ids
 constexpr int DC_WORDS_MIN = 512;
 constexpr int DC_SMEM = DC_WARPS * DC_WORDS * (int)sizeof(uint32_t);
 constexpr int DC_SLOTS = 4, DC_SLOTS_HASHED = 2;  // rows at a time
 constexpr int DC_U = 4;             // searches in flight per lane
-constexpr int DC_GU = 2;            // 16-byte list loads in flight per lane
+constexpr int DC_GU = 3;            // 16-byte list loads in flight per lane
 constexpr int DC_RUNS = 4;          // more rows than this (and bitmaps) in 32 edges: all of them searched
 constexpr int DC_SEARCH = 8;        // target list this many times the row's: searched
 
@@ -404,7 +404,9 @@ constexpr int DC_SEARCH = 8;        // target list this many times the row's: se
 // list's entries are searched in the longer one, flattened over the lanes too.
 // Bound by instruction issue: the per-batch work (sums, bitmaps) is spread
 // over 32 edges whatever their rows, which took this kernel from 3.9 ms (a
-// pass per row) to 2.8 ms on 1024 mixed small graphs (49 M edges).
+// pass per row) to 2.8 ms on 1024 mixed small graphs (49 M edges).  Three
+// blocks with 3 loads in flight a lane against four with 2 (the bitmaps leave
+// room for three): 647 -> 625 us on 256 such graphs; 4 loads 637.
 // MODE 0: counts; 1: triangles of every vertex; 2: common neighbours of one
 // label.  In MODE 1 the hubs of a skewed graph are in most triangles, and
 // additions to one address take turns: the warps spread them over `copies`
