@@ -205,7 +205,7 @@ tc_status tc_batch_count(tc_ctx *ctx, const tc_batch *b, const tc_opts *opts_in,
     cudaGraph_t graph;
     TC_CHECK_CUDA(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
     DevDag dag;
-    tc_status s1 = orient_phase_b(ctx, d, ob, m, false, false, &dag);
+    tc_status s1 = orient_phase_b(ctx, d, ob, m, false, &dag);
     if (s1 == TC_OK) {
       cudaMemsetAsync(ctx->d_total, 0, sizeof(unsigned long long), ctx->stream);
       s1 = run_count(ctx, dag, o, cb, cnt, false);
@@ -279,7 +279,7 @@ tc_status tc_plan_arms(tc_ctx *ctx, const tc_csr *g, const tc_opts *opts_in, int
   float a, bb;
   TC_TRY(orient_front(ctx, d, o, ob, &m, &a, &bb));
   DevDag dag;
-  TC_TRY(orient_phase_b(ctx, d, ob, m, false, false, &dag));
+  TC_TRY(orient_phase_b(ctx, d, ob, m, false, &dag));
   const int64_t T = (m + TILE_EDGES - 1) / TILE_EDGES;
   *tiles_out = T;
   if (T > capacity || (T > 0 && !arms))
@@ -321,7 +321,7 @@ tc_status tc_tile_profile(tc_ctx *ctx, const tc_csr *g, float *features, float *
   float a, bb;
   TC_TRY(orient_front(ctx, d, o, ob, &m, &a, &bb));
   DevDag dag;
-  TC_TRY(orient_phase_b(ctx, d, ob, m, false, false, &dag));
+  TC_TRY(orient_phase_b(ctx, d, ob, m, false, &dag));
   const int64_t T = (m + TILE_EDGES - 1) / TILE_EDGES;
   *tiles_out = T;
   if (T > capacity || (T > 0 && (!features || !costs)))

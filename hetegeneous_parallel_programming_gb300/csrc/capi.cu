@@ -174,7 +174,7 @@ void orient_carve(const tc_ctx *ctx, int64_t n, int64_t nnz, bool perm, bool dag
   b.big_list = bump.take<int32_t>(n);
   b.huge_list = bump.take<int32_t>(n);
   b.seg_counts = bump.take<unsigned>(4);
-  b.rv = bump.take<int32_t>(nnz);
+  b.kv = bump.take<int32_t>(nnz);
   b.ncol = bump.take<int32_t>(mmax);
   b.nsrc = bump.take<int32_t>(mmax);
   b.perm = perm ? bump.take<uint32_t>(mmax) : nullptr;
@@ -638,7 +638,7 @@ tc_status tc_count(tc_ctx *ctx, const tc_csr *g, const tc_opts *opts_in, uint64_
                      (long long)edge_capacity, (long long)m);
   TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[4], ctx->stream));
   DevDag dag;
-  TC_TRY(orient_phase_b(ctx, d, ob, m, want_edges, false, &dag));
+  TC_TRY(orient_phase_b(ctx, d, ob, m, want_edges, &dag));
   TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[5], ctx->stream));
   TC_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_total, 0, sizeof(unsigned long long), ctx->stream));
   TC_TRY(run_count(ctx, dag, o, cb, d_out, true));
@@ -732,7 +732,7 @@ tc_status tc_count_labelled(tc_ctx *ctx, const tc_csr *g, const uint8_t *vertex_
                      (long long)edge_capacity, (long long)m);
   TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[4], ctx->stream));
   DevDag dag;
-  TC_TRY(orient_phase_b(ctx, d, ob, m, want_edges, false, &dag));
+  TC_TRY(orient_phase_b(ctx, d, ob, m, want_edges, &dag));
   TC_TRY(launch_relabel_u8(ctx, d_lab_in, ob.rank, d.n, d_lab));
   TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[5], ctx->stream));
   dag.vlabel = d_lab;
@@ -817,7 +817,7 @@ tc_status tc_count_vertices(tc_ctx *ctx, const tc_csr *g, const tc_opts *opts_in
   st.ms_h2d = elapsed(ctx->ev[0], ctx->ev[1]);
   TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[4], ctx->stream));
   DevDag dag;
-  TC_TRY(orient_phase_b(ctx, d, ob, m, false, false, &dag));
+  TC_TRY(orient_phase_b(ctx, d, ob, m, false, &dag));
   TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[5], ctx->stream));
   if (m > 0) TC_CHECK_CUDA(ctx, cudaMemsetAsync(d_top, 0, sizeof(uint32_t) * (size_t)m, ctx->stream));
   dag.top = d_top;
@@ -1074,7 +1074,7 @@ tc_status tc_orient(tc_ctx *ctx, const tc_csr *g, int64_t *dag_rowptr, int32_t *
   if (g->on_device) ob.dag_col = dag_colidx;
   DevDag dag;
   (void)dag;
-  TC_TRY(orient_phase_b(ctx, d, ob, m, false, true, nullptr));  // original-id columns only, no relabel
+  TC_TRY(orient_phase_b(ctx, d, ob, m, false, nullptr));  // original-id columns only, no relabel
   TC_CHECK_CUDA(ctx, cudaMemcpyAsync(d_rp, ob.orowptr, sizeof(int64_t) * (size_t)(d.n + 1), cudaMemcpyDeviceToDevice,
                                      ctx->stream));
   if (!g->on_device) {

@@ -70,9 +70,9 @@ struct OrientBufs {
   int2 *dv;                    // [n] (out-degree, in-degree) per relabelled vertex
   int32_t *mid_list, *big_list, *huge_list;  // [n] rows for the warp / block / global sorts
   unsigned *seg_counts;        // [4]: mid, big, huge rows; big rows left to the block sort
-  int32_t *rv = nullptr;       // [nnz] rank of every entry's target, written by the kept-count pass
+  int32_t *kv = nullptr;       // [nnz] kept entries' target ranks (ids with dag_col), at the start of each chunk
   // phase B
-  int32_t *ncol, *nsrc;        // [m]
+  int32_t *ncol, *nsrc;        // [nnz] relabelled columns and rows; nsrc first holds the kept entries' rows, as kv does
   uint32_t *perm;              // [m] original slot of each relabelled edge (optional)
   int32_t *dag_col;            // optional original-id DAG output [m]
   int G;                       // blocks of the entry-chunk kernels
@@ -82,9 +82,7 @@ struct OrientBufs {
   const int32_t *vgroup = nullptr;
   int group_bits = 0;
   // batched graphs whose column ids are local: the kept-count pass adds
-  // vtx_off[vgroup[u]] to every id of row u (and range-checks it); only the
-  // kept-count pass reads the column array then (the placement streams the
-  // target ranks it wrote)
+  // vtx_off[vgroup[u]] to every id of row u (and range-checks it)
   const int64_t *vtx_off = nullptr;
   // check ids, sortedness and self loops inside the kept-count pass
   bool validate = false;
@@ -98,8 +96,7 @@ struct OrientBufs {
 void orient_geometry(const tc_ctx *ctx, int64_t nnz, int pieces, int *G, int64_t *chunk);
 tc_status orient_phase_a(tc_ctx *ctx, const DevCSR &g, OrientBufs &b);
 // out == nullptr: only the original-id DAG columns (b.dag_col) are written.
-tc_status orient_phase_b(tc_ctx *ctx, const DevCSR &g, OrientBufs &b, int64_t m, bool want_perm,
-                         bool want_dag_cols, DevDag *out);
+tc_status orient_phase_b(tc_ctx *ctx, const DevCSR &g, OrientBufs &b, int64_t m, bool want_perm, DevDag *out);
 
 tc_status launch_shift_rowptr(tc_ctx *ctx, const int64_t *rowptr, int64_t n, int64_t shift, int64_t *out);
 

@@ -13,21 +13,6 @@ namespace tc {
 
 constexpr int OR_THREADS = 256;
 constexpr int OR_PER = ENTRY_TILE / OR_THREADS;  // 8 entries per thread per tile
-// Every relabelled entry's row (nsrc): 1: the placement writes it next to
-// its column (a second scattered store per entry); 2: the row sorts write it,
-// coalesced, for the rows they visit (rows of one entry included)
-#ifndef TC_PLACE_SRC
-#define TC_PLACE_SRC 2
-#endif
-constexpr bool PLACE_SRC = TC_PLACE_SRC == 1;
-constexpr bool SORT_SRC = TC_PLACE_SRC == 2;
-// 1: the placement reads each row's destination base from rowbase_kernel's
-// per-vertex array; 0: it gathers nrowptr[rank u] and orowptr[u] itself
-#ifndef TC_PLACE_ROWBASE
-#define TC_PLACE_ROWBASE 1
-#endif
-constexpr bool PLACE_ROWBASE = TC_PLACE_ROWBASE != 0;
-
 // src[b .. b + L) = r by threads tid, tid + nt, ... (the row sorts' nsrc writes)
 __device__ __forceinline__ void put_row_src(int32_t *__restrict__ src, int64_t b, int L, int32_t r, int tid, int nt) {
   if (src)
@@ -107,10 +92,16 @@ __global__ void rank_kernel(const uint64_t *__restrict__ keys, int64_t n, uint64
     rank[keys[r] & mask] = (int32_t)r;
 }
 
-// Kept entries per original row (warp-aggregated atomics) and per block chunk.
-// With VALIDATE it also performs validate_col_kernel's checks on the same
-// pass over the adjacency (ids in range, rows strictly ascending, no self
-// loops), so a validated call reads colidx once here instead of twice.
+// Kept entries per original row (warp-aggregated atomics) and per block chunk,
+// and the entries themselves: row in ku, target's rank (cols: the target) in
+// kv, compacted in input order at the start of the chunk's slice.
+// With VALIDATE it also checks the columns on the same pass over the adjacency
+// (ids in range, rows strictly ascending, no self loops), so a validated call
+// reads colidx once here instead of twice.
+// Bound by the random rank gathers, 102 G/s at R-MAT scale 22: loads issued
+// before the rows are known, or fewer of the others, gave nothing, and fewer
+// resident blocks lose 10 % of the orientation.  Compacting costs scale 24 0.3
+// ms (4.9 -> 5.2) and scale 22 nothing (1.31 -> 1.32).
 template <bool VALIDATE>
 __global__ void __launch_bounds__(OR_THREADS, 6) kept_count_kernel(const int64_t *__restrict__ rowptr,
                                                                const int32_t *__restrict__ col, int64_t n,
@@ -118,33 +109,41 @@ __global__ void __launch_bounds__(OR_THREADS, 6) kept_count_kernel(const int64_t
                                                                const int32_t *__restrict__ rank,
                                                                unsigned long long *__restrict__ kept,
                                                                int64_t *__restrict__ bcount, unsigned *flags,
-                                                               int b_off, int32_t *__restrict__ rv_out,
+                                                               int b_off, int32_t *__restrict__ ku,
+                                                               int32_t *__restrict__ kv, int cols,
                                                                const int32_t *__restrict__ vgroup,
                                                                const int64_t *__restrict__ vtx_off) {
   __shared__ int rows[row_slots<ENTRY_TILE>()];
   __shared__ int scan_tmp[32];
-  __shared__ unsigned long long bsum;
-  if (threadIdx.x == 0) bsum = 0;
+  constexpr int NW = OR_THREADS / 32;
+  __shared__ int s_wcnt[2][NW];
   const int blk = (int)blockIdx.x + b_off;  // block of the entry-chunk geometry
   const int64_t b = (int64_t)blk * chunk, e_end = min(nnz, b + chunk);
-  unsigned long long mine = 0;
+  ku += b;
+  kv += b;
   unsigned f = 0;
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned lt = lanemask_lt();
+  // warp w owns entries [w*32*OR_PER, (w+1)*32*OR_PER) of the tile, lane-
+  // strided so every load is coalesced; entry order = (k, lane) order
+  const int wbase = warp * 32 * OR_PER + lane;
   int64_t hint = -1;
+  uint32_t at = 0;  // kept entries of the chunk so far
+  int flip = 0;
   for (int64_t t0 = b; t0 < e_end; t0 += ENTRY_TILE) {
     const int64_t t1 = min(e_end, t0 + ENTRY_TILE);
     expand_rows<ENTRY_TILE>(rowptr, n, t0, t1, rows, scan_tmp, hint);
     // all loads of the tile first, then the rank gathers, then the counts
-    int32_t vv[OR_PER], rv[OR_PER];
+    int32_t vv[OR_PER], rv[OR_PER], uu[OR_PER];
 #pragma unroll
     for (int k = 0; k < OR_PER; ++k) {
-      const int64_t e = t0 + k * OR_THREADS + threadIdx.x;
+      const int64_t e = t0 + wbase + k * 32;
       vv[k] = e < t1 ? col[e] : -1;
     }
     if (vtx_off) {  // batched graphs: local ids plus the base of the row's graph (always range-checked)
 #pragma unroll
       for (int k = 0; k < OR_PER; ++k) {
-        const int64_t e = t0 + k * OR_THREADS + threadIdx.x;
+        const int64_t e = t0 + wbase + k * 32;
         if (e >= t1) continue;
         const int u = rows[rslot((int)(e - t0))];
         int64_t base = 0, size = 0;
@@ -163,16 +162,11 @@ __global__ void __launch_bounds__(OR_THREADS, 6) kept_count_kernel(const int64_t
     }
 #pragma unroll
     for (int k = 0; k < OR_PER; ++k) rv[k] = vv[k] >= 0 && (int64_t)vv[k] < n ? rank[vv[k]] : -1;
-    if (rv_out) {  // the placement streams these instead of gathering them again
-#pragma unroll
-      for (int k = 0; k < OR_PER; ++k) {
-        const int64_t e = t0 + k * OR_THREADS + threadIdx.x;
-        if (e < t1) rv_out[e] = rv[k];
-      }
-    }
+    unsigned bal[OR_PER];
+    int cnt = 0;
 #pragma unroll
     for (int k = 0; k < OR_PER; ++k) {
-      const int64_t e = t0 + k * OR_THREADS + threadIdx.x;
+      const int64_t e = t0 + wbase + k * 32;
       bool keep = false;
       int u = -1;
       if (e < t1) {
@@ -193,25 +187,40 @@ __global__ void __launch_bounds__(OR_THREADS, 6) kept_count_kernel(const int64_t
       const bool head = e < t1 && (lane == 0 || u != u_prev);
       const unsigned hm = __ballot_sync(TC_FULL_MASK, head);
       if (head && km) {
-        const unsigned later = hm & ~(lanemask_lt() | (1u << lane));  // first lanes of the following runs
-        const unsigned run = (later ? (later & (0u - later)) - 1u : 0xffffffffu) & ~lanemask_lt();
+        const unsigned later = hm & ~(lt | (1u << lane));  // first lanes of the following runs
+        const unsigned run = (later ? (later & (0u - later)) - 1u : 0xffffffffu) & ~lt;
         const unsigned c = __popc(km & run);
         if (c) atomicAdd(&kept[u], (unsigned long long)c);
       }
-      mine += keep ? 1 : 0;
+      bal[k] = km;
+      uu[k] = u;
+      if (cols) rv[k] = vv[k];
+      cnt += __popc(km);
     }
+    // the warps' counts, double-buffered (expand_rows of the next tile is the
+    // barrier between its writes and these reads): every warp sums for itself
+    if (lane == 0) s_wcnt[flip][warp] = cnt;
     __syncthreads();
+    const int wc = lane < NW ? s_wcnt[flip][lane] : 0;
+    uint32_t p = at + __reduce_add_sync(TC_FULL_MASK, lane < warp ? wc : 0);
+    at += __reduce_add_sync(TC_FULL_MASK, wc);
+    flip ^= 1;
+#pragma unroll
+    for (int k = 0; k < OR_PER; ++k) {
+      if ((bal[k] >> lane) & 1u) {
+        const uint32_t q = p + __popc(bal[k] & lt);
+        ku[q] = uu[k];
+        kv[q] = rv[k];
+      }
+      p += __popc(bal[k]);
+    }
   }
-  mine = warp_sum(mine);
-  if (lane == 0 && mine) atomicAdd(&bsum, mine);
   if (VALIDATE || vtx_off) {  // batch ids are range-checked even without validation
     f = __reduce_or_sync(TC_FULL_MASK, f);
     if (lane == 0 && f) atomicOr(flags, f);
   }
-  __syncthreads();
-  if (threadIdx.x == 0) bcount[blk] = (int64_t)bsum;
+  if (threadIdx.x == 0) bcount[blk] = (int64_t)at;
 }
-
 
 // Relabelled out-degree (for the row pointers, and with the DAG in-degree,
 // the symmetric degree minus the kept out-degree, as one 8-byte pair the
@@ -292,15 +301,13 @@ tc_status orient_phase_a(tc_ctx *ctx, const DevCSR &g, OrientBufs &b) {
       const int blocks = per < b.G - k * per ? per : b.G - k * per;
       if (b.pieces > 1) TC_CHECK_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->piece_ev[k], 0));
       if (b.validate)
-        kept_count_kernel<true><<<blocks, OR_THREADS, 0, ctx->stream>>>(g.rowptr, g.col, g.n, g.nnz, b.chunk,
-                                                                        b.rank, (unsigned long long *)b.kept,
-                                                                        b.bcount, ctx->d_flags, k * per, b.rv,
-                                                                        b.vgroup, b.vtx_off);
+        kept_count_kernel<true><<<blocks, OR_THREADS, 0, ctx->stream>>>(
+            g.rowptr, g.col, g.n, g.nnz, b.chunk, b.rank, (unsigned long long *)b.kept, b.bcount, ctx->d_flags,
+            k * per, b.nsrc, b.kv, b.dag_col != nullptr, b.vgroup, b.vtx_off);
       else
-        kept_count_kernel<false><<<blocks, OR_THREADS, 0, ctx->stream>>>(g.rowptr, g.col, g.n, g.nnz, b.chunk,
-                                                                         b.rank, (unsigned long long *)b.kept,
-                                                                         b.bcount, ctx->d_flags, k * per, b.rv,
-                                                                         b.vgroup, b.vtx_off);
+        kept_count_kernel<false><<<blocks, OR_THREADS, 0, ctx->stream>>>(
+            g.rowptr, g.col, g.n, g.nnz, b.chunk, b.rank, (unsigned long long *)b.kept, b.bcount, ctx->d_flags,
+            k * per, b.nsrc, b.kv, b.dag_col != nullptr, b.vgroup, b.vtx_off);
       TC_CHECK_LAUNCH(ctx);
     }
     TC_TRY(exclusive_scan_i64(ctx, b.bcount, b.bcount, b.G, b.sort_scratch, b.d_m));
@@ -317,92 +324,63 @@ tc_status orient_phase_a(tc_ctx *ctx, const DevCSR &g, OrientBufs &b) {
   classify_rows_kernel<<<grid_for(ctx, g.n, 256, 8), 256, 0, ctx->stream>>>(b.dnew, g.n, b.mid_list, b.big_list,
                                                                             b.huge_list, b.seg_counts);
   TC_CHECK_LAUNCH(ctx);
-  if (PLACE_ROWBASE) {  // into b.kept, whose counts are spent once orowptr and dnew are made
-    rowbase_kernel<<<grid_for(ctx, g.n, 256, 8), 256, 0, ctx->stream>>>(b.rank, b.nrowptr, b.orowptr, g.n, b.kept);
-    TC_CHECK_LAUNCH(ctx);
-  }
+  // into b.kept, whose counts are spent once orowptr and dnew are made
+  rowbase_kernel<<<grid_for(ctx, g.n, 256, 8), 256, 0, ctx->stream>>>(b.rank, b.nrowptr, b.orowptr, g.n, b.kept);
+  TC_CHECK_LAUNCH(ctx);
   return TC_OK;
 }
 
 // ---- phase B: direct placement + per-row sort ---------------------------------
 
-// Kept entry k (input order, original slot kpos) of row u goes to relabelled
-// slot nrowptr[rank u] + (kpos - orowptr[u]) with value rank v; rows are then
-// sorted by value.
-template <bool VALS, bool DAGCOL, bool RELABEL>
-__global__ void __launch_bounds__(OR_THREADS, 6) place_kernel(const int64_t *__restrict__ rowptr,
-                                                          const int32_t *__restrict__ col, int64_t n, int64_t nnz,
-                                                          int64_t chunk, const int32_t *__restrict__ rank,
+constexpr int PL_THREADS = 256;
+constexpr int PL_UNROLL = 4;
+
+// Kept entry p (input order over the whole graph) of row u goes to relabelled
+// slot rowbase[u] + p; rows are then sorted by value.  With COLS the entries
+// only close up in their order.  The blocks share the entries evenly, however
+// the chunks' slices are filled.
+// Bound by memory, 8 bytes read and 4 written in short runs per kept entry:
+// R-MAT scale 24 (260 M kept) 2.74 -> 0.65 ms and scale 22 855 -> 180 us
+// against a second pass over all entries that looked up their rows and
+// compared their ranks again.
+template <bool VALS, bool COLS>
+__global__ void __launch_bounds__(PL_THREADS) place_kernel(const int32_t *__restrict__ ku, const int32_t *__restrict__ kv,
+                                                          int64_t m, int64_t chunk, int G,
                                                           const int64_t *__restrict__ boff,
-                                                          const int64_t *__restrict__ orowptr,
-                                                          const int64_t *__restrict__ nrowptr,
-                                                          int32_t *__restrict__ ncol, int32_t *__restrict__ nsrc,
-                                                          uint32_t *__restrict__ perm,
-                                                          int32_t *__restrict__ dag_col,
-                                                          const int32_t *__restrict__ rv_in,
-                                                          const int64_t *__restrict__ rowbase) {
-  __shared__ int rows[row_slots<ENTRY_TILE>()];
-  __shared__ int scan_tmp[32];
-  constexpr int NW = OR_THREADS / 32;
-  __shared__ int s_wcnt[2][NW];
-  const int64_t b = (int64_t)blockIdx.x * chunk, e_end = min(nnz, b + chunk);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned lt = lanemask_lt();
-  long long carry = boff[blockIdx.x];
-  int64_t hint = -1;
-  int flip = 0;
-  for (int64_t t0 = b; t0 < e_end; t0 += ENTRY_TILE) {
-    const int64_t t1 = min(e_end, t0 + ENTRY_TILE);
-    expand_rows<ENTRY_TILE>(rowptr, n, t0, t1, rows, scan_tmp, hint);
-    // warp w owns entries [w*32*OR_PER, (w+1)*32*OR_PER) of the tile, lane-
-    // strided so every load is coalesced; entry order = (k, lane) order
-    const int wbase = warp * 32 * OR_PER;
-    int32_t vv[OR_PER], rv[OR_PER], uu[OR_PER];
+                                                          const int64_t *__restrict__ rowbase,
+                                                          int32_t *__restrict__ out, uint32_t *__restrict__ perm) {
+  const int64_t per = (m + gridDim.x - 1) / gridDim.x;
+  const int64_t p0 = (int64_t)blockIdx.x * per, p1 = min(m, p0 + per);
+  if (p0 >= p1) return;
+  int lo = 0, hi = G;  // the last slice that starts at or before p0
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (boff[mid] <= p0) lo = mid;
+    else hi = mid;
+  }
+  for (int s = lo; s < G; ++s) {
+    const int64_t s0 = boff[s], s1 = s + 1 < G ? boff[s + 1] : m;
+    if (s0 >= p1) break;
+    const int64_t a = max(p0, s0), b = min(p1, s1), shift = (int64_t)s * chunk - s0;
+    for (int64_t q = a + threadIdx.x; q < b; q += PL_THREADS * PL_UNROLL) {
+      int32_t u[PL_UNROLL], v[PL_UNROLL];
 #pragma unroll
-    for (int k = 0; k < OR_PER; ++k) {
-      const int i = wbase + k * 32 + lane;
-      const bool in = t0 + i < t1;
-      vv[k] = in && (DAGCOL || !rv_in) ? col[t0 + i] : -1;
-      uu[k] = in ? rows[rslot(i)] : -1;
-      if (rv_in) rv[k] = in ? rv_in[t0 + i] : -1;  // ranks of the targets, from the kept-count pass
-    }
-    if (!rv_in) {
-#pragma unroll
-      for (int k = 0; k < OR_PER; ++k) rv[k] = vv[k] >= 0 && (int64_t)vv[k] < n ? rank[vv[k]] : -1;
-    }
-    unsigned bal[OR_PER];
-    int cnt = 0;
-#pragma unroll
-    for (int k = 0; k < OR_PER; ++k) {
-      const bool keep = uu[k] >= 0 && rv[k] >= 0 && rv[k] > rank[uu[k]];
-      bal[k] = __ballot_sync(TC_FULL_MASK, keep);
-      cnt += __popc(bal[k]);
-    }
-    // the warps' counts, double-buffered (expand_rows of the next tile is the
-    // barrier between its writes and these reads): every warp sums for itself
-    if (lane == 0) s_wcnt[flip][warp] = cnt;
-    __syncthreads();
-    const int wc = lane < NW ? s_wcnt[flip][lane] : 0;
-    const int before = __reduce_add_sync(TC_FULL_MASK, lane < warp ? wc : 0);
-    const int tile_kept = __reduce_add_sync(TC_FULL_MASK, wc);
-    flip ^= 1;
-    long long pos = carry + before;
-#pragma unroll
-    for (int k = 0; k < OR_PER; ++k) {
-      if ((bal[k] >> lane) & 1u) {
-        const long long p = pos + __popc(bal[k] & lt);
-        const int u = uu[k];
-        if (RELABEL) {
-          const long long dst = PLACE_ROWBASE ? rowbase[u] + p : nrowptr[rank[u]] + (p - orowptr[u]);
-          ncol[dst] = rv[k];
-          if (PLACE_SRC) nsrc[dst] = rank[u];
-          if (VALS) perm[dst] = (uint32_t)p;
-        }
-        if (DAGCOL) dag_col[p] = vv[k];
+      for (int k = 0; k < PL_UNROLL; ++k) {
+        const int64_t p = q + k * PL_THREADS;
+        v[k] = p < b ? kv[shift + p] : 0;
+        u[k] = !COLS && p < b ? ku[shift + p] : 0;
       }
-      pos += __popc(bal[k]);
+      int64_t base[PL_UNROLL];
+#pragma unroll
+      for (int k = 0; k < PL_UNROLL; ++k) base[k] = !COLS && q + k * PL_THREADS < b ? rowbase[u[k]] : 0;
+#pragma unroll
+      for (int k = 0; k < PL_UNROLL; ++k) {
+        const int64_t p = q + k * PL_THREADS;
+        if (p >= b) break;
+        out[base[k] + p] = v[k];
+        if (VALS) perm[base[k] + p] = (uint32_t)p;
+      }
     }
-    carry += tile_kept;
   }
 }
 
@@ -1220,7 +1198,7 @@ __global__ void __launch_bounds__(1024) seg_sort_global_kernel(const int64_t *__
 template <bool VALS>
 static tc_status launch_row_sorts(tc_ctx *ctx, const DevCSR &g, OrientBufs &b) {
   uint32_t *pv = VALS ? b.perm : nullptr;
-  int32_t *sv = SORT_SRC ? b.nsrc : nullptr;  // rows written by the sorts (every row visits one)
+  int32_t *sv = b.nsrc;  // rows written by the sorts (every row visits one)
   if (VALS && g.n <= SEG_PACK_PLACE_MAX_N)
     seg_sort_pack_kernel<VALS, true><<<grid_for(ctx, g.n, 256, 8), 256, 0, ctx->stream>>>(b.nrowptr, g.n, b.ncol, pv, sv);
   else if (g.n <= SEG_PACK_MAX_N)
@@ -1268,23 +1246,21 @@ static tc_status launch_row_sorts(tc_ctx *ctx, const DevCSR &g, OrientBufs &b) {
   return TC_OK;
 }
 
-tc_status orient_phase_b(tc_ctx *ctx, const DevCSR &g, OrientBufs &b, int64_t m, bool want_perm, bool want_dag_cols,
-                         DevDag *out) {
-  const bool relabel = out != nullptr;
+tc_status orient_phase_b(tc_ctx *ctx, const DevCSR &g, OrientBufs &b, int64_t m, bool want_perm, DevDag *out) {
   if (g.nnz > 0 && m > 0) {
-#define TC_PLACE(V, D, R)                                                                                        \
-  place_kernel<V, D, R><<<b.G, OR_THREADS, 0, ctx->stream>>>(g.rowptr, g.col, g.n, g.nnz, b.chunk, b.rank, b.bcount, \
-                                                             b.orowptr, b.nrowptr, b.ncol, b.nsrc, b.perm, b.dag_col, \
-                                                             b.rv, b.kept)
-    if (!relabel) TC_PLACE(false, true, false);
-    else if (want_perm && want_dag_cols) TC_PLACE(true, true, true);
-    else if (want_perm) TC_PLACE(true, false, true);
-    else if (want_dag_cols) TC_PLACE(false, true, true);
-    else TC_PLACE(false, false, true);
-#undef TC_PLACE
+    const int blocks = grid_for(ctx, m, PL_THREADS * PL_UNROLL, 8);
+    if (!out)
+      place_kernel<false, true><<<blocks, PL_THREADS, 0, ctx->stream>>>(b.nsrc, b.kv, m, b.chunk, b.G, b.bcount, b.kept,
+                                                                        b.dag_col, nullptr);
+    else if (want_perm)
+      place_kernel<true, false><<<blocks, PL_THREADS, 0, ctx->stream>>>(b.nsrc, b.kv, m, b.chunk, b.G, b.bcount, b.kept,
+                                                                        b.ncol, b.perm);
+    else
+      place_kernel<false, false><<<blocks, PL_THREADS, 0, ctx->stream>>>(b.nsrc, b.kv, m, b.chunk, b.G, b.bcount, b.kept,
+                                                                         b.ncol, nullptr);
     TC_CHECK_LAUNCH(ctx);
   }
-  if (!relabel) return TC_OK;
+  if (!out) return TC_OK;
   // the row sorts keep entries inside their rows, so every entry's row
   // (nsrc) is the same before and after them
   if (m > 0) TC_TRY(want_perm ? launch_row_sorts<true>(ctx, g, b) : launch_row_sorts<false>(ctx, g, b));
