@@ -2543,7 +2543,9 @@ static int64_t pull_key_count(int64_t n, int64_t T, int block_tiles, PullKeys *p
 #endif
 // Bit rows of the hubs' out-lists, one warp per hub row: the warp clears the
 // row, then ORs in its entries, one OR per distinct word (lanes matched by
-// word).  Every entry of a hub row is a hub (it ranks above its row).  Nothing
+// word).  Every entry of a hub row is a hub and ranks above its row, and the
+// readers look above it only, so the 16-byte words below the row's own id are
+// left as they are: half of the 512 MB (R-MAT scale 18: 96 -> 56 us).  Nothing
 // is done when neither PULL nor the wedge tests read them (hub_bits_used).
 __global__ void hub_bits_kernel(DevDag g, int32_t hub0, int wpr4, const int64_t *__restrict__ qoff,
                                 uint4 *__restrict__ bits) {
@@ -2552,7 +2554,7 @@ __global__ void hub_bits_kernel(DevDag g, int32_t hub0, int wpr4, const int64_t 
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < g.n - hub0; row += warps) {
     uint4 *b4 = bits + row * wpr4;
-    for (int q = lane; q < wpr4; q += 32) b4[q] = make_uint4(0u, 0u, 0u, 0u);
+    for (int q = (int)(row >> 7) + lane; q < wpr4; q += 32) b4[q] = make_uint4(0u, 0u, 0u, 0u);
     __syncwarp();
     uint32_t *b = reinterpret_cast<uint32_t *>(b4);
     const int64_t e0 = g.rowptr[hub0 + row], e1 = g.rowptr[hub0 + row + 1];
