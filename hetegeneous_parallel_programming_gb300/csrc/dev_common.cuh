@@ -61,7 +61,7 @@ struct tc_ctx {
   // captured back half of the batched pipeline (batch.cu), keyed by shape,
   // options and the buffers it reads
   cudaGraphExec_t batch_exec = nullptr;
-  int64_t batch_key[14] = {};
+  int64_t batch_key[15] = {};
   int64_t batch_launches = 0;
   // captured front half (group ids, validation, ranks, kept counts, scans)
   cudaGraphExec_t batch_front_exec = nullptr;

@@ -50,3 +50,14 @@ def test_placement(engine, name):
     assert got == total
     drow, dcol = engine.orient(rowptr, colidx)[:2]
     assert np.array_equal(drow, orow) and np.array_equal(dcol, ocol)
+
+
+def test_batch_after_a_change_of_chunks(engine):
+    """The batch's captured second half holds the chunk geometry: a new one is captured when it changes."""
+    batch = tc.gen_batch_host(num_graphs=160, n_min=64, n_max=16384, seed=4)
+    want, _ = engine.batch_count(*batch)
+    was = engine.get_tuning()["orient_blocks_per_sm"]
+    for blocks in (was, 1, 9, was):
+        engine.set_tuning(orient_blocks_per_sm=blocks)
+        got, _ = engine.batch_count(*batch, validate=False)
+        assert np.array_equal(got, want)
