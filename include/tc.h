@@ -170,8 +170,9 @@ tc_status tc_count_dag_range(tc_ctx *ctx, const tc_csr *dag, int64_t row_begin, 
  * that contain u, and *total = number of triangles.  The per-vertex counts
  * the reference's CPU intersection (Graph::intersect_num, graph.cc:376-406)
  * is the building block of, e.g. for clustering coefficients
- * 2*t(u) / (deg(u)*(deg(u)-1)).  Runs the PULL arm on every tile (the
- * selector in opts is ignored; validate is honoured). */
+ * 2*t(u) / (deg(u)*(deg(u)-1)).  Runs on the PULL arm and the wedge tests
+ * of short rows, small graphs on the direct path (the selector in opts does
+ * not choose an arm; validate is honoured). */
 tc_status tc_count_vertices(tc_ctx *ctx, const tc_csr *g, const tc_opts *opts, uint64_t *total,
                             uint64_t *vertex_counts, tc_stats *stats);
 
@@ -180,8 +181,9 @@ tc_status tc_count_vertices(tc_ctx *ctx, const tc_csr *g, const tc_opts *opts, u
  * (Graph::intersect_num(v, u, label), graph.cc:376-391 with the label test);
  * *total sums them over all edges (the triangles whose highest vertex
  * carries the label).  vertex_labels: n bytes, input ids, memory kind of
- * g->on_device; edge_counts as for tc_count.  Runs the PULL arm on every
- * tile (the selector in opts is ignored; validate is honoured). */
+ * g->on_device; edge_counts as for tc_count.  Runs on the same kernels as
+ * tc_count_vertices (the selector in opts does not choose an arm; validate is
+ * honoured). */
 tc_status tc_count_labelled(tc_ctx *ctx, const tc_csr *g, const uint8_t *vertex_labels, int32_t label,
                             const tc_opts *opts, uint64_t *total, uint32_t *edge_counts, int64_t edge_capacity,
                             tc_stats *stats);
@@ -301,7 +303,9 @@ typedef struct tc_batch {
 } tc_batch;
 
 /* Count every graph of the batch in one pass of the engine over the batch's
- * disjoint union (one persistent launch per arm over (graph, tile) items).
+ * disjoint union: with the fixed selector and validation by the direct passes
+ * of small graphs, otherwise (or when the lists are too long for them) by one
+ * persistent launch per arm over (graph, tile) items.
  * totals [num_graphs] receives each graph's exact count (host memory). */
 tc_status tc_batch_count(tc_ctx *ctx, const tc_batch *b, const tc_opts *opts, uint64_t *totals,
                          tc_stats *stats);
