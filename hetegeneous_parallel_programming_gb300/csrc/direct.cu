@@ -117,17 +117,6 @@ __device__ __forceinline__ void entry_rows(const int64_t *__restrict__ rowptr, u
 // counting start and when they end.
 enum { DX_TOTAL, DX_M, DX_ALG, DX_FLAGS, DX_WORK, DX_GUESS, DX_MAXN, DX_DONE, DX_START, DX_COUNT, DX_END, DX_WORDS };
 
-// A small graph's passes are a few microseconds each, so a kernel's launch
-// overlaps the end of the one before it (programmatic dependent launch): it
-// lets its successor be scheduled as it starts, and waits here for its
-// predecessor's results.  With the results written by the last block and no
-// events between the passes, ER n = 300 went from 56.6 to 40.5 us a call, ER n
-// = 16384 from 68 to 51.
-__device__ __forceinline__ void begin_pass() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
 __device__ __forceinline__ unsigned long long clock_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -760,23 +749,6 @@ static unsigned long long direct_max_work(int64_t n, bool per_vertex) {
   const bool exact = n <= 32 * DC_WORDS;
   if (per_vertex) return exact ? 1ull << 29 : 1ull << 27;
   return exact ? 1ull << 30 : 3ull << 27;
-}
-
-// Launches a pass that calls begin_pass.
-template <typename... P, typename... A>
-static cudaError_t launch_pass(tc_ctx *ctx, void (*kernel)(P...), int grid, int threads, int smem, A... args) {
-  cudaLaunchAttribute at = {};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.dynamicSmemBytes = (size_t)smem;
-  cfg.stream = ctx->stream;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  ctx->launches++;
-  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
 tc_status direct_init(tc_ctx *ctx) {

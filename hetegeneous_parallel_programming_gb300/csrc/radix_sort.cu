@@ -96,6 +96,7 @@ __global__ void __launch_bounds__(RS_THREADS) rs_hist_kernel(const uint64_t *__r
                                                             uint32_t *__restrict__ hist,
                                                             uint32_t *__restrict__ total, int G) {
   __shared__ uint32_t cnt[RS_WARPS][256];
+  begin_pass();
   const int warp = threadIdx.x >> 5;
   for (int i = threadIdx.x; i < RS_WARPS * 256; i += RS_THREADS) (&cnt[0][0])[i] = 0;
   __syncthreads();
@@ -129,9 +130,10 @@ __global__ void __launch_bounds__(RS_THREADS) rs_hist_kernel(const uint64_t *__r
 // Digit offsets, block d for digit d: offs[d][b] = (keys with a smaller digit)
 // + (keys with digit d in blocks before b).
 __global__ void __launch_bounds__(RS_THREADS) rs_scan_kernel(const uint32_t *__restrict__ hist,
-                                                            const uint32_t *__restrict__ total,
+                                                            const uint32_t *total,
                                                             uint32_t *__restrict__ offs, int G) {
   __shared__ uint32_t tmp[33];
+  begin_pass();
   const int d = blockIdx.x;
   uint32_t run;
   block_exclusive_scan<uint32_t>((int)threadIdx.x < d ? total[threadIdx.x] : 0u, tmp, &run);
@@ -157,11 +159,12 @@ __global__ void __launch_bounds__(RS_THREADS) rs_scan_kernel(const uint32_t *__r
 // 14 at three 2639.  10 spills 8 bytes at that occupancy, 16 spilled 100.
 __global__ void __launch_bounds__(RS_THREADS, RS_BLOCKS_PER_SM) rs_scatter_kernel(
     const uint64_t *__restrict__ kin, uint64_t *__restrict__ kout, int64_t N, int shift, int dbits, int64_t chunk,
-    const uint32_t *__restrict__ offs, int G) {
+    const uint32_t *offs, int G) {
   __shared__ uint64_t s_key[RS_TILE];
   __shared__ uint16_t s_cnt[RS_WARPS][256];
   __shared__ uint32_t s_base[256];   // where the tile's digit d goes, minus its start in the tile
   __shared__ uint32_t tmp[33];
+  begin_pass();
   static_assert(RS_THREADS == 256, "one thread per digit");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, d_own = threadIdx.x;
   const unsigned lt = lanemask_lt(), dmask = (1u << dbits) - 1u;
@@ -240,13 +243,12 @@ tc_status radix_sort(tc_ctx *ctx, uint64_t *in, uint64_t *k0, uint64_t *k1, int6
   uint64_t *ka = in, *kb = k0;
   for (int p = 0, shift = begin_bit; p < passes; ++p) {
     const int dbits = (bits - (shift - begin_bit) + passes - p - 1) / (passes - p);  // even digits: longer runs
-    rs_hist_kernel<<<g.G, RS_THREADS, 0, ctx->stream>>>(ka, N, shift, (1u << dbits) - 1u, g.chunk, hist, total + p * 256,
-                                                        g.G);
-    TC_CHECK_LAUNCH(ctx);
-    rs_scan_kernel<<<1 << dbits, RS_THREADS, 0, ctx->stream>>>(hist, total + p * 256, offs, g.G);
-    TC_CHECK_LAUNCH(ctx);
-    rs_scatter_kernel<<<g.G, RS_THREADS, 0, ctx->stream>>>(ka, kb, N, shift, dbits, g.chunk, offs, g.G);
-    TC_CHECK_LAUNCH(ctx);
+    TC_CHECK_CUDA(ctx, launch_pass(ctx, rs_hist_kernel, g.G, RS_THREADS, 0, ka, N, shift, (1u << dbits) - 1u, g.chunk,
+                                   hist, total + p * 256, g.G));
+    TC_CHECK_CUDA(ctx, launch_pass(ctx, rs_scan_kernel, 1 << dbits, RS_THREADS, 0, hist, total + p * 256, offs,
+                                   g.G));
+    TC_CHECK_CUDA(ctx, launch_pass(ctx, rs_scatter_kernel, g.G, RS_THREADS, 0, ka, kb, N, shift, dbits, g.chunk,
+                                   offs, g.G));
     shift += dbits;
     ka = kb;
     kb = ka == k0 ? k1 : k0;
@@ -284,6 +286,7 @@ template <typename T>
 __global__ void __launch_bounds__(SC_THREADS) sc_reduce_kernel(const T *__restrict__ in, int64_t N,
                                                               int64_t chunk, int64_t *__restrict__ sums) {
   __shared__ long long tmp[33];
+  begin_pass();
   const int64_t b = (int64_t)blockIdx.x * chunk, e = min(N, b + chunk);
   long long s = 0;
   for (int64_t i = b + threadIdx.x; i < e; i += SC_THREADS) s += in[i];
@@ -294,6 +297,7 @@ __global__ void __launch_bounds__(SC_THREADS) sc_reduce_kernel(const T *__restri
 
 __global__ void __launch_bounds__(1024) sc_top_kernel(int64_t *sums, int G, int64_t *d_total_out) {
   __shared__ long long tmp[33];
+  begin_pass();
   // G <= 4 * SMs: at most a few items per thread
   const int per = (G + blockDim.x - 1) / blockDim.x;
   const int b = threadIdx.x * per, e = min(G, b + per);
@@ -314,8 +318,9 @@ __global__ void __launch_bounds__(1024) sc_top_kernel(int64_t *sums, int G, int6
 
 template <typename T>
 __global__ void __launch_bounds__(SC_THREADS) sc_down_kernel(const T *in, T *out, int64_t N,
-                                                            int64_t chunk, const int64_t *__restrict__ sums) {
+                                                            int64_t chunk, const int64_t *sums) {
   __shared__ long long tmp[33];
+  begin_pass();
   const int64_t b = (int64_t)blockIdx.x * chunk, e = min(N, b + chunk);
   long long carry = sums[blockIdx.x];
   for (int64_t t0 = b; t0 < e; t0 += SC_TILE) {
@@ -343,12 +348,9 @@ tc_status exclusive_scan_i64(tc_ctx *ctx, const int64_t *in, int64_t *out, int64
   if (N <= 0) return TC_OK;
   RsGeom g = sc_geom(ctx, N);
   int64_t *sums = (int64_t *)scratch;
-  sc_reduce_kernel<int64_t><<<g.G, SC_THREADS, 0, ctx->stream>>>(in, N, g.chunk, sums);
-  TC_CHECK_LAUNCH(ctx);
-  sc_top_kernel<<<1, 1024, 0, ctx->stream>>>(sums, g.G, d_total_out);
-  TC_CHECK_LAUNCH(ctx);
-  sc_down_kernel<int64_t><<<g.G, SC_THREADS, 0, ctx->stream>>>(in, out, N, g.chunk, sums);
-  TC_CHECK_LAUNCH(ctx);
+  TC_CHECK_CUDA(ctx, launch_pass(ctx, sc_reduce_kernel<int64_t>, g.G, SC_THREADS, 0, in, N, g.chunk, sums));
+  TC_CHECK_CUDA(ctx, launch_pass(ctx, sc_top_kernel, 1, 1024, 0, sums, g.G, d_total_out));
+  TC_CHECK_CUDA(ctx, launch_pass(ctx, sc_down_kernel<int64_t>, g.G, SC_THREADS, 0, in, out, N, g.chunk, sums));
   return TC_OK;
 }
 
@@ -356,12 +358,9 @@ tc_status exclusive_scan_u32(tc_ctx *ctx, const uint32_t *in, uint32_t *out, int
   if (N <= 0) return TC_OK;
   RsGeom g = sc_geom(ctx, N);
   int64_t *sums = (int64_t *)scratch;
-  sc_reduce_kernel<uint32_t><<<g.G, SC_THREADS, 0, ctx->stream>>>(in, N, g.chunk, sums);
-  TC_CHECK_LAUNCH(ctx);
-  sc_top_kernel<<<1, 1024, 0, ctx->stream>>>(sums, g.G, nullptr);
-  TC_CHECK_LAUNCH(ctx);
-  sc_down_kernel<uint32_t><<<g.G, SC_THREADS, 0, ctx->stream>>>(in, out, N, g.chunk, sums);
-  TC_CHECK_LAUNCH(ctx);
+  TC_CHECK_CUDA(ctx, launch_pass(ctx, sc_reduce_kernel<uint32_t>, g.G, SC_THREADS, 0, in, N, g.chunk, sums));
+  TC_CHECK_CUDA(ctx, launch_pass(ctx, sc_top_kernel, 1, 1024, 0, sums, g.G, nullptr));
+  TC_CHECK_CUDA(ctx, launch_pass(ctx, sc_down_kernel<uint32_t>, g.G, SC_THREADS, 0, in, out, N, g.chunk, sums));
   return TC_OK;
 }
 
