@@ -34,6 +34,7 @@ __global__ void gen_cl_kernel(uint64_t key, const uint64_t *cum, int64_t n, int6
 template <bool HALF>
 __global__ void edge_keys_kernel(const int32_t *__restrict__ src, const int32_t *__restrict__ dst, int64_t M,
                                  int64_t n, int bits, uint64_t *__restrict__ keys) {
+  begin_pass();
   const uint64_t sentinel = (bits >= 32) ? ~0ULL : ((1ULL << (2 * bits)) - 1);
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < M; i += (int64_t)gridDim.x * blockDim.x) {
     const int32_t u = src[i], v = dst[i];
@@ -63,10 +64,11 @@ constexpr int UQ_TILE = UQ_THREADS * UQ_PER;
 // Distinct keys of each tile (WRITE: to their place; off: the tiles' offsets).
 // Keys are sorted; the sentinel is not one.
 template <bool WRITE>
-__global__ void __launch_bounds__(UQ_THREADS) unique_kernel(const uint64_t *__restrict__ keys, int64_t N,
+__global__ void __launch_bounds__(UQ_THREADS) unique_kernel(const uint64_t *keys, int64_t N,
                                                            uint64_t sentinel, uint32_t *__restrict__ cnt,
-                                                           const uint32_t *__restrict__ off,
+                                                           const uint32_t *off,
                                                            uint64_t *__restrict__ out) {
+  begin_pass();
   __shared__ uint32_t s_w[UQ_THREADS / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t w0 = (int64_t)blockIdx.x * UQ_TILE + warp * (32 * UQ_PER);
@@ -107,6 +109,7 @@ __global__ void __launch_bounds__(UQ_THREADS) unique_kernel(const uint64_t *__re
 // start[r] = first of the E keys whose field (key >> shift) & mask is >= r, r in [0, n].
 __global__ void field_start_kernel(const uint64_t *__restrict__ keys, int64_t E, int shift, uint64_t mask, int64_t n,
                                    uint32_t *__restrict__ start) {
+  begin_pass();
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r <= n; r += (int64_t)gridDim.x * blockDim.x) {
     uint32_t lo = 0, hi = (uint32_t)E;
     while (lo < hi) {
@@ -122,6 +125,7 @@ __global__ void field_start_kernel(const uint64_t *__restrict__ keys, int64_t E,
 // neighbour the other field, its slot i + shift_by[row + add].
 __global__ void half_rows_kernel(const uint64_t *__restrict__ keys, int64_t E, int bits, int row_shift,
                                  const uint32_t *__restrict__ shift_by, int add, int32_t *__restrict__ col) {
+  begin_pass();
   const uint64_t mask = (1ULL << bits) - 1;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < E; i += (int64_t)gridDim.x * blockDim.x) {
     const uint64_t k = keys[i];
@@ -132,12 +136,14 @@ __global__ void half_rows_kernel(const uint64_t *__restrict__ keys, int64_t E, i
 
 __global__ void add_starts_kernel(const uint32_t *__restrict__ a, const uint32_t *__restrict__ b, int64_t n,
                                   int64_t *__restrict__ rowptr) {
+  begin_pass();
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r <= n; r += (int64_t)gridDim.x * blockDim.x)
     rowptr[r] = (int64_t)a[r] + (int64_t)b[r];
 }
 
 __global__ void unique_flag_kernel(const uint64_t *__restrict__ keys, int64_t N, uint64_t sentinel,
                                    int64_t *__restrict__ flag) {
+  begin_pass();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
     const uint64_t k = keys[i];
     flag[i] = (k != sentinel && (i == 0 || keys[i - 1] != k)) ? 1 : 0;
@@ -147,6 +153,7 @@ __global__ void unique_flag_kernel(const uint64_t *__restrict__ keys, int64_t N,
 __global__ void unique_scatter_kernel(const uint64_t *__restrict__ keys, const int64_t *__restrict__ pos, int64_t N,
                                       uint64_t sentinel, int bits, int32_t *__restrict__ col,
                                       unsigned long long *__restrict__ deg) {
+  begin_pass();
   const uint64_t mask = (1ULL << bits) - 1;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
     const uint64_t k = keys[i];
@@ -255,22 +262,21 @@ tc_status tc_csr_from_edges(tc_ctx *ctx, int64_t n, int64_t M, const int32_t *sr
   if (M > 0) {
     uint64_t *sk = nullptr;
     if (half) {
-      edge_keys_kernel<true><<<grid_for(ctx, M, 256, 8), 256, 0, ctx->stream>>>(dsrc, ddst, M, n, bits, k0);
-      TC_CHECK_LAUNCH(ctx);
+      TC_CHECK_CUDA(ctx, launch_pass(ctx, edge_keys_kernel<true>, grid_for(ctx, M, 256, 8), 256, 0, dsrc, ddst, M, n,
+                                     bits, k0));
       TC_TRY(radix_sort(ctx, k0, k1, k0, N, 0, 2 * bits, scratch, &sk));
-      unique_kernel<false><<<(unsigned)tiles, UQ_THREADS, 0, ctx->stream>>>(sk, N, sentinel, tile_cnt, nullptr, nullptr);
-      TC_CHECK_LAUNCH(ctx);
+      TC_CHECK_CUDA(ctx, launch_pass(ctx, unique_kernel<false>, (unsigned)tiles, UQ_THREADS, 0, sk, N, sentinel,
+                                     tile_cnt, nullptr, nullptr));
       TC_CHECK_CUDA(ctx, cudaMemsetAsync(tile_cnt + tiles, 0, sizeof(uint32_t), ctx->stream));
       TC_TRY(exclusive_scan_u32(ctx, tile_cnt, tile_cnt, tiles + 1, scratch));
       ctx->h_pinned[0] = 0;
       TC_CHECK_CUDA(ctx, cudaMemcpyAsync(&ctx->h_pinned[0], tile_cnt + tiles, sizeof(uint32_t), cudaMemcpyDeviceToHost,
                                          ctx->stream));
     } else {
-      edge_keys_kernel<false><<<grid_for(ctx, M, 256, 8), 256, 0, ctx->stream>>>(dsrc, ddst, M, n, bits, k0);
-      TC_CHECK_LAUNCH(ctx);
+      TC_CHECK_CUDA(ctx, launch_pass(ctx, edge_keys_kernel<false>, grid_for(ctx, M, 256, 8), 256, 0, dsrc, ddst, M, n,
+                                     bits, k0));
       TC_TRY(radix_sort(ctx, k0, k1, k0, N, 0, 2 * bits, scratch, &sk));
-      unique_flag_kernel<<<grid_for(ctx, N, 256, 8), 256, 0, ctx->stream>>>(sk, N, sentinel, flag);
-      TC_CHECK_LAUNCH(ctx);
+      TC_CHECK_CUDA(ctx, launch_pass(ctx, unique_flag_kernel, grid_for(ctx, N, 256, 8), 256, 0, sk, N, sentinel, flag));
       TC_TRY(exclusive_scan_i64(ctx, flag, flag, N, scratch, (int64_t *)&ctx->d_total[0]));
       TC_CHECK_CUDA(ctx, cudaMemcpyAsync(&ctx->h_pinned[0], ctx->d_total, sizeof(int64_t), cudaMemcpyDeviceToHost,
                                          ctx->stream));
@@ -286,23 +292,22 @@ tc_status tc_csr_from_edges(tc_ctx *ctx, int64_t n, int64_t M, const int32_t *sr
     if (half) {
       const uint64_t mask = (1ULL << bits) - 1;
       uint64_t *uk = sk == k0 ? k1 : k0, *bk = nullptr;
-      unique_kernel<true><<<(unsigned)tiles, UQ_THREADS, 0, ctx->stream>>>(sk, N, sentinel, nullptr, tile_cnt, uk);
-      TC_CHECK_LAUNCH(ctx);
-      field_start_kernel<<<grid_for(ctx, n + 1, 256, 8), 256, 0, ctx->stream>>>(uk, E, bits, mask, n, first);
-      TC_CHECK_LAUNCH(ctx);
+      TC_CHECK_CUDA(ctx, launch_pass(ctx, unique_kernel<true>, (unsigned)tiles, UQ_THREADS, 0, sk, N, sentinel,
+                                     nullptr, tile_cnt, uk));
+      TC_CHECK_CUDA(ctx, launch_pass(ctx, field_start_kernel, grid_for(ctx, n + 1, 256, 8), 256, 0, uk, E, bits, mask,
+                                     n, first));
       TC_TRY(radix_sort(ctx, uk, sk, k2, E, 0, bits, scratch, &bk));
-      field_start_kernel<<<grid_for(ctx, n + 1, 256, 8), 256, 0, ctx->stream>>>(bk, E, 0, mask, n, second);
-      TC_CHECK_LAUNCH(ctx);
+      TC_CHECK_CUDA(ctx, launch_pass(ctx, field_start_kernel, grid_for(ctx, n + 1, 256, 8), 256, 0, bk, E, 0, mask, n,
+                                     second));
       if (E > 0) {
-        half_rows_kernel<<<grid_for(ctx, E, 256, 8), 256, 0, ctx->stream>>>(uk, E, bits, bits, second, 1, dcol);
-        TC_CHECK_LAUNCH(ctx);
-        half_rows_kernel<<<grid_for(ctx, E, 256, 8), 256, 0, ctx->stream>>>(bk, E, bits, 0, first, 0, dcol);
-        TC_CHECK_LAUNCH(ctx);
+        TC_CHECK_CUDA(ctx, launch_pass(ctx, half_rows_kernel, grid_for(ctx, E, 256, 8), 256, 0, uk, E, bits, bits,
+                                       second, 1, dcol));
+        TC_CHECK_CUDA(ctx, launch_pass(ctx, half_rows_kernel, grid_for(ctx, E, 256, 8), 256, 0, bk, E, bits, 0, first,
+                                       0, dcol));
       }
     } else {
-      unique_scatter_kernel<<<grid_for(ctx, N, 256, 8), 256, 0, ctx->stream>>>(sk, flag, N, sentinel, bits, dcol,
-                                                                               (unsigned long long *)deg);
-      TC_CHECK_LAUNCH(ctx);
+      TC_CHECK_CUDA(ctx, launch_pass(ctx, unique_scatter_kernel, grid_for(ctx, N, 256, 8), 256, 0, sk, flag, N,
+                                     sentinel, bits, dcol, (unsigned long long *)deg));
     }
     if (!on_device && nnz > 0)
       TC_CHECK_CUDA(ctx, cudaMemcpyAsync(colidx, dcol_stage, sizeof(int32_t) * nnz, cudaMemcpyDeviceToHost,
@@ -311,8 +316,8 @@ tc_status tc_csr_from_edges(tc_ctx *ctx, int64_t n, int64_t M, const int32_t *sr
     *nnz_out = 0;
   }
   if (half) {
-    add_starts_kernel<<<grid_for(ctx, n + 1, 256, 8), 256, 0, ctx->stream>>>(first, second, n, drow);
-    TC_CHECK_LAUNCH(ctx);
+    TC_CHECK_CUDA(ctx, launch_pass(ctx, add_starts_kernel, grid_for(ctx, n + 1, 256, 8), 256, 0, first, second, n,
+                                   drow));
   } else {
     TC_TRY(exclusive_scan_i64(ctx, deg, drow, n + 1, scratch, nullptr));
   }

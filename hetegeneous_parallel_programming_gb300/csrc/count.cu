@@ -386,9 +386,10 @@ __global__ void __launch_bounds__(PLAN_THREADS) learned_select_kernel(int64_t T,
 // and resets the queue heads.  bin_fill starts at zero.
 __global__ void __launch_bounds__(Q_THREADS) queue_kernel(int64_t T, const int32_t *__restrict__ arm,
                                                          const uint32_t *__restrict__ tile_level,
-                                                         const uint32_t *__restrict__ bin_cnt,
+                                                         const uint32_t *bin_cnt,
                                                          uint32_t *__restrict__ bin_fill, int64_t *__restrict__ qoff,
                                                          uint32_t *__restrict__ qtiles, unsigned *__restrict__ heads) {
+  begin_pass();
   __shared__ uint32_t start[Q_BINS];
   __shared__ uint32_t tmp[33];
   constexpr int PER = Q_BINS / Q_THREADS;
@@ -2251,7 +2252,7 @@ constexpr int WD_U = 4;                   // loads or searches in flight per lan
 constexpr int64_t WD_MIN_TILES = 1024;    // without PULL tiles, fewer do not pay for building the bit rows
 
 // Whether the hub bit rows are built: some tile is PULL's, or BSEARCH_4 has many.
-__device__ __forceinline__ bool hub_bits_used(const int64_t *__restrict__ qoff) {
+__device__ __forceinline__ bool hub_bits_used(const int64_t *qoff) {
   return qoff[TC_ARM_PULL + 1] > qoff[TC_ARM_PULL] ||
          qoff[TC_ARM_BSEARCH_4 + 1] - qoff[TC_ARM_BSEARCH_4] >= WD_MIN_TILES;
 }
@@ -2547,8 +2548,9 @@ static int64_t pull_key_count(int64_t n, int64_t T, int block_tiles, PullKeys *p
 // readers look above it only, so the 16-byte words below the row's own id are
 // left as they are: half of the 512 MB (R-MAT scale 18: 96 -> 56 us).  Nothing
 // is done when neither PULL nor the wedge tests read them (hub_bits_used).
-__global__ void hub_bits_kernel(DevDag g, int32_t hub0, int wpr4, const int64_t *__restrict__ qoff,
+__global__ void hub_bits_kernel(DevDag g, int32_t hub0, int wpr4, const int64_t *qoff,
                                 uint4 *__restrict__ bits) {
+  begin_pass();
   if (!hub_bits_used(qoff)) return;
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
@@ -2679,9 +2681,8 @@ tc_status run_count(tc_ctx *ctx, const DevDag &g_in, const tc_opts &opts_in, Cou
                                              cb.tile_bytes, bin_cnt, cb.arm_bytes);
       TC_CHECK_LAUNCH(ctx);
     }
-    queue_kernel<<<(unsigned)((T + Q_TILES - 1) / Q_TILES), Q_THREADS, 0, ctx->stream>>>(
-        T, cb.arm, cb.tile_level, bin_cnt, bin_fill, cb.qoff, cb.qtiles, ctx->d_heads);
-    TC_CHECK_LAUNCH(ctx);
+    TC_CHECK_CUDA(ctx, launch_pass(ctx, queue_kernel, (unsigned)((T + Q_TILES - 1) / Q_TILES), Q_THREADS, 0, T,
+                                   cb.arm, cb.tile_level, bin_cnt, bin_fill, cb.qoff, cb.qtiles, ctx->d_heads));
   }
   if (cb.tile_cycles && T > 0)
     TC_CHECK_CUDA(ctx, cudaMemsetAsync(cb.tile_cycles, 0, sizeof(unsigned long long) * T, ctx->stream));
@@ -2691,8 +2692,8 @@ tc_status run_count(tc_ctx *ctx, const DevDag &g_in, const tc_opts &opts_in, Cou
   // DAG (rows hold higher ids only)
   const int32_t hub0 = (int32_t)(g.n - hub_rows(g.n));
   if (T > 0 && g.restrict_after && arm_possible(opts, TC_ARM_PULL) && (!g.top || wedge != PLAN_NO_WEDGE)) {
-    hub_bits_kernel<<<ctx->num_sms * 8, 256, 0, ctx->stream>>>(g, hub0, hub_wpr4(g.n), cb.qoff, cb.hub_bits);
-    TC_CHECK_LAUNCH(ctx);
+    TC_CHECK_CUDA(ctx, launch_pass(ctx, hub_bits_kernel, ctx->num_sms * 8, 256, 0, g, hub0, hub_wpr4(g.n), cb.qoff,
+                                   cb.hub_bits));
     g.hub_bits = cb.hub_bits;
     g.hub_wpr4 = hub_wpr4(g.n);
   }
@@ -2781,20 +2782,21 @@ __global__ void __launch_bounds__(VS_THREADS) vertex_sum_kernel(DevDag g, const 
 
 __global__ void vertex_unrank_kernel(const unsigned long long *__restrict__ t, const int32_t *__restrict__ rank,
                                      int64_t n, unsigned long long *__restrict__ out) {
+  begin_pass();
   for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.x * blockDim.x)
     out[u] = t[rank[u]];
 }
 
 __global__ void relabel_u8_kernel(const uint8_t *__restrict__ in, const int32_t *__restrict__ rank, int64_t n,
                                   uint8_t *__restrict__ out) {
+  begin_pass();
   for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.x * blockDim.x)
     out[rank[u]] = in[u];
 }
 
 tc_status launch_relabel_u8(tc_ctx *ctx, const uint8_t *in, const int32_t *rank, int64_t n, uint8_t *out) {
   if (n <= 0) return TC_OK;
-  relabel_u8_kernel<<<grid_for(ctx, n, 256, 8), 256, 0, ctx->stream>>>(in, rank, n, out);
-  TC_CHECK_LAUNCH(ctx);
+  TC_CHECK_CUDA(ctx, launch_pass(ctx, relabel_u8_kernel, grid_for(ctx, n, 256, 8), 256, 0, in, rank, n, out));
   return TC_OK;
 }
 
@@ -2805,8 +2807,7 @@ tc_status launch_vertex_sums(tc_ctx *ctx, const DevDag &g, const uint32_t *c, co
     vertex_sum_kernel<<<grid_for(ctx, g.m, VS_THREADS, 3), VS_THREADS, 0, ctx->stream>>>(g, c, top, t);
     TC_CHECK_LAUNCH(ctx);
   }
-  vertex_unrank_kernel<<<grid_for(ctx, g.n, 256, 8), 256, 0, ctx->stream>>>(t, rank, g.n, out);
-  TC_CHECK_LAUNCH(ctx);
+  TC_CHECK_CUDA(ctx, launch_pass(ctx, vertex_unrank_kernel, grid_for(ctx, g.n, 256, 8), 256, 0, t, rank, g.n, out));
   return TC_OK;
 }
 

@@ -54,6 +54,7 @@ static inline int vertex_bits(int64_t n) { return bit_width_u64(n > 1 ? (uint64_
 
 __global__ void validate_rowptr_kernel(const int64_t *__restrict__ rowptr, int64_t n, int64_t nnz,
                                        unsigned *flags) {
+  begin_pass();
   unsigned f = 0;
   for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u <= n; u += (int64_t)gridDim.x * blockDim.x) {
     const int64_t a = rowptr[u];
@@ -67,9 +68,8 @@ __global__ void validate_rowptr_kernel(const int64_t *__restrict__ rowptr, int64
 }
 
 tc_status launch_validate_rowptr(tc_ctx *ctx, const DevCSR &g) {
-  validate_rowptr_kernel<<<grid_for(ctx, g.n + 1, 256, 8), 256, 0, ctx->stream>>>(g.rowptr, g.n, g.nnz,
-                                                                                  ctx->d_flags);
-  TC_CHECK_LAUNCH(ctx);
+  TC_CHECK_CUDA(ctx, launch_pass(ctx, validate_rowptr_kernel, grid_for(ctx, g.n + 1, 256, 8), 256, 0, g.rowptr, g.n,
+                                 g.nnz, ctx->d_flags));
   return TC_OK;
 }
 
@@ -77,6 +77,7 @@ tc_status launch_validate_rowptr(tc_ctx *ctx, const DevCSR &g) {
 
 __global__ void deg_key_kernel(const int64_t *__restrict__ rowptr, int64_t n, int bits,
                                const int32_t *__restrict__ vgroup, uint64_t *__restrict__ keys) {
+  begin_pass();
   const uint64_t dmax = (bits >= 63) ? ~0ULL : ((1ULL << bits) - 1);
   for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.x * blockDim.x) {
     int64_t d = rowptr[u + 1] - rowptr[u];
@@ -88,6 +89,7 @@ __global__ void deg_key_kernel(const int64_t *__restrict__ rowptr, int64_t n, in
 }
 
 __global__ void rank_kernel(const uint64_t *__restrict__ keys, int64_t n, uint64_t mask, int32_t *__restrict__ rank) {
+  begin_pass();
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x)
     rank[keys[r] & mask] = (int32_t)r;
 }
@@ -228,6 +230,7 @@ __global__ void __launch_bounds__(OR_THREADS, 6) kept_count_kernel(const int64_t
 __global__ void dnew_kernel(const int64_t *__restrict__ kept, const int32_t *__restrict__ rank,
                             const int64_t *__restrict__ rowptr, int64_t n, int64_t *__restrict__ dnew,
                             int2 *__restrict__ dv) {
+  begin_pass();
   for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.x * blockDim.x) {
     const int32_t r = rank[u];
     const int64_t k = kept[u];
@@ -243,6 +246,7 @@ __global__ void dnew_kernel(const int64_t *__restrict__ kept, const int32_t *__r
 // placement reads one value per row instead of gathering nrowptr[rank u].
 __global__ void rowbase_kernel(const int32_t *__restrict__ rank, const int64_t *__restrict__ nrowptr,
                                const int64_t *__restrict__ orowptr, int64_t n, int64_t *__restrict__ rowbase) {
+  begin_pass();
   for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.x * blockDim.x)
     rowbase[u] = nrowptr[rank[u]] - orowptr[u];
 }
@@ -258,6 +262,7 @@ constexpr int SEG_SMEM_MAX = 4096;
 __global__ void classify_rows_kernel(const int64_t *__restrict__ len, int64_t n, int32_t *__restrict__ mid_list,
                                      int32_t *__restrict__ big_list, int32_t *__restrict__ huge_list,
                                      unsigned *counts) {
+  begin_pass();
   const int lane = threadIdx.x & 31;
   const unsigned lt = lanemask_lt();
   for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n; base += (int64_t)gridDim.x * blockDim.x) {
@@ -284,14 +289,14 @@ tc_status orient_phase_a(tc_ctx *ctx, const DevCSR &g, OrientBufs &b) {
   orient_geometry(ctx, g.nnz, b.pieces, &b.G, &b.chunk);
   const int gbits = b.vgroup ? b.group_bits : 0;
   if (2 * bits + gbits > 64) return set_error(ctx, TC_ERR_UNSUPPORTED, "rank key needs %d bits", 2 * bits + gbits);
-  deg_key_kernel<<<grid_for(ctx, g.n, 256, 8), 256, 0, ctx->stream>>>(g.rowptr, g.n, bits, b.vgroup, b.vkeys0);
-  TC_CHECK_LAUNCH(ctx);
+  TC_CHECK_CUDA(ctx, launch_pass(ctx, deg_key_kernel, grid_for(ctx, g.n, 256, 8), 256, 0, g.rowptr, g.n, bits,
+                                 b.vgroup, b.vkeys0));
   // Ids start in ascending order and the sort is stable, so sorting on the
   // (group, degree) bits alone yields the (group, degree, id) order.
   uint64_t *sorted = nullptr;
   TC_TRY(radix_sort(ctx, b.vkeys0, b.vkeys1, b.vkeys0, g.n, bits, 2 * bits + gbits, b.sort_scratch, &sorted));
-  rank_kernel<<<grid_for(ctx, g.n, 256, 8), 256, 0, ctx->stream>>>(sorted, g.n, (1ULL << bits) - 1, b.rank);
-  TC_CHECK_LAUNCH(ctx);
+  TC_CHECK_CUDA(ctx, launch_pass(ctx, rank_kernel, grid_for(ctx, g.n, 256, 8), 256, 0, sorted, g.n,
+                                 (1ULL << bits) - 1, b.rank));
   TC_CHECK_CUDA(ctx, cudaMemsetAsync(b.kept, 0, sizeof(int64_t) * (size_t)(g.n + 1), ctx->stream));
   if (g.nnz > 0) {
     // one launch per arriving piece of the column array (one piece when it
@@ -316,17 +321,15 @@ tc_status orient_phase_a(tc_ctx *ctx, const DevCSR &g, OrientBufs &b) {
   }
   // original-order DAG rowptr, relabelled rowptr, and the row classes
   TC_TRY(exclusive_scan_i64(ctx, b.kept, b.orowptr, g.n + 1, b.sort_scratch, nullptr));
-  dnew_kernel<<<grid_for(ctx, g.n, 256, 8), 256, 0, ctx->stream>>>(b.kept, b.rank, g.rowptr, g.n, b.dnew,
-                                                                    b.dv);
-  TC_CHECK_LAUNCH(ctx);
+  TC_CHECK_CUDA(ctx, launch_pass(ctx, dnew_kernel, grid_for(ctx, g.n, 256, 8), 256, 0, b.kept, b.rank, g.rowptr, g.n,
+                                 b.dnew, b.dv));
   TC_TRY(exclusive_scan_i64(ctx, b.dnew, b.nrowptr, g.n + 1, b.sort_scratch, nullptr));
   TC_CHECK_CUDA(ctx, cudaMemsetAsync(b.seg_counts, 0, sizeof(unsigned) * 4, ctx->stream));
-  classify_rows_kernel<<<grid_for(ctx, g.n, 256, 8), 256, 0, ctx->stream>>>(b.dnew, g.n, b.mid_list, b.big_list,
-                                                                            b.huge_list, b.seg_counts);
-  TC_CHECK_LAUNCH(ctx);
+  TC_CHECK_CUDA(ctx, launch_pass(ctx, classify_rows_kernel, grid_for(ctx, g.n, 256, 8), 256, 0, b.dnew, g.n,
+                                 b.mid_list, b.big_list, b.huge_list, b.seg_counts));
   // into b.kept, whose counts are spent once orowptr and dnew are made
-  rowbase_kernel<<<grid_for(ctx, g.n, 256, 8), 256, 0, ctx->stream>>>(b.rank, b.nrowptr, b.orowptr, g.n, b.kept);
-  TC_CHECK_LAUNCH(ctx);
+  TC_CHECK_CUDA(ctx, launch_pass(ctx, rowbase_kernel, grid_for(ctx, g.n, 256, 8), 256, 0, b.rank, b.nrowptr,
+                                 b.orowptr, g.n, b.kept));
   return TC_OK;
 }
 
@@ -349,6 +352,7 @@ __global__ void __launch_bounds__(PL_THREADS) place_kernel(const int32_t *__rest
                                                           const int64_t *__restrict__ boff,
                                                           const int64_t *__restrict__ rowbase,
                                                           int32_t *__restrict__ out, uint32_t *__restrict__ perm) {
+  begin_pass();
   const int64_t per = (m + gridDim.x - 1) / gridDim.x;
   const int64_t p0 = (int64_t)blockIdx.x * per, p1 = min(m, p0 + per);
   if (p0 >= p1) return;
@@ -630,6 +634,7 @@ template <bool VALS, bool PLACED>
 __global__ void __launch_bounds__(256) seg_sort_pack_kernel(const int64_t *__restrict__ nrowptr, int64_t n,
                                                            int32_t *__restrict__ ncol, uint32_t *__restrict__ perm,
                                                            int32_t *__restrict__ src) {
+  begin_pass();
   __shared__ int32_t s_row[8][2][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const unsigned lt = lanemask_lt(), le = lt | (1u << lane);
@@ -844,6 +849,7 @@ __global__ void __launch_bounds__(256) seg_sort_warpreg_kernel(const int64_t *__
                                                               const int32_t *__restrict__ list,
                                                               const unsigned *count, int32_t *__restrict__ ncol,
                                                               uint32_t *__restrict__ perm, int32_t *__restrict__ src) {
+  begin_pass();
   static_assert(SEG_WARP_MAX == 256, "rows of up to 8 keys per lane");
   const int lane = threadIdx.x & 31;
   const unsigned cnt = *count;
@@ -885,6 +891,7 @@ __global__ void __launch_bounds__(WB_WARPS * 32) seg_sort_warpbits_kernel(const 
                                                                          int32_t *__restrict__ defer,
                                                                          unsigned *defer_count,
                                                                          int32_t *__restrict__ src) {
+  begin_pass();
   __shared__ uint32_t bits_all[WB_WARPS][WB_WORDS];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   uint32_t *bm = bits_all[w];
@@ -1001,6 +1008,7 @@ __global__ void __launch_bounds__(256) seg_sort_rank_kernel(const int64_t *__res
                                                            int32_t *__restrict__ ncol, uint32_t *__restrict__ perm,
                                                            int32_t *__restrict__ defer, unsigned *defer_count,
                                                            int32_t *__restrict__ src) {
+  begin_pass();
   extern __shared__ uint32_t s_mem[];
   uint32_t *bm = s_mem;                                                 // [SEG_RANK_WORDS]
   int32_t *skey = reinterpret_cast<int32_t *>(bm + SEG_RANK_WORDS);     // [SEG_SMEM_MAX]
@@ -1072,6 +1080,7 @@ __global__ void __launch_bounds__(256) seg_sort_smem_kernel(const int64_t *__res
                                                            const int32_t *__restrict__ list, const unsigned *count,
                                                            int32_t *__restrict__ ncol, uint32_t *__restrict__ perm,
                                                            int32_t *__restrict__ src) {
+  begin_pass();
   __shared__ int32_t skey[SEG_SMEM_MAX];
   __shared__ uint32_t sval[VALS ? SEG_SMEM_MAX : 1];
   __shared__ int32_t s_red[2][8];
@@ -1182,6 +1191,7 @@ template <bool VALS>
 __global__ void __launch_bounds__(1024) seg_sort_global_kernel(const int64_t *__restrict__ nrowptr,
                                                               const int32_t *__restrict__ list, const unsigned *count,
                                                               int32_t *ncol, uint32_t *perm, int32_t *src) {
+  begin_pass();
   const unsigned cnt = *count;
   for (unsigned i = blockIdx.x; i < cnt; i += gridDim.x) {
     const int32_t r = list[i];
@@ -1199,66 +1209,67 @@ template <bool VALS>
 static tc_status launch_row_sorts(tc_ctx *ctx, const DevCSR &g, OrientBufs &b) {
   uint32_t *pv = VALS ? b.perm : nullptr;
   int32_t *sv = b.nsrc;  // rows written by the sorts (every row visits one)
-  if (VALS && g.n <= SEG_PACK_PLACE_MAX_N)
-    seg_sort_pack_kernel<VALS, true><<<grid_for(ctx, g.n, 256, 8), 256, 0, ctx->stream>>>(b.nrowptr, g.n, b.ncol, pv, sv);
-  else if (g.n <= SEG_PACK_MAX_N)
-    seg_sort_pack_kernel<VALS, false><<<grid_for(ctx, g.n, 256, 8), 256, 0, ctx->stream>>>(b.nrowptr, g.n, b.ncol, pv, sv);
-  else if (SEG_WARP_CHUNK)
-    seg_sort_warp_chunk_kernel<VALS><<<grid_for(ctx, g.n, 256, 8), 256, 0, ctx->stream>>>(b.nrowptr, g.n, b.ncol,
-                                                                                          pv, sv);
-  else
-    seg_sort_warp_kernel<VALS><<<grid_for(ctx, g.n * 32, 256, 8), 256, 0, ctx->stream>>>(b.nrowptr, g.n, b.ncol, pv,
-                                                                                         sv);
-  TC_CHECK_LAUNCH(ctx);
-  if (SEG_WARP_REG && VALS && g.n <= SEG_PLACE_MAX_N)
-    seg_sort_warpreg_kernel<VALS, true><<<ctx->num_sms * 8, 256, 0, ctx->stream>>>(b.nrowptr, b.mid_list, b.seg_counts,
-                                                                                  b.ncol, pv, sv);
-  else if (SEG_WARP_REG)
-    seg_sort_warpreg_kernel<VALS, false><<<ctx->num_sms * 8, 256, 0, ctx->stream>>>(b.nrowptr, b.mid_list, b.seg_counts,
-                                                                                   b.ncol, pv, sv);
-  else
+  if (VALS && g.n <= SEG_PACK_PLACE_MAX_N) {
+    TC_CHECK_CUDA(ctx, launch_pass(ctx, seg_sort_pack_kernel<VALS, true>, grid_for(ctx, g.n, 256, 8), 256, 0, b.nrowptr,
+                                   g.n, b.ncol, pv, sv));
+  } else if (g.n <= SEG_PACK_MAX_N) {
+    TC_CHECK_CUDA(ctx, launch_pass(ctx, seg_sort_pack_kernel<VALS, false>, grid_for(ctx, g.n, 256, 8), 256, 0, b.nrowptr,
+                                   g.n, b.ncol, pv, sv));
+  } else {
+    if (SEG_WARP_CHUNK)
+      seg_sort_warp_chunk_kernel<VALS><<<grid_for(ctx, g.n, 256, 8), 256, 0, ctx->stream>>>(b.nrowptr, g.n, b.ncol,
+                                                                                            pv, sv);
+    else
+      seg_sort_warp_kernel<VALS><<<grid_for(ctx, g.n * 32, 256, 8), 256, 0, ctx->stream>>>(b.nrowptr, g.n, b.ncol, pv,
+                                                                                           sv);
+    TC_CHECK_LAUNCH(ctx);
+  }
+  if (SEG_WARP_REG && VALS && g.n <= SEG_PLACE_MAX_N) {
+    TC_CHECK_CUDA(ctx, launch_pass(ctx, seg_sort_warpreg_kernel<VALS, true>, ctx->num_sms * 8, 256, 0, b.nrowptr,
+                                   b.mid_list, b.seg_counts, b.ncol, pv, sv));
+  } else if (SEG_WARP_REG) {
+    TC_CHECK_CUDA(ctx, launch_pass(ctx, seg_sort_warpreg_kernel<VALS, false>, ctx->num_sms * 8, 256, 0, b.nrowptr,
+                                   b.mid_list, b.seg_counts, b.ncol, pv, sv));
+  } else {
     seg_sort_warpsmem_kernel<VALS><<<ctx->num_sms * 8, 256, 0, ctx->stream>>>(b.nrowptr, b.mid_list, b.seg_counts,
                                                                             b.ncol, pv, sv);
-  TC_CHECK_LAUNCH(ctx);
+    TC_CHECK_LAUNCH(ctx);
+  }
   if (!VALS && SEG_WARP_BITS) {
     // narrow rows through warp bitmaps; the rest (deferred into mid_list,
     // which the warp sort above has finished with) through the block sort
-    seg_sort_warpbits_kernel<<<ctx->num_sms * 4, WB_WARPS * 32, 0, ctx->stream>>>(
-        b.nrowptr, b.big_list, b.seg_counts + 1, b.ncol, b.mid_list, b.seg_counts + 3, sv);
-    TC_CHECK_LAUNCH(ctx);
-    seg_sort_smem_kernel<VALS><<<ctx->num_sms * 8, 256, 0, ctx->stream>>>(b.nrowptr, b.mid_list, b.seg_counts + 3,
-                                                                          b.ncol, pv, sv);
+    TC_CHECK_CUDA(ctx, launch_pass(ctx, seg_sort_warpbits_kernel, ctx->num_sms * 4, WB_WARPS * 32, 0, b.nrowptr,
+                                   b.big_list, b.seg_counts + 1, b.ncol, b.mid_list, b.seg_counts + 3, sv));
+    TC_CHECK_CUDA(ctx, launch_pass(ctx, seg_sort_smem_kernel<VALS>, ctx->num_sms * 8, 256, 0, b.nrowptr, b.mid_list,
+                                   b.seg_counts + 3, b.ncol, pv, sv));
   } else if (VALS) {
     TC_CHECK_CUDA(ctx, cudaFuncSetAttribute(seg_sort_rank_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SEG_RANK_SMEM));
-    seg_sort_rank_kernel<<<ctx->num_sms * 4, 256, SEG_RANK_SMEM, ctx->stream>>>(
-        b.nrowptr, b.big_list, b.seg_counts + 1, b.ncol, pv, b.mid_list, b.seg_counts + 3, sv);
-    TC_CHECK_LAUNCH(ctx);
-    seg_sort_smem_kernel<VALS><<<ctx->num_sms * 8, 256, 0, ctx->stream>>>(b.nrowptr, b.mid_list, b.seg_counts + 3,
-                                                                          b.ncol, pv, sv);
+    TC_CHECK_CUDA(ctx, launch_pass(ctx, seg_sort_rank_kernel, ctx->num_sms * 4, 256, SEG_RANK_SMEM, b.nrowptr,
+                                   b.big_list, b.seg_counts + 1, b.ncol, pv, b.mid_list, b.seg_counts + 3, sv));
+    TC_CHECK_CUDA(ctx, launch_pass(ctx, seg_sort_smem_kernel<VALS>, ctx->num_sms * 8, 256, 0, b.nrowptr, b.mid_list,
+                                   b.seg_counts + 3, b.ncol, pv, sv));
   } else {
-    seg_sort_smem_kernel<VALS><<<ctx->num_sms * 8, 256, 0, ctx->stream>>>(b.nrowptr, b.big_list, b.seg_counts + 1,
-                                                                          b.ncol, pv, sv);
+    TC_CHECK_CUDA(ctx, launch_pass(ctx, seg_sort_smem_kernel<VALS>, ctx->num_sms * 8, 256, 0, b.nrowptr, b.big_list,
+                                   b.seg_counts + 1, b.ncol, pv, sv));
   }
-  TC_CHECK_LAUNCH(ctx);
-  seg_sort_global_kernel<VALS><<<ctx->num_sms, 1024, 0, ctx->stream>>>(b.nrowptr, b.huge_list, b.seg_counts + 2,
-                                                                       b.ncol, pv, sv);
-  TC_CHECK_LAUNCH(ctx);
+  TC_CHECK_CUDA(ctx, launch_pass(ctx, seg_sort_global_kernel<VALS>, ctx->num_sms, 1024, 0, b.nrowptr, b.huge_list,
+                                 b.seg_counts + 2, b.ncol, pv, sv));
   return TC_OK;
 }
 
 tc_status orient_phase_b(tc_ctx *ctx, const DevCSR &g, OrientBufs &b, int64_t m, bool want_perm, DevDag *out) {
   if (g.nnz > 0 && m > 0) {
     const int blocks = grid_for(ctx, m, PL_THREADS * PL_UNROLL, 8);
-    if (!out)
-      place_kernel<false, true><<<blocks, PL_THREADS, 0, ctx->stream>>>(b.nsrc, b.kv, m, b.chunk, b.G, b.bcount, b.kept,
-                                                                        b.dag_col, nullptr);
-    else if (want_perm)
-      place_kernel<true, false><<<blocks, PL_THREADS, 0, ctx->stream>>>(b.nsrc, b.kv, m, b.chunk, b.G, b.bcount, b.kept,
-                                                                        b.ncol, b.perm);
-    else
-      place_kernel<false, false><<<blocks, PL_THREADS, 0, ctx->stream>>>(b.nsrc, b.kv, m, b.chunk, b.G, b.bcount, b.kept,
-                                                                         b.ncol, nullptr);
-    TC_CHECK_LAUNCH(ctx);
+    if (!out) {
+      TC_CHECK_CUDA(ctx, launch_pass(ctx, place_kernel<false, true>, blocks, PL_THREADS, 0, b.nsrc, b.kv, m, b.chunk,
+                                     b.G, b.bcount, b.kept, b.dag_col, nullptr));
+    } else if (want_perm) {
+      TC_CHECK_CUDA(ctx, launch_pass(ctx, place_kernel<true, false>, blocks, PL_THREADS, 0, b.nsrc, b.kv, m, b.chunk,
+                                     b.G, b.bcount, b.kept, b.ncol, b.perm));
+    } else {
+      TC_CHECK_CUDA(ctx, launch_pass(ctx, place_kernel<false, false>, blocks, PL_THREADS, 0, b.nsrc, b.kv, m, b.chunk,
+                                     b.G, b.bcount, b.kept, b.ncol, nullptr));
+    }
   }
   if (!out) return TC_OK;
   // the row sorts keep entries inside their rows, so every entry's row
@@ -1358,13 +1369,14 @@ tc_status launch_dag_entries(tc_ctx *ctx, const DevCSR &g, bool validate, int32_
 // relative to the range's first entry (tc_count_dag_range).
 __global__ void shift_rowptr_kernel(const int64_t *__restrict__ rowptr, int64_t n, int64_t shift,
                                     int64_t *__restrict__ out) {
+  begin_pass();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i <= n; i += (int64_t)gridDim.x * blockDim.x)
     out[i] = rowptr[i] - shift;
 }
 
 tc_status launch_shift_rowptr(tc_ctx *ctx, const int64_t *rowptr, int64_t n, int64_t shift, int64_t *out) {
-  shift_rowptr_kernel<<<grid_for(ctx, n + 1, 256, 8), 256, 0, ctx->stream>>>(rowptr, n, shift, out);
-  TC_CHECK_LAUNCH(ctx);
+  TC_CHECK_CUDA(ctx, launch_pass(ctx, shift_rowptr_kernel, grid_for(ctx, n + 1, 256, 8), 256, 0, rowptr, n, shift,
+                                 out));
   return TC_OK;
 }
 
