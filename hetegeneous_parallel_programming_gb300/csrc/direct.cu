@@ -27,6 +27,12 @@ constexpr int DR_THREADS = 256;
 constexpr int DR_PER = 4;                             // 32-entry groups per warp
 constexpr int DR_TILE = DR_THREADS * DR_PER;          // entries per block
 constexpr int DR_GROUPS = DR_TILE / 32;
+// Groups per warp in a large batch, whose rows pass is bound by instruction
+// issue: half as many row searches and fixed costs per entry.  Batches of 1.4 M
+// entries 55 -> 57 us up to the counting, 2.5 M 71 -> 69, 8 M 135 -> 121, 98 M
+// 1085 -> 885; a small graph wants more warps (ER n = 16384: 2 us a call lost).
+constexpr int DR_WIDE_PER = 8;
+constexpr int64_t DR_WIDE_MIN_NNZ = int64_t(1) << 21;
 constexpr int DR_SMEM_BLOCKS = 4096;                  // block sums every placing block scans for itself
 static_assert(DR_GROUPS == 32, "one warp scans a block's group counts");
 
@@ -62,40 +68,46 @@ __device__ __forceinline__ uint32_t half_warp_row(const int64_t *__restrict__ ro
 // lane in slot k.  The rows of the first and last entry are searched
 // (half_warp_row); where they are at most 32 apart, each lane holds one row's
 // end and the entries find theirs by shuffles, else by searches between them.
+template <int PER>
 __device__ __forceinline__ void entry_rows(const int64_t *__restrict__ rowptr, uint32_t n, uint32_t w0, uint32_t w1,
-                                           int lane, uint32_t (&row)[DR_PER], uint32_t (&rb)[DR_PER],
-                                           uint32_t (&re)[DR_PER]) {
+                                           int lane, uint32_t (&row)[PER], uint32_t (&rb)[PER],
+                                           uint32_t (&re)[PER]) {
   const uint32_t r = half_warp_row(rowptr, n, lane < 16 ? w0 : w1 - 1, lane);
   const uint32_t r_lo = __shfl_sync(TC_FULL_MASK, r, 0), r_hi = max(r_lo, __shfl_sync(TC_FULL_MASK, r, 16));
   if (r_hi - r_lo < 32) {
     const uint32_t first = low_word(rowptr, r_lo);
     const uint32_t end = low_word(rowptr, min(r_lo + 1 + lane, n));
+    uint32_t i[PER];  // rows from r_lo on that end at or before the entry
 #pragma unroll
-    for (int k = 0; k < DR_PER; ++k) {
-      const uint32_t e = w0 + 32 * k + lane;
-      uint32_t i = 0;  // rows from r_lo on that end at or before e
+    for (int k = 0; k < PER; ++k) i[k] = 0;
 #pragma unroll
-      for (uint32_t step = 16; step >= 1; step >>= 1) {
-        const uint32_t x = __shfl_sync(TC_FULL_MASK, end, i + step - 1);
-        if (x <= e && r_lo + i + step <= r_hi) i += step;
+    for (uint32_t step = 16; step >= 1; step >>= 1) {
+      if (PER > DR_PER && step > r_hi - r_lo) continue;  // (a branch costs the few warps of a small graph more)
+#pragma unroll
+      for (int k = 0; k < PER; ++k) {
+        const uint32_t x = __shfl_sync(TC_FULL_MASK, end, i[k] + step - 1);
+        if (x <= w0 + 32 * k + lane && r_lo + i[k] + step <= r_hi) i[k] += step;
       }
-      row[k] = r_lo + i;
-      re[k] = __shfl_sync(TC_FULL_MASK, end, i);
-      const uint32_t before = __shfl_sync(TC_FULL_MASK, end, i > 0 ? i - 1 : 0);
-      rb[k] = i > 0 ? before : first;
+    }
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+      row[k] = r_lo + i[k];
+      re[k] = __shfl_sync(TC_FULL_MASK, end, i[k]);
+      const uint32_t before = __shfl_sync(TC_FULL_MASK, end, i[k] > 0 ? i[k] - 1 : 0);
+      rb[k] = i[k] > 0 ? before : first;
     }
     return;
   }
-  uint32_t hi[DR_PER];
+  uint32_t hi[PER];
 #pragma unroll
-  for (int k = 0; k < DR_PER; ++k) {
+  for (int k = 0; k < PER; ++k) {
     row[k] = w0 + 32 * k + lane < w1 ? r_lo : r_hi;
     hi[k] = r_hi + 1;
   }
   for (bool more = true; more;) {
     more = false;
 #pragma unroll
-    for (int k = 0; k < DR_PER; ++k) {
+    for (int k = 0; k < PER; ++k) {
       if (hi[k] - row[k] > 1) {
         const uint32_t mid = (row[k] + hi[k]) >> 1;
         if (low_word(rowptr, mid) <= w0 + 32 * k + lane) row[k] = mid;
@@ -105,7 +117,7 @@ __device__ __forceinline__ void entry_rows(const int64_t *__restrict__ rowptr, u
     }
   }
 #pragma unroll
-  for (int k = 0; k < DR_PER; ++k) {
+  for (int k = 0; k < PER; ++k) {
     rb[k] = low_word(rowptr, row[k]);
     re[k] = low_word(rowptr, row[k] + 1);
   }
@@ -172,8 +184,8 @@ __global__ void __launch_bounds__(DR_THREADS) direct_sample_kernel(const int64_t
 // sums to the same (each vertex's d+ counts once per edge at it).
 // With vtx_off the column ids are local to the row's graph (vgroup).  deg: the
 // vertices' degrees, or null (from the row pointers).
-template <bool ORIENT>
-__global__ void __launch_bounds__(DR_THREADS) direct_rows_kernel(
+template <bool ORIENT, int PER>
+__global__ void __launch_bounds__(DR_TILE / PER) direct_rows_kernel(
     const int64_t *__restrict__ rowptr, const int32_t *__restrict__ col, int64_t n, int64_t nnz,
     const int32_t *__restrict__ vgroup, const int64_t *__restrict__ vtx_off, const uint32_t *__restrict__ deg,
     int32_t *__restrict__ ku, int32_t *__restrict__ kv, uint32_t *__restrict__ mask, uint32_t *__restrict__ gpre, uint32_t *__restrict__ bsum,
@@ -201,33 +213,33 @@ __global__ void __launch_bounds__(DR_THREADS) direct_rows_kernel(
     if (a < 0 || a > nnz) f |= VF_ROWPTR_ENDS;
   }
   const int64_t tile = (int64_t)blockIdx.x * DR_TILE;
-  const uint32_t w0 = (uint32_t)tile + warp * (32 * DR_PER);  // below 2^32 where it is used
-  uint32_t row[DR_PER];
-  int32_t vv[DR_PER];
-  unsigned bal[DR_PER];
+  const uint32_t w0 = (uint32_t)tile + warp * (32 * PER);  // below 2^32 where it is used
+  uint32_t row[PER];
+  int32_t vv[PER];
+  unsigned bal[PER];
 #pragma unroll
-  for (int k = 0; k < DR_PER; ++k) {
+  for (int k = 0; k < PER; ++k) {
     row[k] = 0;
     vv[k] = 0;
     bal[k] = 0;
   }
-  if (tile + warp * (32 * DR_PER) < nnz) {
-    const uint32_t w1 = (uint32_t)min(nnz, (int64_t)w0 + 32 * DR_PER);
-    uint32_t rb[DR_PER], re[DR_PER], dv[DR_PER];
+  if (tile + warp * (32 * PER) < nnz) {
+    const uint32_t w1 = (uint32_t)min(nnz, (int64_t)w0 + 32 * PER);
+    uint32_t rb[PER], re[PER], dv[PER];
 #pragma unroll
-    for (int k = 0; k < DR_PER; ++k) vv[k] = w0 + 32 * k + lane < w1 ? __ldg(col + w0 + 32 * k + lane) : -1;
+    for (int k = 0; k < PER; ++k) vv[k] = w0 + 32 * k + lane < w1 ? __ldg(col + w0 + 32 * k + lane) : -1;
     entry_rows(rowptr, (uint32_t)n, w0, w1, lane, row, rb, re);
     int32_t g_lo = 0, g_hi = 0, base = 0;
     uint32_t size = (uint32_t)n;
     if (vtx_off) {  // one graph for the whole warp, mostly
       g_lo = vgroup[__shfl_sync(TC_FULL_MASK, row[0], 0)];
-      g_hi = vgroup[__shfl_sync(TC_FULL_MASK, row[DR_PER - 1], 31)];
+      g_hi = vgroup[__shfl_sync(TC_FULL_MASK, row[PER - 1], 31)];
       base = (int32_t)vtx_off[g_lo];
       size = (uint32_t)(vtx_off[g_lo + 1] - base);
     }
     int32_t prev_last = w0 > 0 ? __ldg(col + w0 - 1) : -1;  // entry before the warp's
 #pragma unroll
-    for (int k = 0; k < DR_PER; ++k) {
+    for (int k = 0; k < PER; ++k) {
       const uint32_t e = w0 + 32 * k + lane;
       if (g_lo != g_hi) {
         const int32_t gi = vgroup[row[k]];
@@ -251,7 +263,7 @@ __global__ void __launch_bounds__(DR_THREADS) direct_rows_kernel(
       }
     }
 #pragma unroll
-    for (int k = 0; k < DR_PER; ++k) {
+    for (int k = 0; k < PER; ++k) {
       const uint32_t du = re[k] - rb[k];
       const bool ok = w0 + 32 * k + lane < w1 && vv[k] >= 0;
       if (ORIENT) {
@@ -269,12 +281,12 @@ __global__ void __launch_bounds__(DR_THREADS) direct_rows_kernel(
   __syncthreads();
   if (threadIdx.x == 0 && s_work) atomicAdd(res + DX_WORK, s_work);
   if (ORIENT) {
-    if (lane < DR_PER) {
+    if (lane < PER) {
       unsigned b = bal[0];
 #pragma unroll
-      for (int k = 1; k < DR_PER; ++k) b = lane == k ? bal[k] : b;
-      s_cnt[warp * DR_PER + lane] = __popc(b);
-      mask[blockIdx.x * DR_GROUPS + warp * DR_PER + lane] = b;
+      for (int k = 1; k < PER; ++k) b = lane == k ? bal[k] : b;
+      s_cnt[warp * PER + lane] = __popc(b);
+      mask[blockIdx.x * DR_GROUPS + warp * PER + lane] = b;
     }
     __syncthreads();
     const uint32_t c = s_cnt[lane];
@@ -289,8 +301,8 @@ __global__ void __launch_bounds__(DR_THREADS) direct_rows_kernel(
       if (lane == 31) bsum[blockIdx.x] = incl;
     }
 #pragma unroll
-    for (int k = 0; k < DR_PER; ++k) {
-      const uint32_t at = __shfl_sync(TC_FULL_MASK, incl - c, warp * DR_PER + k) + __popc(bal[k] & lt);
+    for (int k = 0; k < PER; ++k) {
+      const uint32_t at = __shfl_sync(TC_FULL_MASK, incl - c, warp * PER + k) + __popc(bal[k] & lt);
       if ((bal[k] >> lane) & 1u) {
         ku[tile + at] = (int32_t)row[k];
         kv[tile + at] = vv[k];
@@ -853,7 +865,7 @@ tc_status direct_run(tc_ctx *ctx, const DevCSR &d, const DirectReq &rq, Bump &bu
   DirectDag g{nullptr, 0, nullptr, nullptr, n, 0, n, nullptr, nullptr, rq.labels, rq.label, 0, 0};
   set_bitmaps(g, n);
   if (rq.orient) {
-    TC_CHECK_CUDA(ctx, launch_pass(ctx, direct_rows_kernel<true>, B, DR_THREADS, 0, d.rowptr, d.col, n, nnz, nullptr,
+    TC_CHECK_CUDA(ctx, launch_pass(ctx, direct_rows_kernel<true, DR_PER>, B, DR_THREADS, 0, d.rowptr, d.col, n, nnz, nullptr,
                                    nullptr, nullptr, ku, kv, mask, gpre, bsum, res));
     const bool scan = B > DR_SMEM_BLOCKS;  // too many block sums for a block to scan
     if (scan) {
@@ -866,7 +878,7 @@ tc_status direct_run(tc_ctx *ctx, const DevCSR &d, const DirectReq &rq, Bump &bu
     g.col = col;
     g.src = src;
   } else {
-    TC_CHECK_CUDA(ctx, launch_pass(ctx, direct_rows_kernel<false>, B, DR_THREADS, 0, d.rowptr, d.col, n, nnz, nullptr,
+    TC_CHECK_CUDA(ctx, launch_pass(ctx, direct_rows_kernel<false, DR_PER>, B, DR_THREADS, 0, d.rowptr, d.col, n, nnz, nullptr,
                                    nullptr, nullptr, ku, nullptr, nullptr, nullptr, nullptr, res));
     g.rp = reinterpret_cast<const uint32_t *>(d.rowptr);
     g.shift = 1;
@@ -992,8 +1004,12 @@ tc_status direct_batch(tc_ctx *ctx, const DevCSR &d, const int64_t *vtx_off, int
     return TC_OK;
   }
   const int64_t max_n = (int64_t)h[DX_MAXN];
-  TC_CHECK_CUDA(ctx, launch_pass(ctx, direct_rows_kernel<true>, B, DR_THREADS, 0, d.rowptr, d.col, n, nnz, vgroup, vtx_off,
-                                 deg, ku, kv, mask, gpre, bsum, res));
+  if (nnz >= DR_WIDE_MIN_NNZ)
+    TC_CHECK_CUDA(ctx, launch_pass(ctx, direct_rows_kernel<true, DR_WIDE_PER>, B, DR_TILE / DR_WIDE_PER, 0, d.rowptr,
+                                   d.col, n, nnz, vgroup, vtx_off, deg, ku, kv, mask, gpre, bsum, res));
+  else
+    TC_CHECK_CUDA(ctx, launch_pass(ctx, direct_rows_kernel<true, DR_PER>, B, DR_THREADS, 0, d.rowptr, d.col, n, nnz,
+                                   vgroup, vtx_off, deg, ku, kv, mask, gpre, bsum, res));
   const bool scan = B > DR_SMEM_BLOCKS;
   if (scan) {
     TC_CHECK_CUDA(ctx, cudaMemsetAsync(bsum + B, 0, sizeof(uint32_t), ctx->stream));

@@ -136,3 +136,19 @@ def test_direct_batch_declines_long_lists(engine):
     rowptr = np.concatenate([[0]] + [r[1:] + g * r[-1] for g in range(graphs)])
     got, _ = engine.batch_count(np.arange(graphs + 1) * k, rowptr, np.tile(c, graphs))
     assert got.tolist() == [k * (k - 1) * (k - 2) // 6] * graphs
+
+
+@pytest.mark.parametrize("graphs,n_min,n_max,deg", [(1, 65537, 65537, 30.5), (1, 65537, 65537, 32.1),
+                                                    (9, 9000, 16384, 29.0), (400, 700, 900, 7.0),
+                                                    (3000, 64, 400, 3.0), (3000, 64, 400, 5.0)])
+def test_direct_batches_around_two_million_entries(engine, graphs, n_min, n_max, deg):
+    """The rows pass of a batch takes 8 groups a warp from 2^21 entries on, 4 below."""
+    vtx, rowptr, colidx = tc.gen_batch_host(num_graphs=graphs, n_min=n_min, n_max=n_max, deg_min=deg, deg_max=deg + 1,
+                                            seed=11)
+    totals, stats = engine.batch_count(vtx, rowptr, colidx)
+    for g in range(0, graphs, max(1, graphs // 40)):
+        a, b = int(vtx[g]), int(vtx[g + 1])
+        lo, hi = int(rowptr[a]), int(rowptr[b])
+        assert totals[g] == oracle.triangles(rowptr[a:b + 1] - lo, colidx[lo:hi])
+    assert np.array_equal(totals, engine.batch_count(vtx, rowptr, colidx, validate=False)[0])
+    assert stats["m"] * 2 == len(colidx)
