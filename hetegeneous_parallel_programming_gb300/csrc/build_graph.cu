@@ -54,7 +54,7 @@ __global__ void edge_keys_kernel(const int32_t *__restrict__ src, const int32_t 
 // neighbours (from the second order), then its larger ones (from the first):
 // both parts are ascending, and an entry's slot is its position plus one row
 // offset, so nothing is counted with atomics or scattered at random.
-// R-MAT scale 21 (33.6 M samples): 9.35 -> 2.57 ms; below about 2^18 samples the
+// R-MAT scale 21 (33.6 M samples): 9.35 -> 2.49 ms; below about 2^18 samples the
 // launches of its second sort cost more than half of the keys save.
 constexpr int64_t HALF_MIN_SAMPLES = int64_t(1) << 18;
 constexpr int UQ_THREADS = 256;
