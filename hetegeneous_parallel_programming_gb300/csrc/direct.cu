@@ -136,8 +136,10 @@ __device__ __forceinline__ unsigned long long clock_ns() {
 }
 
 // Whether the later kernels have nothing to do: invalid input, or lists too
-// long.
-__device__ __forceinline__ bool direct_off(const unsigned long long *res, unsigned long long max_work) {
+// long.  It is the first thing they read of what the passes before them wrote:
+// volatile, so that it stays behind begin_pass's wait (a stale "no" would have
+// row pointers used that the rows pass has refused).
+__device__ __forceinline__ bool direct_off(const volatile unsigned long long *res, unsigned long long max_work) {
   return (unsigned)res[DX_FLAGS] || res[DX_WORK] > max_work;
 }
 
@@ -319,9 +321,9 @@ __global__ void __launch_bounds__(DR_TILE / PER) direct_rows_kernel(
 // itself: 16 KB from L2 cost less than three scan launches.
 __global__ void __launch_bounds__(DR_THREADS) direct_place_kernel(
     const int64_t *__restrict__ rowptr, int64_t n, int64_t nnz, int blocks, const uint32_t *__restrict__ bsum,
-    const uint32_t *__restrict__ boff, const uint32_t *__restrict__ mask, const uint32_t *__restrict__ gpre,
+    const uint32_t *boff, const uint32_t *__restrict__ mask, const uint32_t *__restrict__ gpre,
     const int32_t *__restrict__ ku, const int32_t *__restrict__ kv, int32_t *__restrict__ src,
-    int32_t *__restrict__ col, uint32_t *__restrict__ drow, unsigned long long *__restrict__ res,
+    int32_t *__restrict__ col, uint32_t *__restrict__ drow, const unsigned long long *res,
     unsigned long long max_work) {
   __shared__ uint32_t s_off[DR_SMEM_BLOCKS + 1];
   __shared__ uint32_t tmp[33];
@@ -417,8 +419,7 @@ __device__ __forceinline__ void direct_count_block(const DirectDag &g, uint32_t 
                                                    unsigned long long cap, int chunk,
                                                    unsigned long long *__restrict__ vcount, int copies,
                                                    unsigned long long *__restrict__ totals,
-                                                   unsigned long long *__restrict__ res,
-                                                   unsigned long long max_work) {
+                                                   unsigned long long *res, unsigned long long max_work) {
   extern __shared__ __align__(16) uint32_t s_bm[];
   __shared__ int4 s_rec[DC_WARPS][32];
   __shared__ uint32_t s_hits[DC_WARPS][32];
@@ -726,7 +727,7 @@ __global__ void __launch_bounds__(DC_THREADS, DC_BLOCKS) direct_count_kernel(
 // Sums the copies of the vertex counts.
 __global__ void __launch_bounds__(DC_THREADS) direct_vsum_kernel(const unsigned long long *__restrict__ t, int64_t n,
                                                                 int copies, unsigned long long *__restrict__ out,
-                                                                const unsigned long long *__restrict__ res,
+                                                                const unsigned long long *res,
                                                                 unsigned long long max_work) {
   begin_pass();
   if (direct_off(res, max_work)) return;
