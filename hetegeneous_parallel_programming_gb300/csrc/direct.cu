@@ -954,7 +954,19 @@ __global__ void __launch_bounds__(DR_THREADS) direct_group_kernel(const int64_t 
 // vertices (85 M entries, 30 per entry) take 3.6 ms against 7.1 with the
 // general path; the streaming tests run at 2.2 T list entries/s, so the
 // general path's 0.15 ns an edge is reached at about 300.
-constexpr int64_t BATCH_MAX_LEN = 128;
+// A graph beyond the exact bitmaps has its hits, and the entries that only hash
+// alike, confirmed by searches, and pays 4 to 9 ps a list entry.  Per entry of
+// the batch, direct against general (us): ER n = 100 000 7.4 712, 813; geometric
+// 7.8 887, 839; ER 28 1356, 2016; geometric 29 3033, 2046; R-MAT scale 17 38
+// 1698, 1160 and 67 5133, 1846; Chung-Lu n = 2 M 56 8108, 5308; R-MAT scale 18
+// 82 6681, 2071.  What such a batch may have in any case is what one graph may
+// (direct_max_work): there the general path's launches cost more.
+constexpr int64_t BATCH_MAX_LEN = 128, BATCH_MAX_LEN_HASHED = 8;
+
+static unsigned long long batch_max_work(int64_t max_n, int64_t nnz) {
+  if (max_n <= 32 * DC_WORDS) return (unsigned long long)(BATCH_MAX_LEN * std::max<int64_t>(nnz, 1 << 16));
+  return (unsigned long long)std::max<int64_t>(BATCH_MAX_LEN_HASHED * nnz, int64_t(3) << 25);
+}
 
 bool direct_batch_fits(int64_t nnz, const tc_opts &o) {
   return nnz < (int64_t(1) << 31) && o.validate && o.selector == TC_SELECT_FIXED && !o.record_tile_costs;
@@ -982,7 +994,6 @@ tc_status direct_batch(tc_ctx *ctx, const DevCSR &d, const int64_t *vtx_off, int
   uint32_t *deg = bump.take<uint32_t>(n);
   unsigned long long *tot = bump.take<unsigned long long>(G);
   if (bump.overflow) return set_error(ctx, TC_ERR_OOM, "arena overflow");
-  const unsigned long long max_work = (unsigned long long)BATCH_MAX_LEN * (unsigned long long)std::max<int64_t>(nnz, 1 << 16);
   TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[1], ctx->stream));
   TC_CHECK_CUDA(ctx, cudaMemsetAsync(res, 0, sizeof(unsigned long long) * DX_WORDS, ctx->stream));
   TC_CHECK_CUDA(ctx, cudaMemsetAsync(vgroup, 0, sizeof(int32_t) * (size_t)n, ctx->stream));
@@ -1000,11 +1011,12 @@ tc_status direct_batch(tc_ctx *ctx, const DevCSR &d, const int64_t *vtx_off, int
                                      cudaMemcpyDeviceToHost, ctx->stream));
   TC_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   const unsigned long long *h = ctx->h_pinned;
+  const int64_t max_n = (int64_t)h[DX_MAXN];
+  const unsigned long long max_work = batch_max_work(max_n, nnz);
   if (h[DX_GUESS] > max_work) {
     *declined = true;
     return TC_OK;
   }
-  const int64_t max_n = (int64_t)h[DX_MAXN];
   if (nnz >= DR_WIDE_MIN_NNZ)
     TC_CHECK_CUDA(ctx, launch_pass(ctx, direct_rows_kernel<true, DR_WIDE_PER>, B, DR_TILE / DR_WIDE_PER, 0, d.rowptr,
                                    d.col, n, nnz, vgroup, vtx_off, deg, ku, kv, mask, gpre, bsum, res));

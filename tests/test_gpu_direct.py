@@ -152,3 +152,16 @@ def test_direct_batches_around_two_million_entries(engine, graphs, n_min, n_max,
         assert totals[g] == oracle.triangles(rowptr[a:b + 1] - lo, colidx[lo:hi])
     assert np.array_equal(totals, engine.batch_count(vtx, rowptr, colidx, validate=False)[0])
     assert stats["m"] * 2 == len(colidx)
+
+
+@pytest.mark.parametrize("n,degree,count,direct", [(65536, 24.0, 4, True), (65537, 6.0, 2, True), (65537, 6.0, 60, True),
+                                                   (100000, 24.0, 3, True), (100000, 24.0, 4, False),
+                                                   (100000, 24.0, 16, False), (70000, 60.0, 6, False)])
+def test_batches_of_large_graphs_take_the_quicker_path(engine, n, degree, count, direct):
+    """Beyond 65536 vertices hits are confirmed by searches: a list entry costs several times as much there, so
+    such batches go direct only with short lists (8 per entry), or few (3 * 2^25)."""
+    r, c = csr_of(*tc.gen_edges_host(tc.GenSpec("er", n=n, avg_degree=degree, seed=8)))
+    rowptr = np.concatenate([[0]] + [r[1:] + g * r[-1] for g in range(count)])
+    totals, stats = engine.batch_count(np.arange(count + 1) * n, rowptr, np.tile(c, count))
+    assert (stats["tiles_per_arm"]["flat"] == stats["tiles"]) == direct
+    assert totals.tolist() == [engine.count(r, c, validate=False)[0]] * count
