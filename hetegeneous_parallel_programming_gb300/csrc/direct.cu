@@ -740,28 +740,38 @@ __global__ void __launch_bounds__(DC_THREADS) direct_vsum_kernel(const unsigned 
 
 // ---- host side ---------------------------------------------------------------------
 
-// Which calls count directly.  Measured against the general path (us, one
-// call, whole-GPU clock; W = summed list lengths, see direct_rows_kernel):
-//   ER n = 300, 1.5 K entries       297 ->  41    ER n = 16384, degree 16  350 ->  51
-//   R-MAT scale 15, 0.9 M entries   940 -> 142    Chung-Lu n = 50000       974 -> 140
-//   R-MAT scale 16, degree 64, W = 0.50 G        1865 -> 487
-//   complete graph of 1500 vertices, W = 1.7 G    793 -> 835
-// Beyond 65536 vertices hits are confirmed by searches and pay less:
-//   R-MAT scale 18 of flat skew, W = 0.25 G 2383 -> 800; scale 17, W = 0.42 G 1848 -> 1494;
-//   scale 18, W = 1.1 G 2394 -> 3622; ER of 16 M entries 1361 -> 1150.
-// So entries are bounded by what the unsorted order costs, and W, which skew
-// drives and only the device knows, by a limit: past it the kernels return at
-// once and the general path counts.  Per-vertex counts pay
-// an atomic per triangle (scale 16, degree 64: 2010 -> 903; complete graph of
-// 1500: 3161 -> 4250; a 700-clique among 10^6 vertices, W = 0.17 G, 1245 ->
-// 3856) and have the lower limits.
+// Which calls count directly: entries and vertices by a bound, and W = summed
+// list lengths (see direct_rows_kernel), which skew and density drive and only
+// the device knows, by a limit past which the kernels return at once and the
+// general path counts.  Both paths of one build, us a call (direct, general):
+//   exact bitmaps, count: ER n = 300 40, 290; Chung-Lu n = 60 000 W = 84 M 165,
+//     440; R-MAT scale 16 163 M 246, 576, 496 M 487, 670, 990 M 772, 781; scale 14
+//     1.4 G 803, 742; clique of 1300 1.1 G 730, 540
+//   the same, an oriented input: scale 16 990 M 739, 956; ER of degree 250 0.9 G
+//     454, 1888; but clique of 1200 (lists of 1168 on average) 864 M 1000, 660
+//   the same, labelled (a byte gathered per hit): scale 16 163 M 356, 575; scale 15
+//     365 M 620, 586; scale 16 496 M 871, 686; clique of 900 365 M 1153, 629
+//   the same, per vertex (an atomic per triangle): scale 16 51 M 221, 521; 380 M 767,
+//     753; clique of 450 46 M 548, 599; geometric 102 M 527, 484; clique of 640
+//     131 M 1155, 781
+//   hashed bitmaps, count: R-MAT scale 17 38 M 237, 398, 102 M 563, 538, 189 M
+//     927, 560; Chung-Lu n = 300 000 105 M 417, 469; geometric n = 130 000 223 M
+//     1013, 629; ER n = 130 000 221 M 455, 626; clique of 640 133 M 1262, 632
+//   the same, an oriented input: scale 17 102 M 520, 516; scale 18 141 M 752, 646;
+//     Chung-Lu 105 M 379, 735; clique of 640 1236, 1549; geometric 108 M 609, 413
+//   the same, labelled: scale 18 56 M 386, 395; scale 17 102 M 641, 516; geometric
+//     62 M 616, 535; clique of 500 65 M 804, 553
+//   the same, per vertex: scale 19 65 M 435, 433; scale 17 102 M 663, 606; clique
+//     of 500 818, 732
 constexpr int64_t DIRECT_MAX_NNZ = int64_t(1) << 23;
 constexpr int64_t DIRECT_MAX_N = int64_t(1) << 22;
 
-static unsigned long long direct_max_work(int64_t n, bool per_vertex) {
+static unsigned long long direct_max_work(int64_t n, int64_t nnz, const DirectReq &rq) {
   const bool exact = n <= 32 * DC_WORDS;
-  if (per_vertex) return exact ? 1ull << 29 : 1ull << 27;
-  return exact ? 1ull << 30 : 3ull << 27;
+  if (rq.vertex_counts) return exact ? 3ull << 25 : 1ull << 26;
+  if (rq.labels) return exact ? 5ull << 26 : 1ull << 26;
+  if (!rq.orient) return exact ? std::min(1ull << 30, 1024ull * (unsigned long long)nnz) : 1ull << 27;
+  return exact ? 1ull << 30 : 3ull << 25;
 }
 
 tc_status direct_init(tc_ctx *ctx) {
@@ -831,7 +841,7 @@ tc_status direct_run(tc_ctx *ctx, const DevCSR &d, const DirectReq &rq, Bump &bu
   uint32_t *mask = nullptr, *gpre = nullptr, *bsum = nullptr, *boff = nullptr, *drow = nullptr;
   char *scratch = nullptr;
   const int copies = rq.vertex_counts ? vertex_copies(n) : 1;
-  const unsigned long long max_work = direct_max_work(n, rq.vertex_counts != nullptr);
+  const unsigned long long max_work = direct_max_work(n, nnz, rq);
   if (rq.orient) {
     kv = bump.take<int32_t>(nnz);
     mask = bump.take<uint32_t>((int64_t)B * DR_GROUPS);

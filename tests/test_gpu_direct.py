@@ -165,3 +165,45 @@ def test_batches_of_large_graphs_take_the_quicker_path(engine, n, degree, count,
     totals, stats = engine.batch_count(np.arange(count + 1) * n, rowptr, np.tile(c, count))
     assert (stats["tiles_per_arm"]["flat"] == stats["tiles"]) == direct
     assert totals.tolist() == [engine.count(r, c, validate=False)[0]] * count
+
+
+def in_many(k, n, edges=0):
+    """A clique among n vertices, and a path over the first `edges` of them."""
+    i, j = np.triu_indices(k, 1)
+    a = np.arange(edges)
+    return csr_of(n, np.concatenate([i * (n // k), a]), np.concatenate([j * (n // k), a + 1]))
+
+
+def test_limits_of_the_direct_path(engine):
+    """A call goes direct while its lists sum to no more than the limit of its kind, above and below 65536 vertices
+    (exact and hashed bitmaps): a clique of k vertices sums to k (k - 1)^2 / 2."""
+    n = {"exact": 65536, "hashed": 65537}
+    limits = {("count", "exact"): 1 << 30, ("count", "hashed"): 3 << 25, ("dag", "hashed"): 1 << 27,
+              ("labelled", "exact"): 5 << 26, ("labelled", "hashed"): 1 << 26,
+              ("vertices", "exact"): 3 << 25, ("vertices", "hashed"): 1 << 26}
+    for (kind, size), limit in limits.items():
+        k = 1
+        while (k + 1) * k * k // 2 <= limit:
+            k += 1
+        for clique_size, direct in ((k, True), (k + 1, False)):
+            r, c = in_many(clique_size, n[size])
+            want = clique_size * (clique_size - 1) * (clique_size - 2) // 6
+            if kind == "count":
+                total, _, st = engine.count(r, c)
+            elif kind == "dag":
+                total, _, st = engine.count_dag(*oracle.orient(r, c))
+            elif kind == "labelled":
+                total, _, st = engine.count_labelled(r, c, np.zeros(n[size], np.uint8), 0)
+            else:
+                total, _, st = engine.count_vertices(r, c)
+            assert total == want
+            if direct is False or clique_size * (clique_size - 1) < 1 << 20:  # from 2^20 entries a sample decides first
+                assert (st["tiles_per_arm"]["flat"] == st["tiles"]) == direct, (kind, size, clique_size)
+
+
+@pytest.mark.parametrize("k,direct", [(1020, True), (1030, False)])
+def test_oriented_graphs_of_long_lists_take_the_general_path(engine, k, direct):
+    """Below 65536 vertices an oriented graph also goes direct only with lists of 1024 on average at most."""
+    total, _, st = engine.count_dag(*oracle.orient(*in_many(k, 65536)))
+    assert total == k * (k - 1) * (k - 2) // 6
+    assert (st["tiles_per_arm"]["flat"] == st["tiles"]) == direct
