@@ -48,15 +48,21 @@ __global__ void edge_keys_kernel(const int32_t *__restrict__ src, const int32_t 
   }
 }
 
-// Lists of at least HALF_MIN_SAMPLES: the edges as (min, max) keys sort and lose their duplicates at
+// Long lists (half_keys): the edges as (min, max) keys sort and lose their duplicates at
 // half the size of the directed list; a second, stable sort by max gives every
 // vertex its smaller neighbours in order.  Row w of the CSR is its smaller
 // neighbours (from the second order), then its larger ones (from the first):
 // both parts are ascending, and an entry's slot is its position plus one row
 // offset, so nothing is counted with atomics or scattered at random.
-// R-MAT scale 21 (33.6 M samples): 9.35 -> 2.49 ms; below about 2^18 samples the
-// launches of its second sort cost more than half of the keys save.
-constexpr int64_t HALF_MIN_SAMPLES = int64_t(1) << 18;
+// R-MAT scale 21 (33.6 M samples): 9.35 -> 2.49 ms.  Short lists pay more for the
+// launches of the second sort than half of the keys save, and where vertices
+// outnumber the samples every vertex's two row starts are searched for, which
+// the scan of the degrees beats.  Random lists, us, half keys against directed ones:
+// 2^20 samples, n = 2^16 184, 202, 2^19 215, 213, 2^21 281, 249, 2^24 790, 400;
+// 2^22 samples, n = 2^20 435, 541, 2^22 573, 620, 2^23 746, 665, 2^27 5458, 1890;
+// 2^19 samples, n = 2^15 149, 139; 2^18 samples, n = 2^14 131, 112, 2^27 4089, 1255.
+constexpr int64_t HALF_MIN_SAMPLES = int64_t(1) << 20;
+static bool half_keys(int64_t n, int64_t M) { return M >= HALF_MIN_SAMPLES && n <= M; }
 constexpr int UQ_THREADS = 256;
 constexpr int UQ_PER = 8;
 constexpr int UQ_TILE = UQ_THREADS * UQ_PER;
@@ -218,7 +224,7 @@ tc_status tc_csr_from_edges(tc_ctx *ctx, int64_t n, int64_t M, const int32_t *sr
   TC_CHECK_CUDA(ctx, cudaSetDevice(ctx->device));
   const int bits = bit_width_u64(n > 1 ? (uint64_t)(n - 1) : 1);
   const uint64_t sentinel = (1ULL << (2 * bits)) - 1;
-  const bool half = M >= HALF_MIN_SAMPLES;
+  const bool half = half_keys(n, M);
   const int64_t N = half ? M : 2 * M;  // keys
   const int64_t tiles = (N + UQ_TILE - 1) / UQ_TILE;
   const size_t scratch_bytes =
