@@ -85,6 +85,23 @@ __device__ __forceinline__ bool wedge_beats_pull(const PlanStats &s) {
   return s.mean_da <= 64.f && 14.f * s.low_da + (s.mean_da - s.low_da) < 80.f;
 }
 
+// The same for the tiles that fixed_select leaves to the per-edge arms, which per-vertex and
+// labelled counts cannot use: wedge tests or PULL.  With hub bits (see WD_MIN_TILES)
+// a pair of a hub target costs 2.5 ps and another 9 to 12, else each 5 to 6; PULL
+// 100 to 150 ps an edge, less where most tiles of the graph are PULL's and share
+// its tables, so the mean out-degree m / n moves the line.  One call, ms, labelled
+// (per vertex): all these tiles by wedge tests, all by PULL, this rule.  ER n =
+// 150 000, m / n = 30 0.95, 1.08, 0.95 (0.97, 1.15, 0.97); 50 2.01, 1.38, 1.39 (1.93,
+// 1.51, 1.51); n = 100 000, 100 3.64, 1.86, 1.87 (3.50, 2.17, 2.15); geometric n =
+// 200 000, 30 1.12, 1.06, 1.12 (1.08, 1.22, 1.08); 54 2.96, 1.73, 1.75 (2.57, 2.11,
+// 2.12); n = 100 000, 98 3.49, 1.55, 1.56 (3.05, 2.23, 2.24); R-MAT scale 20 of flat
+// skew, 16 2.17, 2.64, 2.17 (2.17, 2.89, 2.16).  A line through a graph's tiles loses
+// to both sides: ER 30 at a cost of 40 1.16, per vertex at 60 1.28.
+__device__ __forceinline__ bool wedge_attributes(const PlanStats &s, bool hub_bits, bool even_long) {
+  const float cost = hub_bits ? s.mean_da + 2.6f * s.low_da : 2.1f * s.mean_da;
+  return cost < (even_long ? 20.f : 120.f);
+}
+
 // MLP cost model (16 -> 64 -> 64 -> arms, ReLU); weights staged in shared
 // memory rounded to bf16, fp32 accumulation.  Returns the arm with the lowest
 // predicted cost.
@@ -150,6 +167,8 @@ struct PullKeys {
     return v >= hub0 ? base + v : lbase + v;
   }
 };
+
+constexpr int64_t WD_MIN_TILES = 1024;  // wedge tests: without PULL tiles, fewer do not pay for building the hub bit rows
 
 // Whether BSEARCH_4's tiles run as wedge tests (wedge_kernel), and whether they
 // and PULL's are the only ones (hits are attributed or filtered: per-vertex and
@@ -327,7 +346,11 @@ __global__ void __launch_bounds__(PLAN_THREADS) plan_kernel(DevDag g, int64_t T,
     for (int k = 0; k < TC_MLP_FEATURES / 4; ++k) fo[k] = make_float4(f[4 * k], f[4 * k + 1], f[4 * k + 2], f[4 * k + 3]);
     int arm = selector == TC_SELECT_FORCE ? force_arm : fixed_select(st);
     bool settled = arm == TC_ARM_PULL;  // the learned selection keeps the PULL decision
-    if (wedge != PLAN_NO_WEDGE && (settled ? wedge_beats_pull(st) : wedge == PLAN_ATTRIBUTE)) arm = TC_ARM_BSEARCH_4;
+    if (settled) {
+      if (wedge != PLAN_NO_WEDGE && wedge_beats_pull(st)) arm = TC_ARM_BSEARCH_4;
+    } else if (wedge == PLAN_ATTRIBUTE) {
+      arm = wedge_attributes(st, T >= WD_MIN_TILES, g.m >= 40 * g.n) ? TC_ARM_BSEARCH_4 : TC_ARM_PULL;
+    }
     const int level = work_level((unsigned long long)p.sda + p.sdb);
     const unsigned long long alg = 4ull * (p.srow + p.sdb + (unsigned long long)(e1 - e0));
     arm_out[t] = arm;
@@ -2249,7 +2272,6 @@ __global__ void __launch_bounds__(PL_THREADS, TC_PL_MIN_BLOCKS) pull_kernel(DevD
 constexpr int WD_THREADS = 256;
 constexpr int WD_WARPS = WD_THREADS / 32;
 constexpr int WD_U = 4;                   // loads or searches in flight per lane
-constexpr int64_t WD_MIN_TILES = 1024;    // without PULL tiles, fewer do not pay for building the bit rows
 
 // Whether the hub bit rows are built: some tile is PULL's, or BSEARCH_4 has many.
 __device__ __forceinline__ bool hub_bits_used(const int64_t *qoff) {

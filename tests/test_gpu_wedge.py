@@ -55,3 +55,29 @@ def test_wedge_tests(engine, n, fans, core, links, noise):
     assert np.array_equal(sum(sums), per_edge)
     assert engine.load_shipped_selector()
     assert engine.count(rowptr, colidx, validate=False, selector="learned")[0] == total
+
+
+@pytest.mark.parametrize("n,k,cliques,pull", [
+    (100000, 100, 1000, "most"),   # even lists, m / n = 49: PULL shares its tables over most tiles
+    (30000, 100, 300, "most"),     # the same, too few tiles for hub bit rows
+    (156000, 60, 2600, "none"),    # m / n = 29
+    (1000000, 100, 100, "none"),   # a few tiles of them among many vertices
+    (300000, 400, 60, "some"),     # m / n = 16, rows of up to 399 entries
+])
+def test_long_even_lists_of_attributed_counts(engine, n, k, cliques, pull):
+    """Disjoint cliques of k vertices on interleaved ids; per-vertex and labelled counts choose between wedge tests
+    and PULL for the tiles that the fixed rule leaves to other arms."""
+    i, j = np.triu_indices(k, 1)
+    first = np.arange(cliques)[:, None]
+    s, d = (first + cliques * i).ravel(), (first + cliques * j).ravel()
+    rowptr, colidx = engine.csr_from_edges(n, s.astype(np.int32), d.astype(np.int32))
+    total, per_vertex, st = engine.count_vertices(rowptr, colidx, validate=False)
+    assert total == cliques * k * (k - 1) * (k - 2) // 6
+    used = np.arange(n) < cliques * k
+    assert np.array_equal(per_vertex, np.where(used, (k - 1) * (k - 2) // 2, 0).astype(np.uint64))
+    labels = (np.arange(n) % 2).astype(np.uint8)
+    parts = [engine.count_labelled(rowptr, colidx, labels, lab, validate=False) for lab in (0, 1)]
+    assert parts[0][0] + parts[1][0] == total
+    for tiles, arms in [(x["tiles"], x["tiles_per_arm"]) for x in (st, parts[0][2])]:
+        share = arms["pull"] / tiles
+        assert {"most": share > 0.5, "none": share == 0, "some": 0 < share < 1}[pull], (share, arms)
