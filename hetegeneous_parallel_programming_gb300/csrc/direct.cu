@@ -155,6 +155,7 @@ __global__ void __launch_bounds__(DR_THREADS) direct_sample_kernel(const int64_t
                                                                   const int32_t *__restrict__ col, int64_t n,
                                                                   int64_t nnz, const int32_t *__restrict__ vgroup,
                                                                   const int64_t *__restrict__ vtx_off,
+                                                                  uint32_t row_begin, uint32_t row_end,
                                                                   unsigned long long *__restrict__ res) {
   if ((unsigned)res[DX_FLAGS]) return;
   const int lane = threadIdx.x & 31;
@@ -168,7 +169,7 @@ __global__ void __launch_bounds__(DR_THREADS) direct_sample_kernel(const int64_t
     const uint32_t e = w0 + 32 * k + lane;
     int64_t v = e < w1 ? col[e] : -1;
     if (vtx_off && v >= 0) v += vtx_off[vgroup[row[k]]];
-    if (v < 0 || v >= n) continue;
+    if (v < 0 || v >= n || row[k] < row_begin || row[k] >= row_end) continue;
     const uint32_t a = re[k] - rb[k], b = low_word(rowptr, (uint32_t)v + 1) - low_word(rowptr, (uint32_t)v);
     len += ORIENT ? min(a, b) : a + b;  // an undirected edge has two entries
   }
@@ -184,13 +185,14 @@ __global__ void __launch_bounds__(DR_THREADS) direct_sample_kernel(const int64_t
 // res[DX_WORK] += the lists' lengths, summed over the edges u->v: d+(u) + d+(v) of an
 // oriented graph, and where the orientation is made here the degree of u, which
 // sums to the same (each vertex's d+ counts once per edge at it).
-// With vtx_off the column ids are local to the row's graph (vgroup).  deg: the
+// Where the graph comes oriented, only the counted rows [row_begin, row_end) have
+// work.  With vtx_off the column ids are local to the row's graph (vgroup).  deg: the
 // vertices' degrees, or null (from the row pointers).
 template <bool ORIENT, int PER>
 __global__ void __launch_bounds__(DR_TILE / PER) direct_rows_kernel(
     const int64_t *__restrict__ rowptr, const int32_t *__restrict__ col, int64_t n, int64_t nnz,
     const int32_t *__restrict__ vgroup, const int64_t *__restrict__ vtx_off, const uint32_t *__restrict__ deg,
-    int32_t *__restrict__ ku, int32_t *__restrict__ kv, uint32_t *__restrict__ mask, uint32_t *__restrict__ gpre, uint32_t *__restrict__ bsum,
+    uint32_t row_begin, uint32_t row_end, int32_t *__restrict__ ku, int32_t *__restrict__ kv, uint32_t *__restrict__ mask, uint32_t *__restrict__ gpre, uint32_t *__restrict__ bsum,
     unsigned long long *__restrict__ res) {
   __shared__ uint32_t s_cnt[DR_GROUPS];
   __shared__ unsigned long long s_work;
@@ -274,7 +276,7 @@ __global__ void __launch_bounds__(DR_TILE / PER) direct_rows_kernel(
         if (keep) len += du;
       } else if (w0 + 32 * k + lane < w1) {
         ku[w0 + 32 * k + lane] = (int32_t)row[k];
-        if (ok) len += (unsigned long long)du + dv[k];
+        if (ok && row[k] >= row_begin && row[k] < row_end) len += (unsigned long long)du + dv[k];
       }
     }
     len = warp_sum(len);
@@ -859,8 +861,8 @@ tc_status direct_run(tc_ctx *ctx, const DevCSR &d, const DirectReq &rq, Bump &bu
   TC_CHECK_CUDA(ctx, cudaMemsetAsync(res, 0, sizeof(unsigned long long) * DX_WORDS, ctx->stream));
   if (nnz >= DS_MIN_NNZ) {
     constexpr int blocks = DS_WARPS / (DR_THREADS / 32);
-    if (rq.orient) direct_sample_kernel<true><<<blocks, DR_THREADS, 0, ctx->stream>>>(d.rowptr, d.col, n, nnz, nullptr, nullptr, res);
-    else direct_sample_kernel<false><<<blocks, DR_THREADS, 0, ctx->stream>>>(d.rowptr, d.col, n, nnz, nullptr, nullptr, res);
+    if (rq.orient) direct_sample_kernel<true><<<blocks, DR_THREADS, 0, ctx->stream>>>(d.rowptr, d.col, n, nnz, nullptr, nullptr, 0, (uint32_t)n, res);
+    else direct_sample_kernel<false><<<blocks, DR_THREADS, 0, ctx->stream>>>(d.rowptr, d.col, n, nnz, nullptr, nullptr, (uint32_t)rq.row_begin, (uint32_t)rq.row_end, res);
     TC_CHECK_LAUNCH(ctx);
     TC_CHECK_CUDA(ctx, cudaMemcpyAsync(&ctx->h_pinned[0], res + DX_GUESS, sizeof(unsigned long long),
                                        cudaMemcpyDeviceToHost, ctx->stream));
@@ -877,7 +879,7 @@ tc_status direct_run(tc_ctx *ctx, const DevCSR &d, const DirectReq &rq, Bump &bu
   set_bitmaps(g, n);
   if (rq.orient) {
     TC_CHECK_CUDA(ctx, launch_pass(ctx, direct_rows_kernel<true, DR_PER>, B, DR_THREADS, 0, d.rowptr, d.col, n, nnz, nullptr,
-                                   nullptr, nullptr, ku, kv, mask, gpre, bsum, res));
+                                   nullptr, nullptr, 0, (uint32_t)n, ku, kv, mask, gpre, bsum, res));
     const bool scan = B > DR_SMEM_BLOCKS;  // too many block sums for a block to scan
     if (scan) {
       TC_CHECK_CUDA(ctx, cudaMemsetAsync(bsum + B, 0, sizeof(uint32_t), ctx->stream));
@@ -890,7 +892,8 @@ tc_status direct_run(tc_ctx *ctx, const DevCSR &d, const DirectReq &rq, Bump &bu
     g.src = src;
   } else {
     TC_CHECK_CUDA(ctx, launch_pass(ctx, direct_rows_kernel<false, DR_PER>, B, DR_THREADS, 0, d.rowptr, d.col, n, nnz, nullptr,
-                                   nullptr, nullptr, ku, nullptr, nullptr, nullptr, nullptr, res));
+                                   nullptr, nullptr, (uint32_t)rq.row_begin, (uint32_t)rq.row_end, ku, nullptr, nullptr,
+                                   nullptr, nullptr, res));
     g.rp = reinterpret_cast<const uint32_t *>(d.rowptr);
     g.shift = 1;
     g.col = d.col;
@@ -1013,7 +1016,7 @@ tc_status direct_batch(tc_ctx *ctx, const DevCSR &d, const int64_t *vtx_off, int
   TC_CHECK_LAUNCH(ctx);
   if (nnz >= DS_MIN_NNZ) {
     direct_sample_kernel<true><<<DS_WARPS / (DR_THREADS / 32), DR_THREADS, 0, ctx->stream>>>(d.rowptr, d.col, n, nnz,
-                                                                                            vgroup, vtx_off, res);
+                                                                                            vgroup, vtx_off, 0, (uint32_t)n, res);
     TC_CHECK_LAUNCH(ctx);
   }
   // the largest graph decides the bitmaps' width, the sampled lists whether to go on
@@ -1029,10 +1032,10 @@ tc_status direct_batch(tc_ctx *ctx, const DevCSR &d, const int64_t *vtx_off, int
   }
   if (nnz >= DR_WIDE_MIN_NNZ)
     TC_CHECK_CUDA(ctx, launch_pass(ctx, direct_rows_kernel<true, DR_WIDE_PER>, B, DR_TILE / DR_WIDE_PER, 0, d.rowptr,
-                                   d.col, n, nnz, vgroup, vtx_off, deg, ku, kv, mask, gpre, bsum, res));
+                                   d.col, n, nnz, vgroup, vtx_off, deg, 0, (uint32_t)n, ku, kv, mask, gpre, bsum, res));
   else
     TC_CHECK_CUDA(ctx, launch_pass(ctx, direct_rows_kernel<true, DR_PER>, B, DR_THREADS, 0, d.rowptr, d.col, n, nnz,
-                                   vgroup, vtx_off, deg, ku, kv, mask, gpre, bsum, res));
+                                   vgroup, vtx_off, deg, 0, (uint32_t)n, ku, kv, mask, gpre, bsum, res));
   const bool scan = B > DR_SMEM_BLOCKS;
   if (scan) {
     TC_CHECK_CUDA(ctx, cudaMemsetAsync(bsum + B, 0, sizeof(uint32_t), ctx->stream));

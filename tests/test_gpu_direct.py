@@ -207,3 +207,20 @@ def test_oriented_graphs_of_long_lists_take_the_general_path(engine, k, direct):
     total, _, st = engine.count_dag(*oracle.orient(*in_many(k, 65536)))
     assert total == k * (k - 1) * (k - 2) // 6
     assert (st["tiles_per_arm"]["flat"] == st["tiles"]) == direct
+
+
+@pytest.mark.parametrize("small", [False, True])  # 2^20 entries and more are sampled first
+def test_a_row_range_is_judged_by_its_own_lists(engine, small):
+    """A range goes direct by the lists of its own rows, however long those of the rest of the graph are."""
+    k, n = 1030 if small else 1500, 65536  # a clique that a whole count leaves to the general path
+    rowptr, colidx = oracle.orient(*in_many(k, n))
+    total = k * (k - 1) * (k - 2) // 6
+    got, _, st = engine.count_dag(rowptr, colidx)
+    assert got == total and st["tiles_per_arm"]["flat"] == 0
+    at = (n // k) * (k // 2)  # one row of the clique: k - 1 - k // 2 targets, their lists meet in every pair
+    d = k - 1 - k // 2
+    for lo, hi, want in ((at, at + 1, d * (d - 1) // 2), (at + 1, at + 2, 0)):
+        got, pe, st = engine.count_dag_range(rowptr, colidx, lo, hi, edge_counts=True)
+        assert got == int(pe.sum()) == want and st["m"] == (d if want else 0)
+        assert st["tiles_per_arm"]["flat"] == st["tiles"], (lo, hi)
+    assert sum(engine.count_dag_range(rowptr, colidx, a, a + n // 8)[0] for a in range(0, n, n // 8)) == total
