@@ -570,6 +570,7 @@ static tc_status count_direct(tc_ctx *ctx, const tc_csr *g, DirectReq rq, uint64
       rq.labels = tmp;
     }
     if (bump.overflow) return set_error(ctx, TC_ERR_OOM, "arena overflow");
+    TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[1], ctx->stream));
   }
   TC_TRY(direct_run(ctx, d, rq, bump, &st, declined));
   if (*declined) return TC_OK;

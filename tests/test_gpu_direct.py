@@ -224,3 +224,18 @@ def test_a_row_range_is_judged_by_its_own_lists(engine, small):
         assert got == int(pe.sum()) == want and st["m"] == (d if want else 0)
         assert st["tiles_per_arm"]["flat"] == st["tiles"], (lo, hi)
     assert sum(engine.count_dag_range(rowptr, colidx, a, a + n // 8)[0] for a in range(0, n, n // 8)) == total
+
+
+def test_times_of_a_direct_call_cover_its_copies(engine):
+    """The parts of a call with host input and output: none overlaps another, the whole holds them all."""
+    rowptr, colidx = rmat(16, 16)
+    labels = np.zeros(len(rowptr) - 1, np.uint8)
+    for call in (lambda: engine.count_vertices(rowptr, colidx), lambda: engine.count(rowptr, colidx, edge_counts=True),
+                 lambda: engine.count_labelled(rowptr, colidx, labels, 0, edge_counts=True)):
+        call()
+        st = call()[-1]
+        assert st["tiles_per_arm"]["flat"] == st["tiles"]
+        assert st["ms_h2d"] > 0 and st["ms_orient"] > 0 and st["ms_count"] > 0 and st["ms_d2h"] > 0
+        parts = st["ms_h2d"] + st["ms_orient"] + st["ms_count"] + st["ms_d2h"]
+        assert parts <= 1.001 * st["ms_total"] + 0.002  # events and the device's clock resolve about a microsecond
+    assert engine.count(rowptr, colidx)[-1]["ms_d2h"] == 0
