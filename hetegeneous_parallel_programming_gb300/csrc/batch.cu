@@ -88,6 +88,7 @@ tc_status tc_batch_count(tc_ctx *ctx, const tc_batch *b, const tc_opts *opts_in,
   d.n = n;
   d.nnz = nnz;
   const int64_t *d_off = b->vtx_off;
+  Declined dc;
   auto stage = [&](Bump &bump) -> tc_status {
     d.rowptr = b->rowptr;
     d.col = b->colidx;
@@ -95,10 +96,12 @@ tc_status tc_batch_count(tc_ctx *ctx, const tc_batch *b, const tc_opts *opts_in,
     int64_t *o1 = bump.take<int64_t>(G + 1), *r1 = bump.take<int64_t>(n + 1);
     int32_t *c1 = bump.take<int32_t>(nnz);
     if (bump.overflow) return set_error(ctx, TC_ERR_OOM, "arena overflow");
-    TC_CHECK_CUDA(ctx, cudaMemcpyAsync(o1, b->vtx_off, sizeof(int64_t) * (G + 1), cudaMemcpyHostToDevice, ctx->stream));
-    TC_CHECK_CUDA(ctx, cudaMemcpyAsync(r1, b->rowptr, sizeof(int64_t) * (n + 1), cudaMemcpyHostToDevice, ctx->stream));
-    if (nnz > 0)
-      TC_CHECK_CUDA(ctx, cudaMemcpyAsync(c1, b->colidx, sizeof(int32_t) * nnz, cudaMemcpyHostToDevice, ctx->stream));
+    if (!dc.kept) {
+      TC_CHECK_CUDA(ctx, cudaMemcpyAsync(o1, b->vtx_off, sizeof(int64_t) * (G + 1), cudaMemcpyHostToDevice, ctx->stream));
+      TC_CHECK_CUDA(ctx, cudaMemcpyAsync(r1, b->rowptr, sizeof(int64_t) * (n + 1), cudaMemcpyHostToDevice, ctx->stream));
+      if (nnz > 0)
+        TC_CHECK_CUDA(ctx, cudaMemcpyAsync(c1, b->colidx, sizeof(int32_t) * nnz, cudaMemcpyHostToDevice, ctx->stream));
+    }
     st.h2d_bytes = sizeof(int64_t) * (G + 1 + n + 1) + sizeof(int32_t) * nnz;
     d_off = o1;
     d.rowptr = r1;
@@ -113,11 +116,12 @@ tc_status tc_batch_count(tc_ctx *ctx, const tc_batch *b, const tc_opts *opts_in,
     Bump bump{ctx->arena, ctx->arena_cap};
     TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
     TC_TRY(stage(bump));
-    bool declined = false;
-    const tc_status s = direct_batch(ctx, d, d_off, G, bump, totals, &st, &declined);
-    if (s == TC_OK && !declined && stats) *stats = st;
-    if (!declined) return s;
-    ctx->launches = 0;
+    const size_t uploaded = bump.used;
+    const tc_status s = direct_batch(ctx, d, d_off, G, bump, totals, &st, &dc.yes);
+    if (s == TC_OK && !dc.yes && stats) *stats = st;
+    if (!dc.yes) return s;
+    dc.kept = uploaded;
+    dc.ms_h2d = elapsed(ctx->ev[0], ctx->ev[1]);
   }
   const int gbits = bit_width_u64((uint64_t)(G > 1 ? G - 1 : 1));
   Sizer sz;
@@ -127,9 +131,9 @@ tc_status tc_batch_count(tc_ctx *ctx, const tc_batch *b, const tc_opts *opts_in,
   sz.used += count_scratch_bytes(ctx, n, nnz);
   sz.take<uint32_t>(nnz);
   sz.take<unsigned long long>(G);
-  TC_TRY(arena_reserve(ctx, sz.used));
+  TC_TRY(arena_reserve(ctx, sz.used, &dc.kept));
   Bump bump{ctx->arena, ctx->arena_cap};
-  TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
+  if (!dc.yes) TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
   TC_TRY(stage(bump));
   const int64_t *d_row = d.rowptr;
   const int32_t *d_col = d.col;
@@ -238,7 +242,7 @@ tc_status tc_batch_count(tc_ctx *ctx, const tc_batch *b, const tc_opts *opts_in,
   TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[7], ctx->stream));
   TC_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   count_stats(ctx, &st, false);
-  st.ms_h2d = elapsed(ctx->ev[0], ctx->ev[1]);
+  st.ms_h2d = dc.yes ? dc.ms_h2d : elapsed(ctx->ev[0], ctx->ev[1]);
   st.ms_orient = ms_a;
   st.ms_count = elapsed(ctx->ev[4], ctx->ev[6]);  // relabel sort + count + sums (one graph launch)
   st.ms_d2h = elapsed(ctx->ev[6], ctx->ev[7]);

@@ -91,7 +91,7 @@ static tc_status h2d_copy(tc_ctx *ctx, void *dst, const void *src, const void *s
 }
 
 // Device copies of a caller CSR (no copy when already on the device).
-tc_status stage_csr(tc_ctx *ctx, const tc_csr *g, Bump &bump, DevCSR &d, uint64_t *h2d, int pieces) {
+tc_status stage_csr(tc_ctx *ctx, const tc_csr *g, Bump &bump, DevCSR &d, uint64_t *h2d, int pieces, bool staged) {
   d.n = g->n;
   d.nnz = g->nnz;
   if (g->on_device) {
@@ -102,6 +102,10 @@ tc_status stage_csr(tc_ctx *ctx, const tc_csr *g, Bump &bump, DevCSR &d, uint64_
   int64_t *rp = bump.take<int64_t>(g->n + 1);
   int32_t *cl = bump.take<int32_t>(g->nnz);
   if (bump.overflow) return set_error(ctx, TC_ERR_OOM, "arena overflow staging the graph");
+  *h2d += sizeof(int64_t) * (size_t)(g->n + 1) + sizeof(int32_t) * (size_t)g->nnz;
+  d.rowptr = rp;
+  d.col = cl;
+  if (staged) return TC_OK;
   const void *rp_dev = mapped_host(g->rowptr);
   const char *cl_dev = static_cast<const char *>(g->nnz > 0 ? mapped_host(g->colidx) : nullptr);
   TC_TRY(h2d_copy(ctx, rp, g->rowptr, rp_dev, sizeof(int64_t) * (size_t)(g->n + 1), ctx->stream));
@@ -124,9 +128,6 @@ tc_status stage_csr(tc_ctx *ctx, const tc_csr *g, Bump &bump, DevCSR &d, uint64_
   } else if (g->nnz > 0) {
     TC_TRY(h2d_copy(ctx, cl, g->colidx, cl_dev, sizeof(int32_t) * (size_t)g->nnz, ctx->stream));
   }
-  *h2d += sizeof(int64_t) * (size_t)(g->n + 1) + sizeof(int32_t) * (size_t)g->nnz;
-  d.rowptr = rp;
-  d.col = cl;
   return TC_OK;
 }
 
@@ -529,10 +530,10 @@ tc_status tc_ctx_sync(tc_ctx *ctx) {
 }
 
 // A small graph's call (direct_fits): input to the device, direct count.
-// The caller's buffers are in the memory kind of g->on_device.  *declined:
-// nothing was counted, the general path has to.
+// The caller's buffers are in the memory kind of g->on_device.  Declined:
+// nothing was counted, the general path has to; its event 0 stays the call's.
 static tc_status count_direct(tc_ctx *ctx, const tc_csr *g, DirectReq rq, uint64_t *total, uint32_t *edge_counts,
-                              uint64_t *vertex_counts, const uint8_t *labels, tc_stats *stats, bool *declined) {
+                              uint64_t *vertex_counts, const uint8_t *labels, tc_stats *stats, Declined *dc) {
   ctx->launches = 0;
   tc_stats st;
   memset(&st, 0, sizeof(st));
@@ -553,7 +554,16 @@ static tc_status count_direct(tc_ctx *ctx, const tc_csr *g, DirectReq rq, uint64
   TC_TRY(stage_csr(ctx, g, bump, d, &st.h2d_bytes));
   rq.edge_counts = edge_counts;
   rq.labels = labels;
+  size_t uploaded = 0;
   if (!g->on_device) {
+    if (labels) {  // after the CSR, as in the general path
+      uint8_t *tmp = bump.take<uint8_t>(g->n);
+      if (bump.overflow) return set_error(ctx, TC_ERR_OOM, "arena overflow");
+      TC_CHECK_CUDA(ctx, cudaMemcpyAsync(tmp, labels, (size_t)g->n, cudaMemcpyHostToDevice, ctx->stream));
+      st.h2d_bytes += (uint64_t)g->n;
+      rq.labels = tmp;
+    }
+    uploaded = bump.used;
     if (edge_counts) {
       rq.edge_host = edge_counts;
       rq.edge_counts = bump.take<uint32_t>(g->nnz);
@@ -562,18 +572,15 @@ static tc_status count_direct(tc_ctx *ctx, const tc_csr *g, DirectReq rq, uint64
       rq.vertex_host = vertex_counts;
       rq.vertex_counts = bump.take<unsigned long long>(g->n);
     }
-    if (labels) {
-      uint8_t *tmp = bump.take<uint8_t>(g->n);
-      if (bump.overflow) return set_error(ctx, TC_ERR_OOM, "arena overflow");
-      TC_CHECK_CUDA(ctx, cudaMemcpyAsync(tmp, labels, (size_t)g->n, cudaMemcpyHostToDevice, ctx->stream));
-      st.h2d_bytes += (uint64_t)g->n;
-      rq.labels = tmp;
-    }
     if (bump.overflow) return set_error(ctx, TC_ERR_OOM, "arena overflow");
     TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[1], ctx->stream));
   }
-  TC_TRY(direct_run(ctx, d, rq, bump, &st, declined));
-  if (*declined) return TC_OK;
+  TC_TRY(direct_run(ctx, d, rq, bump, &st, &dc->yes));
+  if (dc->yes) {
+    dc->kept = uploaded;
+    if (uploaded) dc->ms_h2d = elapsed(ctx->ev[0], ctx->ev[1]);
+    return TC_OK;
+  }
   *total = ctx->h_pinned[0];
   if (stats) *stats = st;
   return TC_OK;
@@ -587,14 +594,14 @@ tc_status tc_count(tc_ctx *ctx, const tc_csr *g, const tc_opts *opts_in, uint64_
   tc_opts_default(&o);
   if (opts_in) o = *opts_in;
   TC_CHECK_CUDA(ctx, cudaSetDevice(ctx->device));
+  ctx->launches = 0;
+  Declined dc;
   if (direct_fits(g->n, g->nnz, o)) {
     DirectReq rq;
     rq.cap = edge_capacity;
-    bool declined = false;
-    const tc_status s = count_direct(ctx, g, rq, total, edge_counts, nullptr, nullptr, stats, &declined);
-    if (!declined) return s;
+    const tc_status s = count_direct(ctx, g, rq, total, edge_counts, nullptr, nullptr, stats, &dc);
+    if (!dc.yes) return s;
   }
-  ctx->launches = 0;
   tc_stats st;
   memset(&st, 0, sizeof(st));
   const bool want_edges = edge_counts != nullptr;
@@ -607,10 +614,10 @@ tc_status tc_count(tc_ctx *ctx, const tc_csr *g, const tc_opts *opts_in, uint64_
   orient_sizes(ctx, g->n, g->nnz, want_edges, false, sz, pieces);
   sz.used += count_scratch_bytes(ctx, g->n, g->nnz);
   if (want_edges && !g->on_device) sz.take<uint32_t>(g->nnz);
-  TC_TRY(arena_reserve(ctx, sz.used));
+  TC_TRY(arena_reserve(ctx, sz.used, &dc.kept));
   Bump bump{ctx->arena, ctx->arena_cap};
   TC_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_flags, 0, sizeof(unsigned) * 8, ctx->stream));
-  TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
+  if (!dc.yes) TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
   // every return waits for the pieces' uploads: none may outlive the call
   // (the arena and the caller's host arrays are only borrowed)
   struct UploadGuard {
@@ -621,7 +628,7 @@ tc_status tc_count(tc_ctx *ctx, const tc_csr *g, const tc_opts *opts_in, uint64_
     }
   } upload_guard{ctx, pieces > 1};
   DevCSR d;
-  TC_TRY(stage_csr(ctx, g, bump, d, &st.h2d_bytes, pieces));
+  TC_TRY(stage_csr(ctx, g, bump, d, &st.h2d_bytes, pieces, dc.kept > 0));
   OrientBufs ob;
   orient_carve(ctx, d.n, d.nnz, want_edges, false, bump, ob, pieces);
   CountBufs cb;
@@ -633,7 +640,7 @@ tc_status tc_count(tc_ctx *ctx, const tc_csr *g, const tc_opts *opts_in, uint64_
   float ms_a = 0;
   TC_TRY(orient_front(ctx, d, o, ob, &m, &st.ms_validate, &ms_a));
   // with pieces the upload ends at the last piece's event (it overlaps the orientation)
-  st.ms_h2d = elapsed(ctx->ev[0], pieces > 1 ? ctx->piece_ev[pieces - 1] : ctx->ev[1]);
+  st.ms_h2d = dc.yes ? dc.ms_h2d : elapsed(ctx->ev[0], pieces > 1 ? ctx->piece_ev[pieces - 1] : ctx->ev[1]);
   if (want_edges && edge_capacity < m)
     return set_error(ctx, TC_ERR_INVALID_ARG, "edge_counts holds %lld entries, %lld oriented edges",
                      (long long)edge_capacity, (long long)m);
@@ -683,15 +690,15 @@ tc_status tc_count_labelled(tc_ctx *ctx, const tc_csr *g, const uint8_t *vertex_
   if (opts_in) o = *opts_in;
   TC_CHECK_CUDA(ctx, cudaSetDevice(ctx->device));
   o.selector = TC_SELECT_FIXED;  // the caller's selector is ignored
+  ctx->launches = 0;
+  Declined dc;
   if (direct_fits(g->n, g->nnz, o)) {
     DirectReq rq;
     rq.cap = edge_capacity;
     rq.label = label;
-    bool declined = false;
-    const tc_status s = count_direct(ctx, g, rq, total, edge_counts, nullptr, vertex_labels, stats, &declined);
-    if (!declined) return s;
+    const tc_status s = count_direct(ctx, g, rq, total, edge_counts, nullptr, vertex_labels, stats, &dc);
+    if (!dc.yes) return s;
   }
-  ctx->launches = 0;
   tc_stats st;
   memset(&st, 0, sizeof(st));
   const bool want_edges = edge_counts != nullptr;
@@ -701,17 +708,18 @@ tc_status tc_count_labelled(tc_ctx *ctx, const tc_csr *g, const uint8_t *vertex_
   sz.used += count_scratch_bytes(ctx, g->n, g->nnz);
   sz.take<uint8_t>(g->n);
   if (want_edges && !g->on_device) sz.take<uint32_t>(g->nnz);
-  TC_TRY(arena_reserve(ctx, sz.used));
+  TC_TRY(arena_reserve(ctx, sz.used, &dc.kept));
   Bump bump{ctx->arena, ctx->arena_cap};
   TC_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_flags, 0, sizeof(unsigned) * 8, ctx->stream));
-  TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
+  if (!dc.yes) TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
   DevCSR d;
-  TC_TRY(stage_csr(ctx, g, bump, d, &st.h2d_bytes));
+  TC_TRY(stage_csr(ctx, g, bump, d, &st.h2d_bytes, 1, dc.kept > 0));
   const uint8_t *d_lab_in = vertex_labels;
   if (!g->on_device) {
     uint8_t *tmp = bump.take<uint8_t>(d.n);
     if (bump.overflow) return set_error(ctx, TC_ERR_OOM, "arena overflow");
-    TC_CHECK_CUDA(ctx, cudaMemcpyAsync(tmp, vertex_labels, (size_t)d.n, cudaMemcpyHostToDevice, ctx->stream));
+    if (!dc.kept)
+      TC_CHECK_CUDA(ctx, cudaMemcpyAsync(tmp, vertex_labels, (size_t)d.n, cudaMemcpyHostToDevice, ctx->stream));
     st.h2d_bytes += (uint64_t)d.n;
     d_lab_in = tmp;
   }
@@ -727,7 +735,7 @@ tc_status tc_count_labelled(tc_ctx *ctx, const tc_csr *g, const uint8_t *vertex_
   int64_t m = 0;
   float ms_a = 0;
   TC_TRY(orient_front(ctx, d, o, ob, &m, &st.ms_validate, &ms_a));
-  st.ms_h2d = elapsed(ctx->ev[0], ctx->ev[1]);
+  st.ms_h2d = dc.yes ? dc.ms_h2d : elapsed(ctx->ev[0], ctx->ev[1]);
   if (want_edges && edge_capacity < m)
     return set_error(ctx, TC_ERR_INVALID_ARG, "edge_counts holds %lld entries, %lld oriented edges",
                      (long long)edge_capacity, (long long)m);
@@ -779,12 +787,12 @@ tc_status tc_count_vertices(tc_ctx *ctx, const tc_csr *g, const tc_opts *opts_in
   if (opts_in) o = *opts_in;
   TC_CHECK_CUDA(ctx, cudaSetDevice(ctx->device));
   o.selector = TC_SELECT_FIXED;  // the caller's selector is ignored
-  if (direct_fits(g->n, g->nnz, o)) {
-    bool declined = false;
-    const tc_status s = count_direct(ctx, g, DirectReq(), total, nullptr, vertex_counts, nullptr, stats, &declined);
-    if (!declined) return s;
-  }
   ctx->launches = 0;
+  Declined dc;
+  if (direct_fits(g->n, g->nnz, o)) {
+    const tc_status s = count_direct(ctx, g, DirectReq(), total, nullptr, vertex_counts, nullptr, stats, &dc);
+    if (!dc.yes) return s;
+  }
   tc_stats st;
   memset(&st, 0, sizeof(st));
   Sizer sz;
@@ -795,12 +803,12 @@ tc_status tc_count_vertices(tc_ctx *ctx, const tc_csr *g, const tc_opts *opts_in
   sz.take<uint32_t>(g->nnz);
   sz.take<unsigned long long>(g->n);
   if (!g->on_device) sz.take<unsigned long long>(g->n);
-  TC_TRY(arena_reserve(ctx, sz.used));
+  TC_TRY(arena_reserve(ctx, sz.used, &dc.kept));
   Bump bump{ctx->arena, ctx->arena_cap};
   TC_CHECK_CUDA(ctx, cudaMemsetAsync(ctx->d_flags, 0, sizeof(unsigned) * 8, ctx->stream));
-  TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
+  if (!dc.yes) TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
   DevCSR d;
-  TC_TRY(stage_csr(ctx, g, bump, d, &st.h2d_bytes));
+  TC_TRY(stage_csr(ctx, g, bump, d, &st.h2d_bytes, 1, dc.kept > 0));
   OrientBufs ob;
   orient_carve(ctx, d.n, d.nnz, false, false, bump, ob);
   CountBufs cb;
@@ -815,7 +823,7 @@ tc_status tc_count_vertices(tc_ctx *ctx, const tc_csr *g, const tc_opts *opts_in
   int64_t m = 0;
   float ms_a = 0;
   TC_TRY(orient_front(ctx, d, o, ob, &m, &st.ms_validate, &ms_a));
-  st.ms_h2d = elapsed(ctx->ev[0], ctx->ev[1]);
+  st.ms_h2d = dc.yes ? dc.ms_h2d : elapsed(ctx->ev[0], ctx->ev[1]);
   TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[4], ctx->stream));
   DevDag dag;
   TC_TRY(orient_phase_b(ctx, d, ob, m, false, &dag));
@@ -885,16 +893,15 @@ static tc_status count_dag_impl(tc_ctx *ctx, const tc_csr *dag_in, const tc_opts
   if (rr && (rr->row_begin < 0 || rr->row_begin > rr->row_end || rr->row_end > dag_in->n))
     return set_error(ctx, TC_ERR_INVALID_ARG, "row range [%lld, %lld) outside [0, %lld]", (long long)rr->row_begin,
                      (long long)rr->row_end, (long long)dag_in->n);
+  Declined dc;
   if (!pr && direct_fits(dag_in->n, m, o)) {  // reads the range's row pointers on the device
     DirectReq rq;
     rq.orient = false;
     rq.row_begin = rr ? rr->row_begin : 0;
     rq.row_end = rr ? rr->row_end : dag_in->n;
     rq.cap = edge_capacity;
-    bool declined = false;
-    const tc_status s = count_direct(ctx, dag_in, rq, total, edge_counts, nullptr, nullptr, stats, &declined);
-    if (!declined) return s;
-    ctx->launches = 0;
+    const tc_status s = count_direct(ctx, dag_in, rq, total, edge_counts, nullptr, nullptr, stats, &dc);
+    if (!dc.yes) return s;
   }
   if (rr) {
     if (dag_in->on_device) {
@@ -926,11 +933,11 @@ static tc_status count_dag_impl(tc_ctx *ctx, const tc_csr *dag_in, const tc_opts
     if (!dag_in->on_device) sz.take<int64_t>(dag_in->n);
     sz.take<unsigned long long>(pr->num_parts);
   }
-  TC_TRY(arena_reserve(ctx, sz.used));
+  TC_TRY(arena_reserve(ctx, sz.used, &dc.kept));
   Bump bump{ctx->arena, ctx->arena_cap};
-  TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
+  if (!dc.yes) TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
   DevCSR d;
-  TC_TRY(stage_csr(ctx, dag_in, bump, d, &st.h2d_bytes));
+  TC_TRY(stage_csr(ctx, dag_in, bump, d, &st.h2d_bytes, 1, dc.kept > 0));
   int32_t *src = bump.take<int32_t>(m);
   int32_t *indeg = bump.take<int32_t>(dag_in->n);
   int64_t *range_rowptr = rr ? bump.take<int64_t>(dag_in->n + 1) : nullptr;
@@ -1008,7 +1015,7 @@ static tc_status count_dag_impl(tc_ctx *ctx, const tc_csr *dag_in, const tc_opts
   TC_TRY(check_wait_flags(ctx));
   *total = ctx->h_pinned[2];
   count_stats(ctx, &st, true);
-  st.ms_h2d = elapsed(ctx->ev[0], ctx->ev[1]);
+  st.ms_h2d = dc.yes ? dc.ms_h2d : elapsed(ctx->ev[0], ctx->ev[1]);
   st.ms_validate = elapsed(ctx->ev[1], ctx->ev[2]);
   st.ms_orient = elapsed(ctx->ev[4], ctx->ev[5]);
   st.ms_d2h = elapsed(ctx->ev[6], ctx->ev[7]);

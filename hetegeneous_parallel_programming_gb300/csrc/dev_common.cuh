@@ -94,8 +94,10 @@ tc_status set_error(tc_ctx *ctx, tc_status st, const char *fmt, ...);
     if (s_ != TC_OK) return s_;       \
   } while (0)
 
-// Make sure the arena holds at least `bytes`; resets the bump pointer.
-tc_status arena_reserve(tc_ctx *ctx, size_t bytes);
+// Make sure the arena holds at least `bytes`; resets the bump pointer.  With
+// `keep` its first *keep bytes stay; *keep becomes 0 where there is no room for
+// the old and the new arena at once.
+tc_status arena_reserve(tc_ctx *ctx, size_t bytes, size_t *keep = nullptr);
 
 static inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 

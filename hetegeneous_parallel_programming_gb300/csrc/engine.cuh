@@ -137,6 +137,14 @@ tc_status count_carve(const tc_ctx *ctx, int64_t n, int64_t m, Bump &bump, Count
 tc_status run_count(tc_ctx *ctx, const DevDag &dag, const tc_opts &opts, CountBufs &cb, uint32_t *out, bool timing);
 void count_stats(tc_ctx *ctx, tc_stats *st, bool timing);
 
+// A call that the direct path declined: what it uploaded, for the general path
+// to go on with (the arena's first `kept` bytes), and how long that took.
+struct Declined {
+  bool yes = false;
+  size_t kept = 0;
+  float ms_h2d = 0.f;
+};
+
 // Direct counting of small graphs (direct.cu): no relabelling, no grouping,
 // one host read at the end.  Validated input only.
 struct DirectReq {
@@ -169,7 +177,9 @@ tc_status direct_batch(tc_ctx *ctx, const DevCSR &d, const int64_t *vtx_off, int
 // pieces > 1 (host input only): rowptr is copied on the ctx stream, the
 // column array in `pieces` uploads on ctx->copy_stream, each recording
 // ctx->piece_ev[k]; the orientation's kept-count pass waits for them.
-tc_status stage_csr(tc_ctx *ctx, const tc_csr *g, Bump &bump, DevCSR &d, uint64_t *h2d, int pieces = 1);
+// staged: the arrays already lie where the bump's next takes put them.
+tc_status stage_csr(tc_ctx *ctx, const tc_csr *g, Bump &bump, DevCSR &d, uint64_t *h2d, int pieces = 1,
+                    bool staged = false);
 void orient_sizes(const tc_ctx *ctx, int64_t n, int64_t nnz, bool perm, bool dagcol, Sizer &sz, int pieces = 1);
 void orient_carve(const tc_ctx *ctx, int64_t n, int64_t nnz, bool perm, bool dagcol, Bump &bump, OrientBufs &b,
                   int pieces = 1);

@@ -28,16 +28,33 @@ tc_status set_error(tc_ctx *ctx, tc_status st, const char *fmt, ...) {
   return st;
 }
 
-tc_status arena_reserve(tc_ctx *ctx, size_t bytes) {
+tc_status arena_reserve(tc_ctx *ctx, size_t bytes, size_t *keep) {
   ctx->arena_used = 0;
   if (bytes <= ctx->arena_cap) return TC_OK;
+  size_t cap = align_up(bytes + bytes / 8, size_t(1) << 20);
+  char *larger = nullptr;
+  if (keep && *keep > 0) {
+    if (cudaMalloc((void **)&larger, cap) == cudaSuccess) {
+      const cudaError_t e = cudaMemcpyAsync(larger, ctx->arena, *keep, cudaMemcpyDeviceToDevice, ctx->stream);
+      if (e != cudaSuccess) cudaFree(larger);
+      TC_CHECK_CUDA(ctx, e);
+    } else {
+      (void)cudaGetLastError();
+      larger = nullptr;
+      *keep = 0;
+    }
+  }
   if (ctx->arena) {
     TC_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     TC_CHECK_CUDA(ctx, cudaFree(ctx->arena));
     ctx->arena = nullptr;
     ctx->arena_cap = 0;
   }
-  size_t cap = align_up(bytes + bytes / 8, size_t(1) << 20);
+  if (larger) {
+    ctx->arena = larger;
+    ctx->arena_cap = cap;
+    return TC_OK;
+  }
   cudaError_t e = cudaMalloc((void **)&ctx->arena, cap);
   if (e != cudaSuccess) {
     (void)cudaGetLastError();

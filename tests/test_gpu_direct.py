@@ -1,6 +1,8 @@
 """Direct counting of small graphs (csrc/direct.cu): validated calls with the
 fixed selector below its size limits.  Counts are whole numbers, so every
 comparison is for equality."""
+import time
+
 import numpy as np
 import pytest
 
@@ -239,3 +241,41 @@ def test_times_of_a_direct_call_cover_its_copies(engine):
         parts = st["ms_h2d"] + st["ms_orient"] + st["ms_count"] + st["ms_d2h"]
         assert parts <= 1.001 * st["ms_total"] + 0.002  # events and the device's clock resolve about a microsecond
     assert engine.count(rowptr, colidx)[-1]["ms_d2h"] == 0
+
+
+def quickest(call, reps=5):
+    call()
+    times = []
+    for _ in range(reps):
+        t = time.perf_counter()
+        st = call()[-1]
+        times.append((time.perf_counter() - t) * 1e3)
+    return min(times), st
+
+
+def test_declined_host_calls_upload_once(engine):
+    """What a declined call has uploaded stays for the general path: unvalidated calls take that path at once and
+    upload once too, so the difference of the times is less than half an upload (tens of MB)."""
+    n, s, d = tc.gen_edges_host(tc.GenSpec("rmat", scale=22, edge_factor=0.95, seed=3))
+    rowptr, colidx = engine.csr_from_edges(n, s, d)
+    assert (1 << 22) < len(colidx) <= (1 << 23)
+    labels = (np.arange(n) % 3).astype(np.uint8)
+    drow, dcol = engine.orient(rowptr, colidx)
+    k, graphs = 700, 30
+    r, c = clique(k, k, 0)
+    batch = (np.arange(graphs + 1) * k, np.concatenate([[0]] + [r[1:] + g * r[-1] for g in range(graphs)]), np.tile(c, graphs))
+    for call in (lambda v: engine.count(rowptr, colidx, validate=v), lambda v: engine.count_vertices(rowptr, colidx, validate=v),
+                 lambda v: engine.count_labelled(rowptr, colidx, labels, 1, validate=v),
+                 lambda v: engine.batch_count(*batch, validate=v)):
+        declined, st = quickest(lambda: call(True))
+        general, gen = quickest(lambda: call(False))
+        assert st["tiles_per_arm"]["flat"] == 0 and st["h2d_bytes"] == gen["h2d_bytes"] > 1 << 25
+        assert np.array_equal(call(True)[0], call(False)[0])
+        assert st["ms_h2d"] > 0 and declined < general + 0.5 * st["ms_h2d"], (declined, general, st["ms_h2d"])
+        assert st["ms_total"] >= st["ms_h2d"] + st["ms_orient"] + st["ms_count"]
+    with tc.Engine(0) as fresh:  # the arena grows between the two paths
+        assert fresh.count_labelled(rowptr, colidx, labels, 1)[0] == engine.count_labelled(rowptr, colidx, labels, 1)[0]
+    with tc.Engine(0) as fresh:
+        assert fresh.batch_count(*batch)[0].tolist() == [k * (k - 1) * (k - 2) // 6] * graphs
+    with tc.Engine(0) as fresh:
+        assert fresh.count_dag(drow, dcol)[0] == engine.count(rowptr, colidx)[0]
