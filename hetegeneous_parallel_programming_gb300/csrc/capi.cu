@@ -264,6 +264,11 @@ static tc_status check_wait_flags(tc_ctx *ctx) {
   return TC_OK;
 }
 
+// tc_count; with `tuned` always on the general path, whose settings the
+// autotuners time (the direct passes of small graphs read none of them).
+static tc_status count_graph(tc_ctx *ctx, const tc_csr *g, const tc_opts *opts_in, uint64_t *total,
+                             uint32_t *edge_counts, int64_t edge_capacity, tc_stats *stats, bool tuned);
+
 extern "C" {
 
 tc_status tc_set_pull_chunks(tc_ctx *ctx, int32_t item, int32_t item_min) {
@@ -306,7 +311,7 @@ tc_status tc_autotune_pull(tc_ctx *ctx, const tc_csr *g, const tc_opts *opts, co
     for (int32_t r = 0; r <= reps; ++r) {  // r == 0 warms up
       uint64_t total = 0;
       tc_stats st;
-      const tc_status s = tc_count(ctx, g, opts, &total, nullptr, 0, &st);
+      const tc_status s = count_graph(ctx, g, opts, &total, nullptr, 0, &st, true);
       if (s != TC_OK) return restore(s);
       if (i == 0 && r == 0) first_total = total;
       if (total != first_total)
@@ -373,7 +378,7 @@ tc_status tc_autotune(tc_ctx *ctx, const tc_csr *g, const tc_opts *opts, int32_t
     for (int32_t r = 0; r <= reps; ++r) {
       uint64_t total = 0;
       tc_stats st;
-      TC_TRY(tc_count(ctx, g, opts, &total, nullptr, 0, &st));
+      TC_TRY(count_graph(ctx, g, opts, &total, nullptr, 0, &st, true));
       if (!have_total) {
         first_total = total;
         have_total = true;
@@ -586,8 +591,15 @@ static tc_status count_direct(tc_ctx *ctx, const tc_csr *g, DirectReq rq, uint64
   return TC_OK;
 }
 
-tc_status tc_count(tc_ctx *ctx, const tc_csr *g, const tc_opts *opts_in, uint64_t *total, uint32_t *edge_counts,
+tc_status tc_count(tc_ctx *ctx, const tc_csr *g, const tc_opts *opts, uint64_t *total, uint32_t *edge_counts,
                    int64_t edge_capacity, tc_stats *stats) {
+  return count_graph(ctx, g, opts, total, edge_counts, edge_capacity, stats, false);
+}
+
+}  // extern "C"
+
+static tc_status count_graph(tc_ctx *ctx, const tc_csr *g, const tc_opts *opts_in, uint64_t *total,
+                             uint32_t *edge_counts, int64_t edge_capacity, tc_stats *stats, bool tuned) {
   if (!ctx || !total) return set_error(ctx, TC_ERR_INVALID_ARG, "null ctx or total");
   TC_TRY(check_csr_args(ctx, g));
   tc_opts o;
@@ -596,7 +608,7 @@ tc_status tc_count(tc_ctx *ctx, const tc_csr *g, const tc_opts *opts_in, uint64_
   TC_CHECK_CUDA(ctx, cudaSetDevice(ctx->device));
   ctx->launches = 0;
   Declined dc;
-  if (direct_fits(g->n, g->nnz, o)) {
+  if (!tuned && direct_fits(g->n, g->nnz, o)) {
     DirectReq rq;
     rq.cap = edge_capacity;
     const tc_status s = count_direct(ctx, g, rq, total, edge_counts, nullptr, nullptr, stats, &dc);
@@ -676,6 +688,7 @@ tc_status tc_count(tc_ctx *ctx, const tc_csr *g, const tc_opts *opts_in, uint64_
   return TC_OK;
 }
 
+extern "C" {
 
 // Labelled counts: for every oriented edge u->v, the common out-neighbours w
 // whose label is `label` (the reference's labelled intersection, on the DAG).

@@ -96,6 +96,9 @@ typedef struct tc_stats {
   float ms_h2d, ms_validate, ms_orient, ms_plan, ms_count, ms_scatter, ms_d2h, ms_total;
   int64_t m;                       /* oriented edges                          */
   int64_t tiles;                   /* 4096-edge tiles                         */
+  /* Small validated graphs and batches with the fixed selector are counted
+   * directly, in input ids and without the arms' queues: such a call reports
+   * all of its tiles as TC_ARM_FLAT's, whose kernel it does not run. */
   int64_t tiles_per_arm[TC_NUM_ARMS];
   int64_t kernel_launches;         /* engine kernels launched by the call     */
   uint64_t h2d_bytes, d2h_bytes;
@@ -201,14 +204,16 @@ tc_status tc_get_pull_chunks(const tc_ctx *ctx, int32_t *item, int32_t *item_min
  * each of the ncand candidate chunk sizes (item_min = max(32, item / 4)),
  * `reps` times each after one warm-up call, and keeps the candidate with the
  * lowest device time (CUDA events on the ctx stream, best of reps) in the
- * ctx.  ms[i] (optional, ncand entries) receives candidate i's time, *best
+ * ctx.  Every count runs the kernels that the chunks belong to, also on a
+ * small graph that tc_count counts directly without them.  ms[i] (optional, ncand entries) receives candidate i's time, *best
  * (optional) the chosen size.  Every candidate's total must agree, else
  * TC_ERR_INVALID_GRAPH is returned and the ctx keeps its previous sizes. */
 tc_status tc_autotune_pull(tc_ctx *ctx, const tc_csr *g, const tc_opts *opts, const int32_t *candidates,
                            int32_t ncand, int32_t reps, float *ms, int32_t *best);
 
 /* Run-time tuning of one ctx.  Results never depend on it; speed does, per
- * graph.
+ * graph.  Small graphs that are counted directly (see tc_stats) read none of
+ * it.
  *   pull_item, pull_item_min  PULL work chunks (tc_set_pull_chunks)
  *   pull_block_tiles          4096-edge tiles per PULL source block: the hub
  *                             targets' in-edges are grouped per block of rows
@@ -239,8 +244,8 @@ tc_status tc_set_tuning(tc_ctx *ctx, const tc_tuning *t);
  * size (256, 512, 1024), the source-block size (1280, 2560, 5120 tiles),
  * the dense ratio (1/2, 1/1, 2/1) and the orientation geometry (3, 6, 12
  * chunks per SM), one dimension at a time with the others at their best so
- * far.  Every trial counts g (the tc_count contract) once to warm up and
- * `reps` times, keeping the best device time (CUDA events on the ctx
+ * far.  Every trial counts g (the tc_count contract, on the tuned kernels
+ * also where tc_count would count g directly) once to warm up and `reps` times, keeping the best device time (CUDA events on the ctx
  * stream); every trial must count the same triangles, else
  * TC_ERR_INVALID_GRAPH is returned and the ctx keeps its previous tuning.
  * best (optional) receives the chosen tuning, *best_ms its time and

@@ -279,3 +279,21 @@ def test_declined_host_calls_upload_once(engine):
         assert fresh.batch_count(*batch)[0].tolist() == [k * (k - 1) * (k - 2) // 6] * graphs
     with tc.Engine(0) as fresh:
         assert fresh.count_dag(drow, dcol)[0] == engine.count(rowptr, colidx)[0]
+
+
+def test_autotuners_time_the_path_they_tune(engine):
+    """The settings belong to the general path, so that is what a trial runs, also on a graph that counts directly."""
+    rowptr, colidx = rmat(16, 16)
+    old = engine.get_tuning()
+
+    def device_ms(validate):
+        return min(engine.count(rowptr, colidx, validate=validate)[-1]["ms_total"] for _ in range(6))
+    direct, general = device_ms(True), device_ms(False)
+    assert direct < general
+    try:
+        _, ms = engine.autotune_pull(rowptr, colidx, candidates=(256, 512), reps=3)
+        assert min(ms.values()) > (direct + general) / 2, (ms, direct, general)
+        _, best, trials = engine.autotune(rowptr, colidx, reps=3)
+        assert trials > 4 and best > (direct + general) / 2, (best, direct, general)
+    finally:
+        engine.set_tuning(**old)
