@@ -41,3 +41,32 @@ def test_payload_follows_the_rows(engine, n):
     got, pe, _ = engine.count(rowptr, colidx, edge_counts=True, validate=False)  # the general path
     assert got == total and np.array_equal(pe, per_edge)
     assert engine.count(rowptr, colidx, validate=False, force_arm="merge8")[0] == total
+
+
+@pytest.mark.parametrize("n", [1 << 27, (1 << 27) + 1])
+def test_short_rows_on_both_sides_of_the_packed_ids(engine, n):
+    """Rows of at most 32 entries sort packed up to 2^27 vertices and one by one beyond: rows of 1 to 33 entries
+    over a small dense part, on ids up to the last."""
+    rng = np.random.default_rng(n)
+    pool, leaves = 60, 200
+    s, d = [], []
+    lengths = list(range(1, 34)) * 40
+    for i, length in enumerate(lengths):
+        s.append(np.full(length, pool + i))
+        d.append(rng.choice(pool, length, replace=False))
+    first_leaf = pool + len(lengths)
+    s.append(first_leaf + np.arange(pool * leaves))
+    d.append(np.repeat(np.arange(pool), leaves))
+    i, j = np.triu_indices(pool, 1)
+    s.append(i)
+    d.append(j)
+    used = first_leaf + pool * leaves
+    ids = np.unique(rng.integers(0, n - 1, 2 * used))[:used - 1]
+    ids = rng.permutation(np.append(ids, n - 1))
+    rowptr, colidx = engine.csr_from_edges(n, ids[np.concatenate(s)].astype(np.int32),
+                                           ids[np.concatenate(d)].astype(np.int32))
+    total, per_edge, orow, _ = oracle.triangles(rowptr, colidx, per_edge=True)
+    assert set(range(1, 34)) <= set(np.diff(orow).tolist())
+    got, pe, _ = engine.count(rowptr, colidx, edge_counts=True, force_arm="bsearch4")
+    assert got == total and np.array_equal(pe, per_edge)
+    assert engine.count(rowptr, colidx, force_arm="merge8")[0] == total
