@@ -41,7 +41,7 @@ constexpr bool PL_INTERLEAVE = TC_PL_INTERLEAVE != 0;
 #ifndef TC_PLAN_UNROLL
 #define TC_PLAN_UNROLL 2
 #endif
-constexpr int PLAN_UNROLL = TC_PLAN_UNROLL;  // plan_kernel: edges per lane with their gathers in flight
+constexpr int PLAN_UNROLL = TC_PLAN_UNROLL;  // plan_kernel: edges per thread with their gathers in flight
 
 // ---- plan: features + selection ------------------------------------------------
 
@@ -50,8 +50,7 @@ struct PlanStats {
   float mean_in;  // mean DAG in-degree of the edges' targets
   float alr;  // mean |log2 ratio| of the two list lengths
   float low_da;  // mean row suffix of the edges whose targets are not hubs (wedge tests), per edge of the tile
-  float nrows, maxdr, maxwin, frac;
-  float bins[6];
+  float nrows, maxdr, maxwin;
 };
 
 __device__ __forceinline__ float flog2p1(float x) { return __log2f(1.0f + x); }

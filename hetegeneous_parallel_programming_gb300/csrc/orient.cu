@@ -18,23 +18,6 @@ __device__ __forceinline__ void put_row_src(int32_t *__restrict__ src, int64_t b
   if (src)
     for (int k = tid; k < L; k += nt) src[b + k] = r;
 }
-// 1: rows of <= 32 entries are sorted by a warp per 32 consecutive rows
-#ifndef TC_SEG_WARP_CHUNK
-#define TC_SEG_WARP_CHUNK 1
-#endif
-constexpr bool SEG_WARP_CHUNK = TC_SEG_WARP_CHUNK != 0;
-// 1: rows of 33..256 entries are sorted with their keys in registers
-// (seg_sort_warpreg_kernel); 0: in a warp's shared-memory slice
-#ifndef TC_SEG_WARP_REG
-#define TC_SEG_WARP_REG 1
-#endif
-constexpr bool SEG_WARP_REG = TC_SEG_WARP_REG != 0;
-// 1: rows of 257..4096 entries whose ids span <= 32768 values are sorted
-// through a warp's bitmap (seg_sort_warpbits_kernel) before the block sort
-#ifndef TC_SEG_WARP_BITS
-#define TC_SEG_WARP_BITS 1
-#endif
-constexpr bool SEG_WARP_BITS = TC_SEG_WARP_BITS != 0;
 
 void orient_geometry(const tc_ctx *ctx, int64_t nnz, int pieces, int *G, int64_t *chunk) {
   int64_t tiles = (nnz + ENTRY_TILE - 1) / ENTRY_TILE;
@@ -251,9 +234,9 @@ __global__ void rowbase_kernel(const int32_t *__restrict__ rank, const int64_t *
     rowbase[u] = nrowptr[rank[u]] - orowptr[u];
 }
 
-// Rows of the relabelled DAG longer than a warp's registers go to list-driven
-// sorts: up to SEG_WARP_MAX entries one warp in its own shared-memory slice,
-// up to SEG_SMEM_MAX one block in shared memory, beyond that one block in
+// Rows of the relabelled DAG of more than 32 entries go to list-driven sorts:
+// up to SEG_WARP_MAX entries one warp, the keys in its registers, up to
+// SEG_SMEM_MAX a warp's or a block's shared memory, beyond that one block in
 // place in global memory.  Lists are filled with warp-aggregated atomics
 // (their order is irrelevant).
 constexpr int SEG_WARP_MAX = 256;
@@ -464,17 +447,16 @@ __device__ __forceinline__ void chunk_stages32(int32_t *key, uint32_t *val, int 
   }
 }
 
-// The flip network for a list in shared memory of up to 32 * 32 * blocks
-// entries, by the block (SYNC_BLOCK) or by one warp: stages with comparator
-// distance >= 32 in shared memory, the rest in registers, 32 entries per
-// warp at a time.
-template <bool VALS, bool SYNC_BLOCK>
+// The flip network for a list in shared memory, by the block: stages with
+// comparator distance >= 32 in shared memory, the rest in registers, 32
+// entries per warp at a time.
+template <bool VALS>
 __device__ void hybrid_flip_bitonic(int32_t *key, uint32_t *val, int L, int warp, int nwarps, int lane) {
   int P = 32;
   while (P < L) P <<= 1;
-  const int nth = SYNC_BLOCK ? (int)blockDim.x : 32, tid = SYNC_BLOCK ? (int)threadIdx.x : lane;
+  const int nth = (int)blockDim.x, tid = (int)threadIdx.x;
   for (int c0 = warp * 32; c0 < P; c0 += nwarps * 32) chunk_stages32<VALS, true>(key, val, c0, L, lane);
-  if (SYNC_BLOCK) __syncthreads(); else __syncwarp();
+  __syncthreads();
   for (int k = 64; k <= P; k <<= 1) {
     const int h = k >> 1;
     for (int t = tid; t < P / 2; t += nth) {
@@ -482,60 +464,21 @@ __device__ void hybrid_flip_bitonic(int32_t *key, uint32_t *val, int L, int warp
       const int a = blk * k + off, bb = blk * k + k - 1 - off;
       if (bb < L) cmp_swap<VALS>(key, val, a, bb);
     }
-    if (SYNC_BLOCK) __syncthreads(); else __syncwarp();
+    __syncthreads();
     for (int j = k >> 2; j >= 32; j >>= 1) {
       for (int t = tid; t < P / 2; t += nth) {
         const int a = (t / j) * 2 * j + (t % j), bb = a + j;
         if (bb < L) cmp_swap<VALS>(key, val, a, bb);
       }
-      if (SYNC_BLOCK) __syncthreads(); else __syncwarp();
+      __syncthreads();
     }
     for (int c0 = warp * 32; c0 < P; c0 += nwarps * 32) chunk_stages32<VALS, false>(key, val, c0, L, lane);
-    if (SYNC_BLOCK) __syncthreads(); else __syncwarp();
+    __syncthreads();
   }
 }
 
-template <bool VALS>
-__global__ void seg_sort_warp_kernel(const int64_t *__restrict__ nrowptr, int64_t n, int32_t *__restrict__ ncol,
-                                     uint32_t *__restrict__ perm, int32_t *__restrict__ src) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n; r += warps) {
-    const int64_t b = nrowptr[r];
-    const int L = (int)(nrowptr[r + 1] - b);
-    if (L <= 32) put_row_src(src, b, L, (int32_t)r, lane, 32);
-    if (L < 2 || L > 32) continue;
-    int32_t key = lane < L ? ncol[b + lane] : INT32_MAX;
-    uint32_t val = (VALS && lane < L) ? perm[b + lane] : 0u;
-    int P = 2;  // levels up to the row's padded length only (warp-uniform)
-    while (P < L) P <<= 1;
-#pragma unroll
-    for (int k = 2; k <= 32; k <<= 1) {
-      if (k > P) break;
-      {
-        const int partner = lane ^ (k - 1);
-        const int32_t ok = __shfl_sync(TC_FULL_MASK, key, partner);
-        const uint32_t ov = VALS ? __shfl_sync(TC_FULL_MASK, val, partner) : 0u;
-        const bool take = lane < partner ? ok < key : ok > key;
-        if (take) { key = ok; if (VALS) val = ov; }
-      }
-#pragma unroll
-      for (int j = k >> 2; j >= 1; j >>= 1) {
-        const int partner = lane ^ j;
-        const int32_t ok = __shfl_sync(TC_FULL_MASK, key, partner);
-        const uint32_t ov = VALS ? __shfl_sync(TC_FULL_MASK, val, partner) : 0u;
-        const bool take = lane < partner ? ok < key : ok > key;
-        if (take) { key = ok; if (VALS) val = ov; }
-      }
-    }
-    if (lane < L) {
-      ncol[b + lane] = key;
-      if (VALS) perm[b + lane] = val;
-    }
-  }
-}
-
-// The same sort with a warp per 32 consecutive rows: the warp reads their 33
+// Rows of at most 32 entries of graphs beyond 2^27 vertices (see
+// seg_sort_pack_kernel), a warp per 32 consecutive rows: the warp reads their 33
 // row pointers with one coalesced load, then sorts the rows one after
 // another, loading the next row while it sorts the current one, so a row
 // costs one memory round trip instead of the two dependent ones (its
@@ -958,40 +901,6 @@ __global__ void __launch_bounds__(WB_WARPS * 32) seg_sort_warpbits_kernel(const 
   }
 }
 
-// Rows of 33..SEG_WARP_MAX entries: one warp per row sorts in its own slice
-// of shared memory with the same flip network (register stages for
-// distances below 32), synchronising with __syncwarp.
-template <bool VALS>
-__global__ void __launch_bounds__(256) seg_sort_warpsmem_kernel(const int64_t *__restrict__ nrowptr,
-                                                               const int32_t *__restrict__ list,
-                                                               const unsigned *count, int32_t *__restrict__ ncol,
-                                                               uint32_t *__restrict__ perm, int32_t *__restrict__ src) {
-  __shared__ int32_t skey_all[8][SEG_WARP_MAX];
-  __shared__ uint32_t sval_all[VALS ? 8 : 1][VALS ? SEG_WARP_MAX : 1];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  int32_t *key = skey_all[w];
-  uint32_t *val = VALS ? sval_all[w] : nullptr;
-  const unsigned cnt = *count;
-  const unsigned warps = gridDim.x * (blockDim.x >> 5);
-  for (unsigned i = blockIdx.x * (blockDim.x >> 5) + w; i < cnt; i += warps) {
-    const int32_t r = list[i];
-    const int64_t b = nrowptr[r];
-    const int L = (int)(nrowptr[r + 1] - b);
-    for (int k = lane; k < L; k += 32) {
-      key[k] = ncol[b + k];
-      if (VALS) val[k] = perm[b + k];
-    }
-    __syncwarp();
-    hybrid_flip_bitonic<VALS, false>(key, val, L, 0, 1, lane);
-    for (int k = lane; k < L; k += 32) {
-      ncol[b + k] = key[k];
-      if (VALS) perm[b + k] = val[k];
-    }
-    put_row_src(src, b, L, r, lane, 32);
-    __syncwarp();
-  }
-}
-
 // Rows without payload whose ids span at most SEG_SMEM_MAX * 32 values are
 // sorted through a bitmap in the key buffer: one bit per entry (a row's ids
 // are distinct), a block prefix of the words' popcounts, then every thread
@@ -1155,7 +1064,7 @@ __global__ void __launch_bounds__(256) seg_sort_smem_kernel(const int64_t *__res
           for (int j = 0; j < SEG_BITMAP_KEYS; ++j)
             if ((int)threadIdx.x + 256 * j < L) skey[threadIdx.x + 256 * j] = x[j];
           __syncthreads();
-          hybrid_flip_bitonic<VALS, true>(skey, sval, L, warp, blockDim.x >> 5, lane);
+          hybrid_flip_bitonic<VALS>(skey, sval, L, warp, blockDim.x >> 5, lane);
           for (int k = threadIdx.x; k < L; k += blockDim.x) ncol[b + k] = skey[k];
           __syncthreads();
           continue;
@@ -1178,7 +1087,7 @@ __global__ void __launch_bounds__(256) seg_sort_smem_kernel(const int64_t *__res
       if (VALS) sval[k] = perm[b + k];
     }
     __syncthreads();
-    hybrid_flip_bitonic<VALS, true>(skey, sval, L, threadIdx.x >> 5, blockDim.x >> 5, threadIdx.x & 31);
+    hybrid_flip_bitonic<VALS>(skey, sval, L, threadIdx.x >> 5, blockDim.x >> 5, threadIdx.x & 31);
     for (int k = threadIdx.x; k < L; k += blockDim.x) {
       ncol[b + k] = skey[k];
       if (VALS) perm[b + k] = sval[k];
@@ -1216,42 +1125,29 @@ static tc_status launch_row_sorts(tc_ctx *ctx, const DevCSR &g, OrientBufs &b) {
     TC_CHECK_CUDA(ctx, launch_pass(ctx, seg_sort_pack_kernel<VALS, false>, grid_for(ctx, g.n, 256, 8), 256, 0, b.nrowptr,
                                    g.n, b.ncol, pv, sv));
   } else {
-    if (SEG_WARP_CHUNK)
-      seg_sort_warp_chunk_kernel<VALS><<<grid_for(ctx, g.n, 256, 8), 256, 0, ctx->stream>>>(b.nrowptr, g.n, b.ncol,
-                                                                                            pv, sv);
-    else
-      seg_sort_warp_kernel<VALS><<<grid_for(ctx, g.n * 32, 256, 8), 256, 0, ctx->stream>>>(b.nrowptr, g.n, b.ncol, pv,
-                                                                                           sv);
+    seg_sort_warp_chunk_kernel<VALS><<<grid_for(ctx, g.n, 256, 8), 256, 0, ctx->stream>>>(b.nrowptr, g.n, b.ncol, pv,
+                                                                                          sv);
     TC_CHECK_LAUNCH(ctx);
   }
-  if (SEG_WARP_REG && VALS && g.n <= SEG_PLACE_MAX_N) {
+  if (VALS && g.n <= SEG_PLACE_MAX_N) {
     TC_CHECK_CUDA(ctx, launch_pass(ctx, seg_sort_warpreg_kernel<VALS, true>, ctx->num_sms * 8, 256, 0, b.nrowptr,
                                    b.mid_list, b.seg_counts, b.ncol, pv, sv));
-  } else if (SEG_WARP_REG) {
+  } else {
     TC_CHECK_CUDA(ctx, launch_pass(ctx, seg_sort_warpreg_kernel<VALS, false>, ctx->num_sms * 8, 256, 0, b.nrowptr,
                                    b.mid_list, b.seg_counts, b.ncol, pv, sv));
-  } else {
-    seg_sort_warpsmem_kernel<VALS><<<ctx->num_sms * 8, 256, 0, ctx->stream>>>(b.nrowptr, b.mid_list, b.seg_counts,
-                                                                            b.ncol, pv, sv);
-    TC_CHECK_LAUNCH(ctx);
   }
-  if (!VALS && SEG_WARP_BITS) {
-    // narrow rows through warp bitmaps; the rest (deferred into mid_list,
-    // which the warp sort above has finished with) through the block sort
+  // narrow rows through bitmaps; the rest (deferred into mid_list, which the
+  // warp sort above has finished with) through the block sort
+  if (!VALS) {
     TC_CHECK_CUDA(ctx, launch_pass(ctx, seg_sort_warpbits_kernel, ctx->num_sms * 4, WB_WARPS * 32, 0, b.nrowptr,
                                    b.big_list, b.seg_counts + 1, b.ncol, b.mid_list, b.seg_counts + 3, sv));
-    TC_CHECK_CUDA(ctx, launch_pass(ctx, seg_sort_smem_kernel<VALS>, ctx->num_sms * 8, 256, 0, b.nrowptr, b.mid_list,
-                                   b.seg_counts + 3, b.ncol, pv, sv));
-  } else if (VALS) {
+  } else {
     TC_CHECK_CUDA(ctx, cudaFuncSetAttribute(seg_sort_rank_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SEG_RANK_SMEM));
     TC_CHECK_CUDA(ctx, launch_pass(ctx, seg_sort_rank_kernel, ctx->num_sms * 4, 256, SEG_RANK_SMEM, b.nrowptr,
                                    b.big_list, b.seg_counts + 1, b.ncol, pv, b.mid_list, b.seg_counts + 3, sv));
-    TC_CHECK_CUDA(ctx, launch_pass(ctx, seg_sort_smem_kernel<VALS>, ctx->num_sms * 8, 256, 0, b.nrowptr, b.mid_list,
-                                   b.seg_counts + 3, b.ncol, pv, sv));
-  } else {
-    TC_CHECK_CUDA(ctx, launch_pass(ctx, seg_sort_smem_kernel<VALS>, ctx->num_sms * 8, 256, 0, b.nrowptr, b.big_list,
-                                   b.seg_counts + 1, b.ncol, pv, sv));
   }
+  TC_CHECK_CUDA(ctx, launch_pass(ctx, seg_sort_smem_kernel<VALS>, ctx->num_sms * 8, 256, 0, b.nrowptr, b.mid_list,
+                                 b.seg_counts + 3, b.ncol, pv, sv));
   TC_CHECK_CUDA(ctx, launch_pass(ctx, seg_sort_global_kernel<VALS>, ctx->num_sms, 1024, 0, b.nrowptr, b.huge_list,
                                  b.seg_counts + 2, b.ncol, pv, sv));
   return TC_OK;
