@@ -1192,8 +1192,13 @@ tc_status orient_phase_b(tc_ctx *ctx, const DevCSR &g, OrientBufs &b, int64_t m,
 // edges, whole call: 2826 -> 2731 us against a pass each for the checks, the
 // sources and the in-degrees.  Of that the table gives 18 us; 4096 slots give 10
 // more there, but are twice as much to clear and add on small inputs.
+// A chunk costs its entries and the rows between them, which a skewed sparse
+// graph heaps up in a few chunks: 16 chunks an SM, of at least 3 tiles while that
+// leaves 4 an SM.  R-MAT scale 25 with 33 M edges, 4 -> 16 chunks an SM 2.53 -> 1.42
+// ms, scale 24 1.45 -> 0.84; scale 20, 17 M edges 178 -> 163 us; scale 19, 5.9 M 107
+// with 4, 105 with 6, 114 with 16.
 constexpr int DE_SLOTS = 2048;
-constexpr int DE_BLOCKS_PER_SM = 4;
+constexpr int DE_CHUNKS_PER_SM = 16, DE_MIN_CHUNKS_PER_SM = 4, DE_MIN_TILES = 3;
 __global__ void __launch_bounds__(OR_THREADS) dag_entries_kernel(const int64_t *__restrict__ rowptr,
                                                                 const int32_t *__restrict__ col, int64_t n,
                                                                 int64_t m, int64_t chunk, int32_t *__restrict__ src,
@@ -1253,7 +1258,8 @@ tc_status launch_dag_entries(tc_ctx *ctx, const DevCSR &g, bool validate, int32_
   TC_CHECK_CUDA(ctx, cudaMemsetAsync(indeg, 0, sizeof(int32_t) * (size_t)g.n, ctx->stream));
   if (g.nnz <= 0) return TC_OK;
   const int64_t tiles = (g.nnz + ENTRY_TILE - 1) / ENTRY_TILE;
-  const int64_t want = std::min<int64_t>(tiles, (int64_t)ctx->num_sms * DE_BLOCKS_PER_SM);
+  const int64_t most = std::min<int64_t>((int64_t)ctx->num_sms * DE_CHUNKS_PER_SM, tiles / DE_MIN_TILES);
+  const int64_t want = std::min<int64_t>(tiles, std::max<int64_t>((int64_t)ctx->num_sms * DE_MIN_CHUNKS_PER_SM, most));
   const int64_t chunk = (tiles + want - 1) / want * ENTRY_TILE;
   dag_entries_kernel<<<(int)((g.nnz + chunk - 1) / chunk), OR_THREADS, 0, ctx->stream>>>(
       g.rowptr, g.col, g.n, g.nnz, chunk, src, indeg, validate ? ctx->d_flags : nullptr);
