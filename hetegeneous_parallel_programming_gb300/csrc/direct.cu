@@ -7,7 +7,8 @@
 // u->v stays is a comparison of (degree, id) pairs, input rows are sorted, so
 // the kept entries of a row already are, and kept entries compacted in input
 // order are the reference's own edge order (graph.cc:279-290).  Three
-// launches and one host read at the end:
+// launches and one host read at the end (from 2^20 entries on, and for a batch,
+// one more host read before them):
 //   direct_rows   row, validity and direction of every entry; each block
 //                 compacts its kept entries into its own slice
 //   direct_place  slices to their final place, DAG row pointers
@@ -29,7 +30,7 @@ constexpr int DR_PER = 4;                             // 32-entry groups per war
 constexpr int DR_TILE = DR_THREADS * DR_PER;          // entries per block
 constexpr int DR_GROUPS = DR_TILE / 32;
 // Groups per warp in a large batch, whose rows pass is bound by instruction
-// issue: half as many row searches and fixed costs per entry.  Batches of 1.4 M
+// issue (73 % of cycles): half as many row searches and fixed costs per entry.  Batches of 1.4 M
 // entries 55 -> 57 us up to the counting, 2.5 M 71 -> 69, 8 M 135 -> 121, 98 M
 // 1085 -> 885; a small graph wants more warps (ER n = 16384: 2 us a call lost).
 constexpr int DR_WIDE_PER = 8;
@@ -154,7 +155,7 @@ __device__ __forceinline__ bool direct_off(const unsigned long long *res, unsign
 
 // A guess of DX_WORK (see direct_rows_kernel) from DS_WARPS runs of 128 entries
 // spread evenly over a large graph.  The host reads it before the passes over
-// all entries start (12 us), which costs a graph whose lists are too long 25
+// all entries start (12 us), which costs a graph whose lists are too long 43
 // us instead of 170 (R-MAT scale 18).
 constexpr int DS_WARPS = 512;
 constexpr int64_t DS_MIN_NNZ = int64_t(1) << 20;  // below, the pass itself is as quick
@@ -416,9 +417,11 @@ constexpr int DC_SEARCH = 8;        // target list this many times the row's: se
 // confirmed by a search of the row.  Where the edges have more than 4 rows (and
 // more than there are bitmaps), or a target's list is much longer than the row's, the shorter
 // list's entries are searched in the longer one, flattened over the lanes too.
-// Bound by instruction issue: the per-batch work (sums, bitmaps) is spread
-// over 32 edges whatever their rows, which took this kernel from 3.9 ms (a
-// pass per row) to 2.8 ms on 1024 mixed small graphs (49 M edges).  Three
+// Bound by instruction issue at the 24 warps that the bitmaps leave an SM (54 %
+// of cycles issue, 3.5 warps wait on L2 for each that does; 256 mixed graphs): the
+// per-batch work (sums, bitmaps) is spread over 32 edges whatever their rows,
+// which took this kernel from 3.9 ms (a pass per row) to 2.8 ms on 1024 mixed
+// small graphs (49 M edges).  Three
 // blocks with 3 loads in flight a lane against four with 2 (the bitmaps leave
 // room for three): 647 -> 625 us on 256 such graphs; 4 loads 637.
 // MODE 0: counts; 1: triangles of every vertex; 2: common neighbours of one

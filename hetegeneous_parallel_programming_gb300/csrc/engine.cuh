@@ -146,7 +146,8 @@ struct Declined {
 };
 
 // Direct counting of small graphs (direct.cu): no relabelling, no grouping,
-// one host read at the end.  Validated input only.
+// a host read at the end, and from 2^20 entries on one before the passes.
+// Validated input only.
 struct DirectReq {
   bool orient = true;                  // false: the graph is an oriented one
   int64_t row_begin = 0, row_end = 0;  // counted rows of an oriented graph

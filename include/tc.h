@@ -49,7 +49,10 @@ typedef enum tc_status {
 /* Compressed sparse rows.  For tc_count / tc_orient the graph is the
  * symmetric adjacency of a simple undirected graph (each row sorted strictly
  * ascending, no self loops), i.e. what Graph::Graph loads.  For tc_count_dag
- * it is an oriented graph with sorted rows (what Graph::orientation leaves). */
+ * it is an oriented graph with sorted rows (what Graph::orientation leaves).
+ * An oriented graph on the device is counted in place, and the aligned 16-byte
+ * blocks that hold its columns are read whole: up to 12 bytes before colidx and
+ * after colidx + nnz are loaded, and not used. */
 typedef struct tc_csr {
   int64_t n;               /* vertices                                        */
   int64_t nnz;             /* column entries (2m for a symmetric graph)       */
