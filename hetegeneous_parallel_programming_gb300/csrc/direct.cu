@@ -738,6 +738,16 @@ __global__ void __launch_bounds__(DC_THREADS, DC_BLOCKS) direct_count_kernel(
   }
 }
 
+// Clears the caller's vertex counts where they are counted in place (one copy),
+// once the graph is known to be counted: a refused call leaves them as they were.
+__global__ void __launch_bounds__(DC_THREADS) direct_clear_kernel(unsigned long long *__restrict__ out, int64_t n,
+                                                                 const unsigned long long *res,
+                                                                 unsigned long long max_work) {
+  begin_pass();
+  if (direct_off(res, max_work)) return;
+  for (int64_t u = (int64_t)blockIdx.x * DC_THREADS + threadIdx.x; u < n; u += (int64_t)gridDim.x * DC_THREADS) out[u] = 0;
+}
+
 // Sums the copies of the vertex counts.
 __global__ void __launch_bounds__(DC_THREADS) direct_vsum_kernel(const unsigned long long *__restrict__ t, int64_t n,
                                                                 int copies, unsigned long long *__restrict__ out,
@@ -884,7 +894,7 @@ tc_status direct_run(tc_ctx *ctx, const DevCSR &d, const DirectReq &rq, Bump &bu
       return TC_OK;
     }
   }
-  if (rq.vertex_counts)
+  if (copies > 1)
     TC_CHECK_CUDA(ctx, cudaMemsetAsync(vcount, 0, sizeof(unsigned long long) * (size_t)(n * copies), ctx->stream));
   unsigned long long *h = ctx->h_pinned;  // page-locked: the device writes it where it lies
   DirectDag g{nullptr, 0, nullptr, nullptr, n, 0, n, nullptr, nullptr, rq.labels, rq.label, 0, 0};
@@ -892,6 +902,9 @@ tc_status direct_run(tc_ctx *ctx, const DevCSR &d, const DirectReq &rq, Bump &bu
   if (rq.orient) {
     TC_CHECK_CUDA(ctx, launch_pass(ctx, direct_rows_kernel<true, DR_PER>, B, DR_THREADS, 0, d.rowptr, d.col, n, nnz, nullptr,
                                    nullptr, nullptr, 0, (uint32_t)n, ku, kv, mask, gpre, bsum, res));
+    if (rq.vertex_counts && copies == 1)
+      TC_CHECK_CUDA(ctx, launch_pass(ctx, direct_clear_kernel, grid_for(ctx, n, DC_THREADS, 8), DC_THREADS, 0, vcount, n,
+                                     res, max_work));
     const bool scan = B > DR_SMEM_BLOCKS;  // too many block sums for a block to scan
     if (scan) {
       TC_CHECK_CUDA(ctx, cudaMemsetAsync(bsum + B, 0, sizeof(uint32_t), ctx->stream));

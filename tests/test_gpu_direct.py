@@ -297,3 +297,28 @@ def test_autotuners_time_the_path_they_tune(engine):
         assert trials > 4 and best > (direct + general) / 2, (best, direct, general)
     finally:
         engine.set_tuning(**old)
+
+
+@pytest.mark.parametrize("n", [1 << 21, (1 << 21) + 1])  # from one copy of the counts per 2^22 / n warps to a single one
+def test_refused_calls_leave_the_outputs_alone(engine, n):
+    torch = pytest.importorskip("torch")
+    rowptr = np.full(n + 1, 6, np.int64)
+    rowptr[:4] = [0, 2, 4, 6]
+    good, bad = np.array([1, 2, 0, 2, 0, 1]), np.array([1, 2, 0, 2, 0, n])
+    out = torch.full((n,), 77, dtype=torch.int64, device="cuda")
+    edges = torch.full((6,), 77, dtype=torch.int32, device="cuda")
+    rp = torch.from_numpy(rowptr).cuda()
+    for cols in (bad, good):
+        cl = torch.from_numpy(cols.astype(np.int32)).cuda()
+        torch.cuda.synchronize()
+        args = (n, 6, rp.data_ptr(), cl.data_ptr())
+        if cols is good:
+            assert engine.count_vertices_device(*args, out.data_ptr())[0] == 1
+            assert out[:4].tolist() == [1, 1, 1, 0] and int(out.sum()) == 3
+            continue
+        for call in (lambda: engine.count_vertices_device(*args, out.data_ptr()),
+                     lambda: engine.count_device(*args, edge_counts_ptr=edges.data_ptr(), edge_capacity=6)):
+            with pytest.raises(tc.TCError) as e:
+                call()
+            assert e.value.status == 2
+        assert bool((out == 77).all()) and bool((edges == 77).all())
