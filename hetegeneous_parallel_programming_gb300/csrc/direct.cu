@@ -767,35 +767,39 @@ __global__ void __launch_bounds__(DC_THREADS) direct_vsum_kernel(const unsigned 
 // Which calls count directly: entries and vertices by a bound, and W = summed
 // list lengths (see direct_rows_kernel), which skew and density drive and only
 // the device knows, by a limit past which the kernels return at once and the
-// general path counts.  Both paths of one build, us a call (direct, general):
+// general path counts, 45 us later than if it had been asked.  Both paths of one
+// build, us a call (direct, general asked at once); the lines lie where the direct
+// one costs as much as declining, lower where dense parts would lose more:
 //   exact bitmaps, count: ER n = 300 40, 290; Chung-Lu n = 60 000 W = 84 M 165,
 //     440; R-MAT scale 16 163 M 246, 576, 496 M 487, 670, 990 M 772, 781; scale 14
 //     1.4 G 803, 742; clique of 1300 1.1 G 730, 540
 //   the same, an oriented input: scale 16 990 M 739, 956; ER of degree 250 0.9 G
 //     454, 1888; but clique of 1200 (lists of 1168 on average) 864 M 1000, 660
-//   the same, labelled (a byte gathered per hit): scale 16 163 M 356, 575; scale 15
-//     365 M 620, 586; scale 16 496 M 871, 686; clique of 900 365 M 1153, 629
+//   the same, labelled (a byte gathered per hit): scale 16 163 M 356, 575; scale 14
+//     349 M 560, 598; scale 15 365 M 620, 586; clique of 900 365 M 1153, 629
 //   the same, per vertex (an atomic per triangle): scale 16 51 M 221, 521; 380 M 767,
-//     753; clique of 450 46 M 548, 599; geometric 102 M 527, 484; clique of 640
-//     131 M 1155, 781
+//     753; scale 13 120 M 469, 536; clique of 450 46 M 548, 599; geometric 102 M 527,
+//     484; clique of 640 131 M 1155, 781
 //   hashed bitmaps, count: R-MAT scale 17 38 M 237, 398, 102 M 563, 538, 189 M
-//     927, 560; Chung-Lu n = 300 000 105 M 417, 469; geometric n = 130 000 223 M
+//     927, 560; Chung-Lu n = 300 000 105 M 417, 469; R-MAT
+//     scale 20 of flat skew 116 M 597, 585; geometric n = 130 000 223 M
 //     1013, 629; ER n = 130 000 221 M 455, 626; clique of 640 133 M 1262, 632
 //   the same, an oriented input: scale 17 102 M 520, 516; scale 18 141 M 752, 646;
-//     Chung-Lu 105 M 379, 735; clique of 640 1236, 1549; geometric 108 M 609, 413
-//   the same, labelled: scale 18 56 M 386, 395; scale 17 102 M 641, 516; geometric
-//     62 M 616, 535; clique of 500 65 M 804, 553
-//   the same, per vertex: scale 19 65 M 435, 433; scale 17 102 M 663, 606; clique
-//     of 500 818, 732
+//     Chung-Lu 105 M 379, 735, n = 100 000 162 M 616, 1133; scale 17 189 M 932, 601;
+//     clique of 640 1236, 1549; geometric 108 M 609, 413
+//   the same, labelled: scale 18 56 M 386, 395; Chung-Lu n = 1 M 68 M 298, 458;
+//     scale 17 102 M 641, 516; geometric 83 M 528, 472; clique of 500 65 M 804, 553
+//   the same, per vertex: scale 19 65 M 435, 433; geometric 83 M 518, 466; scale 17
+//     102 M 663, 606; clique of 500 818, 732
 constexpr int64_t DIRECT_MAX_NNZ = int64_t(1) << 23;
 constexpr int64_t DIRECT_MAX_N = int64_t(1) << 22;
 
 static unsigned long long direct_max_work(int64_t n, int64_t nnz, const DirectReq &rq) {
   const bool exact = n <= 32 * DC_WORDS;
-  if (rq.vertex_counts) return exact ? 3ull << 25 : 1ull << 26;
-  if (rq.labels) return exact ? 5ull << 26 : 1ull << 26;
-  if (!rq.orient) return exact ? std::min(1ull << 30, 1024ull * (unsigned long long)nnz) : 1ull << 27;
-  return exact ? 1ull << 30 : 3ull << 25;
+  if (rq.vertex_counts) return exact ? 15ull << 23 : 5ull << 24;
+  if (rq.labels) return exact ? 21ull << 24 : 3ull << 25;
+  if (!rq.orient) return exact ? std::min(1ull << 30, 1024ull * (unsigned long long)nnz) : 5ull << 25;
+  return exact ? 1ull << 30 : 7ull << 24;
 }
 
 tc_status direct_init(tc_ctx *ctx) {
@@ -1001,8 +1005,8 @@ __global__ void __launch_bounds__(DR_THREADS) direct_group_kernel(const int64_t 
 // the batch, direct against general (us): ER n = 100 000 7.4 712, 813; geometric
 // 7.8 887, 839; ER 28 1356, 2016; geometric 29 3033, 2046; R-MAT scale 17 38
 // 1698, 1160 and 67 5133, 1846; Chung-Lu n = 2 M 56 8108, 5308; R-MAT scale 18
-// 82 6681, 2071.  What such a batch may have in any case is what one graph may
-// (direct_max_work): there the general path's launches cost more.
+// 82 6681, 2071.  What such a batch may have in any case is near what one graph
+// may (direct_max_work): there the general path's launches cost more.
 constexpr int64_t BATCH_MAX_LEN = 128, BATCH_MAX_LEN_HASHED = 8;
 
 static unsigned long long batch_max_work(int64_t max_n, int64_t nnz) {

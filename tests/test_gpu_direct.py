@@ -180,9 +180,9 @@ def test_limits_of_the_direct_path(engine):
     """A call goes direct while its lists sum to no more than the limit of its kind, above and below 65536 vertices
     (exact and hashed bitmaps): a clique of k vertices sums to k (k - 1)^2 / 2."""
     n = {"exact": 65536, "hashed": 65537}
-    limits = {("count", "exact"): 1 << 30, ("count", "hashed"): 3 << 25, ("dag", "hashed"): 1 << 27,
-              ("labelled", "exact"): 5 << 26, ("labelled", "hashed"): 1 << 26,
-              ("vertices", "exact"): 3 << 25, ("vertices", "hashed"): 1 << 26}
+    limits = {("count", "exact"): 1 << 30, ("count", "hashed"): 7 << 24, ("dag", "hashed"): 5 << 25,
+              ("labelled", "exact"): 21 << 24, ("labelled", "hashed"): 3 << 25,
+              ("vertices", "exact"): 15 << 23, ("vertices", "hashed"): 5 << 24}
     for (kind, size), limit in limits.items():
         k = 1
         while (k + 1) * k * k // 2 <= limit:
