@@ -578,12 +578,12 @@ static tc_status count_direct(tc_ctx *ctx, const tc_csr *g, DirectReq rq, uint64
       rq.vertex_counts = bump.take<unsigned long long>(g->n);
     }
     if (bump.overflow) return set_error(ctx, TC_ERR_OOM, "arena overflow");
-    TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[1], ctx->stream));
+    if (st.h2d_bytes >= DIRECT_TIMED_H2D) TC_CHECK_CUDA(ctx, cudaEventRecord(ctx->ev[1], ctx->stream));
   }
   TC_TRY(direct_run(ctx, d, rq, bump, &st, &dc->yes));
   if (dc->yes) {
     dc->kept = uploaded;
-    if (uploaded) dc->ms_h2d = elapsed(ctx->ev[0], ctx->ev[1]);
+    if (st.h2d_bytes >= DIRECT_TIMED_H2D) dc->ms_h2d = elapsed(ctx->ev[0], ctx->ev[1]);
     return TC_OK;
   }
   *total = ctx->h_pinned[0];

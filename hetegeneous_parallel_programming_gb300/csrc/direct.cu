@@ -962,8 +962,10 @@ tc_status direct_run(tc_ctx *ctx, const DevCSR &d, const DirectReq &rq, Bump &bu
   // events between the passes would keep them apart: the parts are the device
   // clock's, and the copies back, which the host waits for, the host's (events
   // and a wait of their own took 14 of 288 us, Chung-Lu n = 50 000 per vertex)
-  st->ms_total = elapsed(ctx->ev[0], ctx->ev[6]) + st->ms_d2h;
-  st->ms_h2d = st->h2d_bytes ? elapsed(ctx->ev[0], ctx->ev[1]) : 0.f;
+  const float on_device = elapsed(ctx->ev[0], ctx->ev[6]);
+  st->ms_total = on_device + st->ms_d2h;
+  if (st->h2d_bytes >= DIRECT_TIMED_H2D) st->ms_h2d = elapsed(ctx->ev[0], ctx->ev[1]);
+  else if (st->h2d_bytes) st->ms_h2d = std::max(0.f, on_device - 1e-6f * (float)(h[DX_END] - h[DX_START]));
   st->ms_orient = 1e-6f * (float)(h[DX_COUNT] - h[DX_START]);
   st->ms_arm[TC_ARM_FLAT] = st->ms_count = 1e-6f * (float)(h[DX_END] - h[DX_COUNT]);
   st->d2h_bytes += sizeof(unsigned long long) + (rq.edge_host ? sizeof(uint32_t) * (size_t)m : 0) +

@@ -159,12 +159,14 @@ struct DirectReq {
   const uint8_t *labels = nullptr;     // device, input ids
   int label = 0;
 };
+constexpr uint64_t DIRECT_TIMED_H2D = 1 << 20;
 tc_status direct_init(tc_ctx *ctx);  // once per ctx
 bool direct_fits(int64_t n, int64_t nnz, const tc_opts &o);
 void direct_sizes(const tc_ctx *ctx, int64_t n, int64_t nnz, const DirectReq &rq, Sizer &sz);
 // Leaves the total in ctx->h_pinned[0] and fills st (its h2d fields are the
-// caller's); the ctx's event 0 marks the call's start, event 1 the end of its
-// uploads where there are any.  *declined: the lists
+// caller's); the ctx's event 0 marks the call's start, event 1 the end of
+// uploads of at least DIRECT_TIMED_H2D bytes (an event of their own costs small
+// calls 2 to 4 us of 50).  *declined: the lists
 // are too long for it, nothing was counted.
 tc_status direct_run(tc_ctx *ctx, const DevCSR &d, const DirectReq &rq, Bump &bump, tc_stats *st, bool *declined);
 
